@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <map>
 #include <memory>
@@ -145,6 +146,23 @@ void dfree_idle(T *&p) {
     p = nullptr;
 }
 
+// Letter buffers have zeros before their first letter, and callers add 64
+// after the last: extensions read whole blocks.
+constexpr size_t kFrontPad = 64;
+cudaError_t alloc_letters(uint8_t **p, size_t n) {
+    cudaError_t e = dalloc(p, n + kFrontPad);
+    if (e != cudaSuccess)
+        return e;
+    e = cudaMemset(*p, 0, n + kFrontPad);
+    *p += kFrontPad;
+    return e;
+}
+void free_letters(uint8_t *&p) {
+    if (p)
+        p -= kFrontPad;
+    dfree(p);
+}
+
 // Device guard: make `dev` current for the scope.
 struct DeviceScope {
     int prev = -1;
@@ -176,11 +194,16 @@ struct LaunchClass {
     int smem_diag;   // per-warp 16-bit table entries (small for the global class)
     int first;       // groups [first, first + count) of the batch's group list
     int count;
+    int cell;        // bytes of a diagonal cell in byte_kernel (0: these groups cannot use it)
+    int table_len;   // its cells per warp
 };
 struct LaunchShape {
     int threads;
     int blocks;
     int team;        // groups per tile (warps that share each subject)
+    int byte_threads;   // CTA and grid of byte_kernel (0: not used)
+    int byte_blocks;
+    int n_long;      // subjects left to wordfinder_kernel: the longest n_long
 };
 constexpr int kMaxLaunchClasses = 32;
 
@@ -191,6 +214,7 @@ struct hbg_db {
     int64_t n_res = 0;
     int64_t letters_len = 0;
     int32_t max_len = 0;
+    std::vector<int32_t> sched_len;   // subject lengths in scheduling order (descending)
     uint8_t *d_letters = nullptr;
     int64_t *d_off = nullptr;
     int32_t *d_len = nullptr;
@@ -213,7 +237,10 @@ struct hbg_batch {
     uint32_t *d_pv = nullptr;
     uint16_t *d_qcells = nullptr;
     int32_t *d_group_list = nullptr;   // groups ordered by launch class
+    uint32_t *d_packed = nullptr;      // cells of byte_kernel
     std::vector<LaunchClass> classes;
+    bool repeated_entries = false;     // a caller's lookup table lists an offset twice in a cell
+    bool tuned = false;                // the caller chose tiles or table placement (hbg_batch_tune)
     int64_t device_bytes = 0;
     int32_t tile_subjects = 0;   // 0 = automatic (hbg_batch_tune)
     int64_t tile_bytes = 0;      // > 0: tiles of about this many subject letters (hbg_batch_schedule)
@@ -237,6 +264,8 @@ struct hbg_result {
     unsigned int *d_tile = nullptr;
     uint32_t *d_gdiag = nullptr;
     int64_t gdiag_entries = 0;
+    uint16_t *d_side = nullptr;   // flag ends of byte_kernel
+    int64_t side_entries = 0;
     int32_t gdiag_len = 0;   // entries per (CTA, warp) slice of the global diagonal tables
     uint64_t *d_keys = nullptr;
     uint32_t *d_vals = nullptr;
@@ -263,13 +292,16 @@ namespace {
 int64_t batch_device_bytes(const hbg::HostBatch &h) {
     return (int64_t)(h.groups.size() * sizeof(HbgGroup) + h.contexts.size() * sizeof(HbgContext) +
                      h.queries.size() * sizeof(HbgQueryDesc) + h.letters.size() + h.ctx_of.size() * 4 +
-                     h.cells.size() * 4 + h.entries.size() * 2 + h.pv.size() * 4 + h.query_cells.size() * 2);
+                     h.cells.size() * 4 + h.entries.size() * 2 + h.pv.size() * 4 + h.query_cells.size() * 2 +
+                     h.groups.size() * HBG_NUM_CELLS * 4);
 }
 
 void free_batch_device(hbg_batch *b) {
     dfree_idle(b->d_groups);
     dfree_idle(b->d_ctx);
     dfree_idle(b->d_queries);
+    if (b->d_letters)
+        b->d_letters -= kFrontPad;
     dfree_idle(b->d_letters);
     dfree_idle(b->d_ctx_of);
     dfree_idle(b->d_cells);
@@ -277,6 +309,7 @@ void free_batch_device(hbg_batch *b) {
     dfree_idle(b->d_pv);
     dfree_idle(b->d_qcells);
     dfree_idle(b->d_group_list);
+    dfree_idle(b->d_packed);
 }
 
 int upload_batch_buffers(hbg_batch *b, int device);
@@ -298,21 +331,48 @@ int upload_batch(hbg_batch *b, int device) {
     return rc;
 }
 
+// Longest diagonal tables byte_kernel is used for.  With 16-bit cells a
+// 4096-entry table leaves room for 22 warps per SM (9.2 ms for a 4056-letter
+// query against 400,000 subjects; 8-bit cells, 24 warps: 10.3 ms, the sweeps
+// cut its rounds of extensions short; wordfinder_kernel: 13.9 ms).  At 8192
+// entries 8-bit cells are ahead (8152 letters against 200,000 subjects: 9.5 ms
+// with 22 warps, 12.2 ms with 16-bit cells and 12 warps, wordfinder_kernel
+// 16.1 ms); longer tables leave too few warps.
+constexpr int kByteTable16 = 4096;
+constexpr int kByteTable8 = 8192;
+
+// Bytes of a diagonal cell in byte_kernel for a group, 0 when it cannot take
+// the group: its window, table, cell counts or entry count do not fit, or the
+// caller's own table lists an offset twice in a cell (two hits in one place).
+int byte_cell(const hbg_batch *b, int32_t g) {
+    const hbg::HostBatch &h = b->host;
+    const HbgGroup &G = h.groups[g];
+    const uint32_t *cs = h.cells.data() + (size_t)g * HBG_CELL_STRIDE;
+    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.diag_len > kByteTable8 ||
+        cs[HBG_NUM_CELLS] >= (uint32_t)hbg::kByteMaxEntries || b->repeated_entries)
+        return 0;
+    if (G.glen > hbg::kByteMaxCount)             // a cell has at most one entry per letter
+        for (int w = 0; w < HBG_NUM_CELLS; ++w)
+            if (cs[w + 1] - cs[w] > (uint32_t)hbg::kByteMaxCount)
+                return 0;
+    return G.diag_len <= kByteTable16 ? 2 : 1;
+}
+
 int upload_batch_buffers(hbg_batch *b, int device) {
     const hbg::HostBatch &h = b->host;
     CU(dalloc(&b->d_groups, h.groups.size()));
     CU(dalloc(&b->d_ctx, h.contexts.size()));
     CU(dalloc(&b->d_queries, h.queries.size()));
-    CU(dalloc(&b->d_letters, h.letters.size() + 64));
+    CU(alloc_letters(&b->d_letters, h.letters.size() + 64));
     CU(dalloc(&b->d_ctx_of, h.ctx_of.size() + 16));
     CU(dalloc(&b->d_cells, h.cells.size()));
-    CU(dalloc(&b->d_entries, h.entries.size() + 8));
+    CU(dalloc(&b->d_entries, h.entries.size() + 64));   // byte_kernel reads up to 31 past a cell
     CU(dalloc(&b->d_pv, h.pv.size()));
     CU(dalloc(&b->d_qcells, h.query_cells.size()));
+    CU(dalloc(&b->d_packed, h.groups.size() * HBG_NUM_CELLS));
     CU(cudaMemcpy(b->d_groups, h.groups.data(), h.groups.size() * sizeof(HbgGroup), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(b->d_ctx, h.contexts.data(), h.contexts.size() * sizeof(HbgContext), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(b->d_queries, h.queries.data(), h.queries.size() * sizeof(HbgQueryDesc), cudaMemcpyHostToDevice));
-    CU(cudaMemset(b->d_letters, 0, h.letters.size() + 64));
     CU(cudaMemcpy(b->d_letters, h.letters.data(), h.letters.size(), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(b->d_ctx_of, h.ctx_of.data(), h.ctx_of.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(b->d_cells, h.cells.data(), h.cells.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
@@ -326,11 +386,13 @@ int upload_batch_buffers(hbg_batch *b, int device) {
         // shared memory its table needs (the rest is L1 for cells and entries:
         // one 350-aa query vs 10 M subjects 8 % faster than with 2048-entry
         // tables for every group); global-table groups form their own class
-        std::vector<std::pair<std::pair<int, int>, int32_t>> keyed;
+        std::vector<std::pair<std::array<int, 3>, int32_t>> keyed;
         for (int32_t g = 0; g < (int32_t)h.groups.size(); ++g) {
             const HbgGroup &G = h.groups[g];
             const int size = G.placement ? 64 : std::max<int>(64, G.diag_len);
-            keyed.push_back({{G.mode, size}, g});
+            // byte_kernel's table, with the cell size in the low bits
+            const int cell = byte_cell(b, g);
+            keyed.push_back({{G.mode, size, cell ? 4 * std::max<int>(64, G.diag_len) + cell : 0}, g});
         }
         std::stable_sort(keyed.begin(), keyed.end(),
                          [](const auto &x, const auto &y) { return x.first < y.first; });
@@ -339,8 +401,8 @@ int upload_batch_buffers(hbg_batch *b, int device) {
         for (size_t i = 0; i < keyed.size(); ++i) {
             const bool global = h.groups[keyed[i].second].placement != 0;
             if (i == 0 || keyed[i].first != keyed[i - 1].first)
-                b->classes.push_back(LaunchClass{keyed[i].first.first + (global ? 2 : 0), keyed[i].first.second,
-                                                 (int)i, 0});
+                b->classes.push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
+                                                 keyed[i].first[2] & 3, keyed[i].first[2] / 4});
             b->classes.back().count++;
             list.push_back(keyed[i].second);
         }
@@ -349,6 +411,8 @@ int upload_batch_buffers(hbg_batch *b, int device) {
         CU(dalloc(&b->d_group_list, list.size()));
         CU(cudaMemcpy(b->d_group_list, list.data(), list.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
+    CU(hbg::launch_pack_cells(b->d_cells, (int32_t)h.groups.size(), b->d_packed, 0));
+    CU(cudaStreamSynchronize(0));   // the search may run on any stream
     b->device_bytes = batch_device_bytes(h);
     b->device = device;
     return HBG_OK;
@@ -368,14 +432,14 @@ int32_t global_diag_len(const hbg::HostBatch &h, const hbg_db *db) {
 // up to 128, fewer when the class has too little work to give every CTA about
 // eight tiles (small databases and single queries would otherwise leave most
 // SMs idle).
-int32_t class_tile_subjects(const hbg_batch *b, const hbg_db *db, const LaunchClass &lc, int blocks) {
+int32_t class_tile_subjects(const hbg_batch *b, int32_t n_subj, const hbg_db *db, const LaunchClass &lc, int blocks) {
     if (b->tile_subjects > 0)
         return b->tile_subjects;
     if (b->tile_bytes > 0) {                  // subjects of the database's mean length
         const int64_t mean = std::max<int64_t>(1, db->n_res / std::max<int32_t>(1, db->n));
         return (int32_t)std::max<int64_t>(1, std::min<int64_t>(1 << 20, b->tile_bytes / mean));
     }
-    const int64_t want = (int64_t)db->n * lc.count / (8 * (int64_t)std::max(blocks, 1));
+    const int64_t want = (int64_t)n_subj * lc.count / (8 * (int64_t)std::max(blocks, 1));
     return (int32_t)std::max<int64_t>(8, std::min<int64_t>(128, want));
 }
 
@@ -414,9 +478,40 @@ int plan_launches(const hbg_batch *b, const hbg_gpu_options &o, int device, std:
         if (best_t == 0)
             return fail(HBG_ERR_TOO_LONG, "group diagonal tables exceed shared memory");
         const int blocks = o.num_blocksx > 0 ? o.num_blocksx : sms * best_per;
-        out->push_back(LaunchShape{best_t, blocks, std::min(b->team, best_t / 32)});
+        out->push_back(LaunchShape{best_t, blocks, std::min(b->team, best_t / 32), 0, 0, 0});
     }
     return HBG_OK;
+}
+
+// Which classes byte_kernel takes, with which CTA, and the subjects that stay
+// with wordfinder_kernel: those whose positions do not fit its cells.
+void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, int device,
+                std::vector<LaunchShape> *shapes) {
+    hbg_gpu_options std_opt;
+    hbg_default_gpu_options(&std_opt);
+    if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx || b->tuned || b->team > 1 ||
+        b->tile_bytes > 0)
+        return;                                  // the caller chose a launch shape of wordfinder_kernel
+    int optin = 0, sms = 1;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    for (size_t c = 0; c < b->classes.size(); ++c) {
+        const LaunchClass &lc = b->classes[c];
+        LaunchShape &sh = (*shapes)[c];
+        if (!lc.cell || (lc.mode & 1))
+            continue;
+        // one CTA per SM, with as many warps as their tables leave room for
+        int t = hbg::kByteThreads;
+        while (t > 0 && hbg::byte_smem_bytes(lc.cell, t, lc.table_len) > (size_t)optin)
+            t -= 32;
+        if (t < 64)
+            continue;
+        const int32_t cut = lc.cell == 2 ? 0x7ffe - b->host.window : 0xffff;
+        const auto &L = db->sched_len;
+        sh.n_long = (int)(std::partition_point(L.begin(), L.end(), [&](int32_t l) { return l > cut; }) - L.begin());
+        sh.byte_threads = t;
+        sh.byte_blocks = sms;
+    }
 }
 
 void drop_graph(hbg_result *r) {
@@ -436,6 +531,7 @@ void free_result_device(hbg_result *r) {
     dfree_idle(r->d_counters);
     dfree_idle(r->d_tile);
     dfree_idle(r->d_gdiag);
+    dfree_idle(r->d_side);
     dfree_idle(r->d_keys);
     dfree_idle(r->d_vals);
     dfree_idle(r->d_hist);
@@ -450,6 +546,14 @@ void free_result_device(hbg_result *r) {
     }
 }
 
+// Some class or subject of this search goes to wordfinder_kernel.
+bool uses_wordfinder(const hbg_result *r) {
+    for (const LaunchShape &sh : r->shapes)
+        if (sh.byte_threads == 0 || sh.n_long > 0)
+            return true;
+    return false;
+}
+
 // Allocate (or grow) the result's device buffers for capacity cap.
 int prepare_result(hbg_result *r, int64_t cap) {
     const hbg::HostBatch &h = r->batch->host;
@@ -461,19 +565,19 @@ int prepare_result(hbg_result *r, int64_t cap) {
     }
     // a failed allocation below leaves the recorded size at 0, so the next
     // search allocates again instead of using a missing buffer
-    if (r->n_counters < 1 + 6 * nq + ng) {   // first use, or a larger batch
+    if (r->n_counters < 1 + 6 * nq + 2 * ng) {   // first use, or a larger batch
         drop_graph(r);
         dfree(r->d_counters);
         if (r->h_counters)
             cudaFreeHost(r->h_counters);
         r->h_counters = nullptr;
         r->n_counters = 0;
-        CU(dalloc(&r->d_counters, 1 + 6 * nq + ng));
-        CU(cudaMallocHost((void **)&r->h_counters, (1 + 6 * nq + ng) * sizeof(unsigned long long)));
-        r->n_counters = 1 + 6 * nq + ng;
+        CU(dalloc(&r->d_counters, 1 + 6 * nq + 2 * ng));
+        CU(cudaMallocHost((void **)&r->h_counters, (1 + 6 * nq + 2 * ng) * sizeof(unsigned long long)));
+        r->n_counters = 1 + 6 * nq + 2 * ng;
     }
     r->gdiag_len = global_diag_len(h, r->db);
-    if (r->gdiag_len > 0) {
+    if (r->gdiag_len > 0 && uses_wordfinder(r)) {
         const int64_t need = (int64_t)r->blocks * (r->threads / 32) * r->gdiag_len;
         if (need > r->gdiag_entries) {
             drop_graph(r);
@@ -482,6 +586,18 @@ int prepare_result(hbg_result *r, int64_t cap) {
             CU(dalloc(&r->d_gdiag, (size_t)need));
             r->gdiag_entries = need;
         }
+    }
+    int64_t side = 0;
+    for (size_t c = 0; c < r->shapes.size(); ++c)
+        if (r->shapes[c].byte_threads > 0 && r->batch->classes[c].cell == 1)
+            side = std::max<int64_t>(side, (int64_t)r->shapes[c].byte_blocks * (r->shapes[c].byte_threads / 32) *
+                                               r->batch->classes[c].table_len);
+    if (side > r->side_entries) {
+        drop_graph(r);
+        dfree(r->d_side);
+        r->side_entries = 0;
+        CU(dalloc(&r->d_side, (size_t)side));
+        r->side_entries = side;
     }
     if (cap > r->cap) {
         drop_graph(r);
@@ -501,6 +617,37 @@ int prepare_result(hbg_result *r, int64_t cap) {
     return HBG_OK;
 }
 
+// byte_kernel's view of a database and of one launch class of a batch; the
+// caller adds counters, scratch and outputs.
+hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass &lc, const LaunchShape &sh) {
+    hbg::ByteArgs t;
+    memset(&t, 0, sizeof(t));
+    t.db = db->d_letters;
+    t.db_off = db->d_off;
+    t.db_len = db->d_len;
+    t.order = db->d_order;
+    t.sub_lo = sh.n_long;
+    t.n_subj = db->n - sh.n_long;
+    t.groups = b->d_groups;
+    t.group_list = b->d_group_list + lc.first;
+    t.n_list = lc.count;
+    t.packed = b->d_packed;
+    t.entries = b->d_entries;
+    t.pv = b->d_pv;
+    t.letters = b->d_letters;
+    t.ctx_of = b->d_ctx_of;
+    t.contexts = b->d_ctx;
+    t.queries = b->d_queries;
+    t.window = b->host.window;
+    t.table_len = lc.table_len;
+    // the first subjects are the longest: a take of them is at most an eighth
+    // of a warp's share of the letters
+    const int64_t warps = (int64_t)sh.byte_blocks * (sh.byte_threads / 32);
+    t.chunk = (int32_t)std::max<int64_t>(
+        1, std::min<int64_t>(16, db->n_res * lc.count / (8 * warps * std::max<int32_t>(1, db->max_len))));
+    return t;
+}
+
 // Enqueue one search on r->stream: counter resets, the word finder, the
 // ordering pass, the lookup-hit counters and the copy of the counters to
 // pinned host memory.  No host synchronisation, so it can be captured.
@@ -511,7 +658,7 @@ int enqueue_search(hbg_result *r) {
     cudaStream_t st = r->stream;
     CU(cudaMemsetAsync(r->d_counters, 0, r->n_counters * sizeof(unsigned long long), st));
     CU(cudaMemsetAsync(r->d_tile, 0, kMaxLaunchClasses * sizeof(unsigned int), st));
-    if (r->d_gdiag)
+    if (r->d_gdiag && uses_wordfinder(r))
         CU(cudaMemsetAsync(r->d_gdiag, 0, (size_t)r->gdiag_entries * sizeof(uint32_t), st));
 
     hbg::WordFinderArgs a;
@@ -555,11 +702,31 @@ int enqueue_search(hbg_result *r) {
     const unsigned ev_flags =
         cap_status == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     CU(cudaEventRecordWithFlags(r->ev[0], st, ev_flags));
+    int wf_launches = 0;
     if (db->n > 0)   // the caller has run wordfinder_configure (not a stream operation)
         for (size_t c = 0; c < b->classes.size(); ++c) {
             const LaunchClass &lc = b->classes[c];
-            a.tile_subjects = class_tile_subjects(b, db, lc, r->shapes[c].blocks);
-            a.tiles_per_group = (db->n + a.tile_subjects - 1) / a.tile_subjects;
+            const LaunchShape &sh = r->shapes[c];
+            if (sh.byte_threads > 0) {
+                hbg::ByteArgs t = byte_args(db, b, lc, sh);
+                t.next = r->d_counters + 1 + 6 * nq + ng;
+                t.side = r->d_side;
+                t.hsps = a.hsps;
+                t.hsp_count = a.hsp_count;
+                t.hsp_cap = a.hsp_cap;
+                t.q_extended = a.q_extended;
+                t.q_kept = a.q_kept;
+                if (t.n_subj > 0) {
+                    CU(hbg::launch_byte(t, lc.cell, sh.byte_blocks, sh.byte_threads, st));
+                    ++wf_launches;
+                }
+                if (sh.n_long == 0)
+                    continue;
+            }
+            ++wf_launches;
+            a.n_subj = sh.byte_threads > 0 ? sh.n_long : db->n;
+            a.tile_subjects = class_tile_subjects(b, a.n_subj, db, lc, r->shapes[c].blocks);
+            a.tiles_per_group = (a.n_subj + a.tile_subjects - 1) / a.tile_subjects;
             a.team = r->shapes[c].team;
             a.n_list = lc.count;
             a.group_list = b->d_group_list + lc.first;
@@ -593,7 +760,7 @@ int enqueue_search(hbg_result *r) {
     CU(hbg::launch_order(o, st));
     {
         const int bits = o.bits_q + o.bits_s + o.bits_so + o.bits_qo;
-        r->launches = (db->n > 0 ? (int32_t)b->classes.size() : 0) + (hbg::order_max_blocks(r->cap) > 0 ? 3 + 3 * ((bits + 7) / 8) : 0) +
+        r->launches = wf_launches + (hbg::order_max_blocks(r->cap) > 0 ? 3 + 3 * ((bits + 7) / 8) : 0) +
                       (nq > 0 ? 1 : 0);
     }
     CU(hbg::launch_query_hits(db->d_hist, b->d_qcells, (int32_t)nq, r->d_counters + 1 + 2 * nq, st));
@@ -720,7 +887,7 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
     db->device = device;
     DeviceScope ds(db->device);
     auto bail = [&](int code) {
-        dfree(db->d_letters);
+        free_letters(db->d_letters);
         dfree(db->d_off);
         dfree(db->d_len);
         dfree(db->d_order);
@@ -735,12 +902,11 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
             return bail(fail(e_ == cudaErrorMemoryAllocation ? HBG_ERR_NOMEM : HBG_ERR_CUDA, \
                              std::string(#call) + ": " + cudaGetErrorString(e_)));  \
     } while (0)
-    CUB(dalloc(&db->d_letters, (size_t)letters_len));
+    CUB(alloc_letters(&db->d_letters, (size_t)letters_len));
     CUB(dalloc(&db->d_off, (size_t)n));
     CUB(dalloc(&db->d_len, (size_t)n));
     CUB(dalloc(&db->d_order, (size_t)n));
     CUB(dalloc(&db->d_hist, HBG_NUM_CELLS));
-    CUB(cudaMemset(db->d_letters, 0, (size_t)letters_len));
     {
         int code = HBG_OK;
         std::string err = fill(db->d_letters, &code);
@@ -756,6 +922,9 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
     CUB(hbg::launch_db_histogram(db->d_letters, letters_len, db->d_hist, 0));
     CUB(cudaDeviceSynchronize());
 #undef CUB
+    db->sched_len.resize(n);
+    for (int32_t i = 0; i < n; ++i)
+        db->sched_len[i] = len[order[i]];
     db->n = n;
     db->n_res = total;
     db->letters_len = letters_len;
@@ -1017,7 +1186,7 @@ int hbg_db_close(hbg_db *db) {
     if (!db)
         return fail(HBG_ERR_INVALID, "null db");
     DeviceScope ds(db->device);
-    dfree(db->d_letters);
+    free_letters(db->d_letters);
     dfree(db->d_off);
     dfree(db->d_len);
     dfree(db->d_order);
@@ -1177,6 +1346,8 @@ int hbg_batch_create_from_smallbone(const hbg_query *query, const hbg_word_param
                 v.assign(overflow + c.payload.cursor, overflow + c.payload.cursor + c.num_used);
             }
             std::sort(v.begin(), v.end());
+            if (std::adjacent_find(v.begin(), v.end()) != v.end())
+                (*out)->repeated_entries = true;
             for (uint16_t x : v)
                 if ((int32_t)x + HBG_WORD_SIZE > qlen)
                     goto bad;
@@ -1244,6 +1415,7 @@ int hbg_batch_tune(hbg_batch *b, int32_t tile_subjects, int32_t global_tables) {
     if (b->device >= 0)
         return fail(HBG_ERR_STATE, "batch already uploaded: tune before the first search");
     b->tile_subjects = tile_subjects;
+    b->tuned = b->tuned || tile_subjects > 0 || global_tables;
     if (global_tables) {
         hbg::HostBatch &h = b->host;
         for (HbgGroup &G : h.groups) {
@@ -1313,7 +1485,8 @@ int hbg_mem_required(const hbg_db *db, const hbg_batch *b, int64_t cap, int64_t 
         cap = std::max<int64_t>(1 << 20, (int64_t)db->n);
     const hbg::HostBatch &h = b->host;
     int64_t batch_bytes = (int64_t)(h.letters.size() + h.ctx_of.size() * 4 + h.cells.size() * 4 +
-                                    h.entries.size() * 2 + h.pv.size() * 4 + h.query_cells.size() * 2);
+                                    h.entries.size() * 2 + h.pv.size() * 4 + h.query_cells.size() * 2 +
+                                    h.groups.size() * HBG_NUM_CELLS * 4);
     int64_t per_hsp = 2 * (int64_t)sizeof(hbg_hsp) + 2 * 8 + 2 * 4;
     int64_t gdiag = 0;
     if (global_diag_len(h, db) > 0) {
@@ -1366,7 +1539,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     }
     r->opt = o;
     r->stream = (cudaStream_t)stream;
-    if (hbg::wordfinder_configure() != cudaSuccess) {
+    if (hbg::wordfinder_configure() != cudaSuccess || hbg::byte_configure() != cudaSuccess) {
         if (!*out)
             delete r;
         return fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
@@ -1377,6 +1550,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
             delete r;
         return rc;
     }
+    plan_bytes(batch, db, o, db->device, &r->shapes);
     r->shape_opt = o;
     r->blocks = 0;
     r->threads = 32;
@@ -1635,10 +1809,12 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     if (rc != HBG_OK)
         return rc;
     CU(hbg::wordfinder_configure());
+    CU(hbg::byte_configure());
     std::vector<LaunchShape> shapes;   // host-side only; no device allocation
     rc = plan_launches(batch, o, db->device, &shapes);
     if (rc != HBG_OK)
         return rc;
+    plan_bytes(batch, db, o, db->device, &shapes);
     cudaStream_t st = (cudaStream_t)stream;
     unsigned char *base = (unsigned char *)scratch;
     unsigned int *tile = (unsigned int *)base;
@@ -1682,8 +1858,24 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     if (db->n > 0) {
         for (size_t c = 0; c < batch->classes.size(); ++c) {
             const LaunchClass &lc = batch->classes[c];
-            a.tile_subjects = class_tile_subjects(batch, db, lc, shapes[c].blocks);
-            a.tiles_per_group = (db->n + a.tile_subjects - 1) / a.tile_subjects;
+            if (shapes[c].byte_threads > 0) {
+                // 16-bit cells (longer groups are refused above), so no side
+                // table; the group counters serve as subject counters
+                hbg::ByteArgs t = byte_args(db, batch, lc, shapes[c]);
+                t.next = g_hits;
+                t.hsps = a.hsps;
+                t.hsp_count = a.hsp_count;
+                t.hsp_cap = a.hsp_cap;
+                t.q_extended = a.q_extended;
+                t.q_kept = a.q_kept;
+                if (t.n_subj > 0)
+                    CU(hbg::launch_byte(t, lc.cell, shapes[c].byte_blocks, shapes[c].byte_threads, st));
+                if (shapes[c].n_long == 0)
+                    continue;
+            }
+            a.n_subj = shapes[c].byte_threads > 0 ? shapes[c].n_long : db->n;
+            a.tile_subjects = class_tile_subjects(batch, a.n_subj, db, lc, shapes[c].blocks);
+            a.tiles_per_group = (a.n_subj + a.tile_subjects - 1) / a.tile_subjects;
             a.team = shapes[c].team;
             a.n_list = lc.count;
             a.group_list = batch->d_group_list + lc.first;

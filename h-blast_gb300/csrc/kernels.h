@@ -64,6 +64,46 @@ cudaError_t wordfinder_occupancy(int mode, int threads, int smem_diag, int team,
 cudaError_t launch_wordfinder(const WordFinderArgs &a, int mode, int blocks, int threads,
                               cudaStream_t stream);
 
+// The word finder with small diagonal cells in shared memory (bytefinder.cu):
+// the scheduled subjects [sub_lo, sub_lo + n_subj), for the groups of
+// group_list.
+constexpr int kByteThreads = 768;     // largest CTA
+constexpr int kByteMinWindow = 5;     // smallest and largest two-hit window
+constexpr int kByteMaxWindow = 64;
+constexpr int kByteMaxCount = 1023;   // most entries of a cell
+constexpr int kByteMaxEntries = 1 << 22;   // entries of a group are fewer
+struct ByteArgs {
+    const uint8_t *db;
+    const int64_t *db_off;
+    const int32_t *db_len;
+    const int32_t *order;
+    int32_t sub_lo, n_subj;
+    const HbgGroup *groups;
+    const int32_t *group_list;
+    const uint32_t *packed;       // n_groups x HBG_NUM_CELLS: first entry | count << 22
+    const uint16_t *entries;
+    const uint32_t *pv;
+    const uint8_t *letters;
+    const int32_t *ctx_of;
+    const HbgContext *contexts;
+    const HbgQueryDesc *queries;
+    int32_t window;
+    int32_t table_len;            // cells per warp, at least every group's diag_len
+    int32_t n_list;
+    int32_t chunk;                // subjects a warp takes at a time, 1..32
+    unsigned long long *next;     // per group: subjects taken, zeroed before launch
+    uint16_t *side;               // 8-bit cells: blocks x warps x table_len flag ends (need no clearing)
+    hbg_hsp *hsps;
+    unsigned long long *hsp_count;
+    int64_t hsp_cap;
+    unsigned long long *q_extended;
+    unsigned long long *q_kept;
+};
+size_t byte_smem_bytes(int cell_bytes, int threads, int table_len);
+cudaError_t byte_configure();
+cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threads, cudaStream_t stream);
+cudaError_t launch_pack_cells(const uint32_t *cells, int32_t n_groups, uint32_t *packed, cudaStream_t stream);
+
 // Ordering pass: sort HSPs by (query, subject, s_off, q_off).
 struct OrderArgs {
     const hbg_hsp *in;

@@ -1,0 +1,111 @@
+"""The shared-memory word finder at the edges of its ranges: table sizes (16- and
+8-bit cells, and the first lengths past them), two-hit windows, subject lengths
+around its chunks, sweeps and position limits, X-drop extremes, and the batches
+it leaves to the general kernel.  Bit-exact against the CPU oracle (integer
+work, tolerance 0)."""
+import numpy as np
+import pytest
+
+import hblast
+from hblast import synth
+from oracle import oracle
+from test_gpu_parity import check, contexts_query
+from test_host import smallbone_from_csr
+
+pytestmark = pytest.mark.gpu
+
+
+def database(rng, q, extra=()):
+    """Subjects of every length 1..70 and some around a sweep, cut from mutated
+    copies of q, so that they hold hits, and a few of the given lengths."""
+    lens = list(range(1, 71)) + [150, 191, 192, 193, 206, 207, 208, 248, 249, 300, 1000, 3000] + list(extra)
+    subs = []
+    for n in lens:
+        s = synth.random_letters(rng, n)
+        for at in range(0, n, 160):
+            m = min(n - at, 90, len(q))
+            a = int(rng.integers(0, len(q) - m + 1))
+            s[at:at + m] = synth.mutate(rng, q[a:a + m], rng.uniform(0.4, 1.0))
+        subs.append(s)
+    off = np.zeros(len(subs) + 1, np.int64)
+    off[1:] = np.cumsum([len(s) for s in subs])
+    return np.concatenate(subs), off
+
+
+@pytest.mark.parametrize("qlen,window", [(3, 40), (24, 40), (25, 40), (700, 5), (700, 4), (700, 64), (700, 65), (2008, 40),
+                                         (2009, 40), (4056, 40), (4057, 40), (8152, 40), (8152, 7), (8153, 40)])
+def test_table_edges(built, qlen, window):
+    rng = np.random.default_rng(qlen + window)
+    q = synth.random_letters(rng, qlen)
+    res, off = database(rng, q)
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 20)]
+    gdb = hblast.Database(res, off)
+    got = hblast.search(gdb, hblast.Batch.proteins(pqs, window=window))
+    # check() compares with the default window
+    ref, subj, cnt = oracle.search(oracle.Query.blastp(q, 16, 20), res, off, window=window)
+    h = got.hsps
+    assert len(h) == len(ref) and np.array_equal(h["subject"], subj)
+    for f, g in (("q_start", "q_start"), ("s_start", "s_start"), ("q_off", "q_off"), ("s_off", "s_off"),
+                 ("len", "len"), ("score", "score")):
+        assert np.array_equal(h[g], ref[f]), f
+    st = got.stats[0]
+    assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
+
+
+@pytest.mark.parametrize("qlen,lens", [(300, (32725, 32726, 32727, 32766, 40000)), (5000, (32726, 65534, 65535, 65536, 70000))])
+def test_long_subjects(built, qlen, lens):
+    """Subjects at and past the largest position a cell holds: the longer ones
+    go to the general kernel, all in one result."""
+    rng = np.random.default_rng(qlen)
+    q = synth.random_letters(rng, qlen)
+    res, off = database(rng, q, lens)
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 30)]
+    check(hblast.search(hblast.Database(res, off), hblast.Batch.proteins(pqs)), pqs, res, off)
+
+
+def test_many_tiny_subjects_and_repeats(built):
+    """Hundreds of subjects of a few letters in a row (flag codes of the 8-bit
+    cells go round), low-complexity subjects and queries: long chains on one
+    diagonal, blocked hits, cells of about a thousand entries and more."""
+    rng = np.random.default_rng(5)
+    unit = synth.random_letters(rng, 11)
+    q8 = np.concatenate([np.tile(unit, 40), synth.random_letters(rng, 5000)])
+    subs = [q8[a:a + int(rng.integers(3, 9))] for a in rng.integers(0, 5000, 900)]
+    subs += [np.tile(unit, int(rng.integers(2, 30))) for _ in range(60)]
+    subs += [np.full(n, 11, np.uint8) for n in (3, 40, 500)]
+    off = np.zeros(len(subs) + 1, np.int64)
+    off[1:] = np.cumsum([len(s) for s in subs])
+    res = np.concatenate(subs)
+    pqs = [hblast.ProteinQuery.blastp(x, 16, 20) for x in
+           (q8, np.tile(unit, 60), np.full(1000, 11, np.uint8), np.full(1030, 11, np.uint8))]
+    gdb = hblast.Database(res, off)
+    for k, pq in enumerate(pqs):
+        check(hblast.search(gdb, hblast.Batch.proteins([pq])), [pq], res, off)
+
+
+@pytest.mark.parametrize("xdrop", [0, 1, 7, 200])
+def test_xdrop_extremes(built, xdrop):
+    rng = np.random.default_rng(xdrop)
+    parts = [synth.random_letters(rng, n) for n in (40, 300, 5)]
+    pq = contexts_query(parts, [xdrop] * 3, [11, 25, 11])
+    res, off = database(rng, parts[1])
+    check(hblast.search(hblast.Database(res, off), hblast.Batch.proteins([pq])), [pq], res, off)
+
+
+def test_table_with_repeated_offsets(built):
+    """A caller's own table that lists offsets twice: the second hit in one
+    place changes nothing."""
+    rng = np.random.default_rng(9)
+    q = synth.random_letters(rng, 200)
+    res, off = database(rng, q)
+    pq = hblast.ProteinQuery.blastp(q, 16, 20)
+    cs, ents = oracle.lookup_table(oracle.Query.blastp(q, 16, 20), 11)
+
+    def table(rep):
+        return hblast.Batch.from_smallbone(pq, *smallbone_from_csr(cs * rep, np.repeat(ents, rep)))
+
+    gdb = hblast.Database(res, off)
+    one, two = hblast.search(gdb, table(1)), hblast.search(gdb, table(2))
+    assert len(one.hsps) > 0
+    assert np.array_equal(one.hsps, two.hsps)
+    check(one, [pq], res, off)
