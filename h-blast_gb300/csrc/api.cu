@@ -331,15 +331,16 @@ int upload_batch(hbg_batch *b, int device) {
     return rc;
 }
 
-// Longest diagonal tables byte_kernel is used for.  With 16-bit cells a
-// 4096-entry table leaves room for 22 warps per SM (9.2 ms for a 4056-letter
-// query against 400,000 subjects; 8-bit cells, 24 warps: 10.3 ms, the sweeps
-// cut its rounds of extensions short; wordfinder_kernel: 13.9 ms).  At 8192
-// entries 8-bit cells are ahead (8152 letters against 200,000 subjects: 9.5 ms
-// with 22 warps, 12.2 ms with 16-bit cells and 12 warps, wordfinder_kernel
-// 16.1 ms); longer tables leave too few warps.
+// Longest diagonal tables byte_kernel keeps in 16-bit cells: 4096 entries leave
+// room for 22 warps per SM (9.2 ms for a 4056-letter query against 400,000
+// subjects; 8-bit cells, 24 warps: 10.3 ms, the sweeps cut its rounds of
+// extensions short).  Longer tables take 8-bit cells (8152 letters against
+// 200,000 subjects: 9.5 ms, 12.2 ms with 16-bit cells and 12 warps).
 constexpr int kByteTable16 = 4096;
-constexpr int kByteTable8 = 8192;
+// Fewest warps per SM it is used with.  Against 20,000 subjects, ms here and
+// with wordfinder_kernel: 20,000 letters (10 warps) 3.7 / 8.1, 35,000 (6 warps)
+// 9.9 / 18.0, 50,000 (4) 20.6 / 32.3, 64,900 (3, the longest) 35.2 / 45.4.
+constexpr int kByteMinWarps = 2;
 
 // Bytes of a diagonal cell in byte_kernel for a group, 0 when it cannot take
 // the group: its window, table, cell counts or entry count do not fit, or the
@@ -348,13 +349,9 @@ int byte_cell(const hbg_batch *b, int32_t g) {
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
     const uint32_t *cs = h.cells.data() + (size_t)g * HBG_CELL_STRIDE;
-    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.diag_len > kByteTable8 ||
-        cs[HBG_NUM_CELLS] >= (uint32_t)hbg::kByteMaxEntries || b->repeated_entries)
+    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow ||
+        G.max_count > hbg::kByteMaxCount || cs[HBG_NUM_CELLS] >= (uint32_t)hbg::kByteMaxEntries || b->repeated_entries)
         return 0;
-    if (G.glen > hbg::kByteMaxCount)             // a cell has at most one entry per letter
-        for (int w = 0; w < HBG_NUM_CELLS; ++w)
-            if (cs[w + 1] - cs[w] > (uint32_t)hbg::kByteMaxCount)
-                return 0;
     return G.diag_len <= kByteTable16 ? 2 : 1;
 }
 
@@ -403,7 +400,11 @@ int upload_batch_buffers(hbg_batch *b, int device) {
             if (i == 0 || keyed[i].first != keyed[i - 1].first)
                 b->classes.push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
                                                  keyed[i].first[2] & 3, keyed[i].first[2] / 4});
-            b->classes.back().count++;
+            LaunchClass &lc = b->classes.back();
+            lc.count++;
+            if (lc.cell == 1)              // the longest group's exact table
+                lc.table_len = std::max(lc.count == 1 ? 0 : lc.table_len,
+                                        hbg::byte_table_len(h.groups[keyed[i].second].glen + h.window));
             list.push_back(keyed[i].second);
         }
         if ((int)b->classes.size() > kMaxLaunchClasses)
@@ -504,7 +505,7 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
         int t = hbg::kByteThreads;
         while (t > 0 && hbg::byte_smem_bytes(lc.cell, t, lc.table_len) > (size_t)optin)
             t -= 32;
-        if (t < 64)
+        if (t < 32 * kByteMinWarps)
             continue;
         const int32_t cut = lc.cell == 2 ? 0x7ffe - b->host.window : 0xffff;
         const auto &L = db->sched_len;
@@ -1358,6 +1359,7 @@ int hbg_batch_create_from_smallbone(const hbg_query *query, const hbg_word_param
                 v.assign(overflow + c.payload.cursor, overflow + c.payload.cursor + c.num_used);
             }
             std::sort(v.begin(), v.end());
+            h.groups[0].max_count = std::max(h.groups[0].max_count, c.num_used);
             if (std::adjacent_find(v.begin(), v.end()) != v.end())
                 (*out)->repeated_entries = true;
             for (uint16_t x : v)

@@ -17,10 +17,10 @@
 //   to position `end` (NCBI's DiagStruct flag), 0xffff pending.  The table is
 //   cleared when a subject's positions would not fit.
 //
-//   8-bit cells (twice the table in the same memory): positions to 247;
-//   248..254 a flag of the subject with that number modulo 7, its end in a
-//   side table in global memory; 255 pending.  Every ~200 letters `sweep`
-//   moves the base up.
+//   8-bit cells (for longer tables, whose length is then exact instead of a
+//   power of two): positions to 247; 248..254 a flag of the subject with that
+//   number modulo 7, its end in a side table in global memory; 255 pending.
+//   Every ~200 letters `sweep` moves the base up.
 //
 // The rules are NCBI aa_ungapped.c's two-hit state machine (H-BLAST
 // h_blast_kernel.cu:672-871); the extension is in extend.h.
@@ -89,7 +89,7 @@ struct Item {
     const uint8_t *s;        // subject letters
     int S, j;                // its length and ordinal id
     unsigned tab, mem;       // shared-memory offsets of the warp's cells and WarpMem
-    unsigned mask;           // table length - 1
+    unsigned len;            // table length: a power of two for 16-bit cells, exact for 8-bit ones
     unsigned span;           // window - 3
     int rel;                 // position of subject offset 0
     int code;                // 8-bit cells: flag code of this subject
@@ -118,18 +118,36 @@ __device__ __forceinline__ bool is_flag(int v) {
     return (unsigned)(v - Cells<Cell>::kFlag) < (unsigned)(Cells<Cell>::kPending - Cells<Cell>::kFlag);
 }
 
+// A hit's place in the subject as the batches carry it: the offset, for 8-bit
+// cells with the offset modulo the table length in the upper half.  The cell of
+// query offset q is (q - offset) modulo the table length.
+template <typename Cell>
+__device__ __forceinline__ int offset_of(unsigned place) {
+    return (int)(sizeof(Cell) == 1 ? place & 0xffffu : place);
+}
+template <typename Cell>
+__device__ __forceinline__ unsigned place_of(const Item<Cell> &it, int s_h) {
+    return sizeof(Cell) == 1 ? (unsigned)s_h | (((unsigned)s_h % it.len) << 16) : (unsigned)s_h;
+}
+template <typename Cell>
+__device__ __forceinline__ unsigned cell_of(const Item<Cell> &it, unsigned place, int q) {
+    if (sizeof(Cell) == 2)
+        return ((unsigned)q - place) & (it.len - 1u);
+    const unsigned d = (unsigned)q - (place >> 16);
+    return min(d, d + it.len);
+}
+
 // The general case of apply_hits: chains of lanes that share a diagonal, and
 // special states.  A chain's state goes from lane to lane, in order, by
 // shuffles, and its last lane writes the cell.  Chains are found through the
 // cells: every lane writes its number and reads back whose number stayed; who
 // reads another's says so in that lane's word of `chain`.  Warp-collective.
 template <typename Cell>
-__device__ __forceinline__ void apply_chains(const Item<Cell> &it, Queues &W, bool act, int s_h, int q, int v, int &nv,
+__device__ __forceinline__ void apply_chains(const Item<Cell> &it, Queues &W, bool act, unsigned d, int s_h, int q, int v, int &nv,
                                              int &diff, bool &trig) {
     using K = Cells<Cell>;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const unsigned d = (unsigned)(q - s_h) & it.mask;
     const int pos = s_h + it.rel;
     Cell &cell = smem_at<Cell>(it.tab + d * (unsigned)sizeof(Cell));
     if (act)
@@ -197,11 +215,12 @@ __device__ __forceinline__ void apply_chains(const Item<Cell> &it, Queues &W, bo
 // state -- go through apply_chains.  Full: every lane is active.
 // Warp-collective.
 template <bool Full, typename Cell>
-__device__ __forceinline__ void apply_hits(const Item<Cell> &it, Queues &W, bool act, int s_h, int q) {
+__device__ __forceinline__ void apply_hits(const Item<Cell> &it, Queues &W, bool act, unsigned place, int q) {
     using K = Cells<Cell>;
     const int lane = threadIdx.x & 31;
     const unsigned lt = (1u << lane) - 1u;
-    const unsigned d = (unsigned)(q - s_h) & it.mask;
+    const int s_h = offset_of<Cell>(place);
+    const unsigned d = cell_of(it, place, q);
     const int pos = s_h + it.rel;
     Cell &cell = smem_at<Cell>(it.tab + d * (unsigned)sizeof(Cell));
     int v = 0, t = pos;
@@ -224,7 +243,7 @@ __device__ __forceinline__ void apply_hits(const Item<Cell> &it, Queues &W, bool
     const bool hard = v >= K::kFlag ||
                       (shared && ((unsigned)(t - pos + 1) > 2u || trig || (unsigned)(t - v - 3) < it.span));
     if (__any_sync(kAll, hard)) {
-        apply_chains(it, W, Full || act, s_h, q, v, nv, diff, trig);
+        apply_chains(it, W, Full || act, d, s_h, q, v, nv, diff, trig);
     } else if ((Full || act) && (shared ? reset && pos < t : nv != pos)) {
         cell = (Cell)nv;
     }
@@ -280,7 +299,7 @@ __device__ __noinline__ Queues flush(const Item<Cell> it, const ByteArgs &a, Que
                         a.hsps[o] = out;
                     }
                 }
-                const unsigned d = (unsigned)(q - s_h) & it.mask;
+                const unsigned d = cell_of(it, place_of(it, s_h), q);
                 int v = s_h + it.rel;
                 if (e.right) {
                     const int end = e.s_last_off - 2;      // hits before it are passed
@@ -312,7 +331,7 @@ __device__ __noinline__ Queues flush(const Item<Cell> it, const ByteArgs &a, Que
             }
             const bool act = b0 + lane < nb;
             const uint32_t rec = act ? wm.blk[src + b0 + lane] : 0u;
-            apply_hits<false>(it, W, act, (int)(rec & 0xffffu), (int)(rec >> 16));
+            apply_hits<false>(it, W, act, place_of(it, (int)(rec & 0xffffu)), (int)(rec >> 16));
         }
     } while (drain && (W.n_tasks > 0 || W.n_blk > 0));
     return W;
@@ -410,7 +429,9 @@ __device__ __forceinline__ void process_item(Item<Cell> &it, const ByteArgs &a, 
     stage_issue(wm, it.s, it.S, 1, lane);
     int next = 0;
     uint32_t carry = 0;        // hits of earlier chunks not applied yet, in lanes 0..carry-1
-    int s_n = 0, q_n = 0;      // this lane's next hit
+    unsigned s_n = 0;          // this lane's next hit
+    int q_n = 0;
+    unsigned s_mod = 0;        // 8-bit cells: s0 modulo the table length
     // the next chunk's cells are loaded while this chunk's hits are applied,
     // and each batch's query offsets while the previous batch is applied
     uint32_t cell_next = it.S >= 3 ? scan_words(it.s, it.S, next, wm, pv, packed, 0) : 0u;
@@ -424,8 +445,14 @@ __device__ __forceinline__ void process_item(Item<Cell> &it, const ByteArgs &a, 
             if (W.n_tasks > 0 || W.n_blk > 0)
                 W = flush(it, a, W, true);
             const int r = s0 + it.rel - (int)it.span - 3;
-            sweep(it.tab, it.mask + 1, r, it.code);
+            sweep(it.tab, it.len, r, it.code);
             it.rel -= r;
+        }
+        unsigned place = (unsigned)(s0 + lane);
+        if (sizeof(Cell) == 1) {
+            const unsigned m = s_mod + lane;
+            place |= (m >= it.len ? m - it.len : m) << 16;
+            s_mod = s_mod + 32 >= it.len ? s_mod + 32 - it.len : s_mod + 32;
         }
         const uint32_t cell = cell_next;
         if (s0 + 32 <= it.S - 3)
@@ -447,7 +474,7 @@ __device__ __forceinline__ void process_item(Item<Cell> &it, const ByteArgs &a, 
         __syncwarp();              // the previous chunk's list has been read
         if (c != 0)
             smem_at<uint2>(list + 8u * (unsigned)__popc(nz & (le >> 1))) =
-                make_uint2((unsigned)(s0 + lane), (cell & 0x3fffffu) - start);
+                make_uint2(place, (cell & 0x3fffffu) - start);
         else
             start = 0x80000000u;   // starts nothing
         __syncwarp();
@@ -463,24 +490,25 @@ __device__ __forceinline__ void process_item(Item<Cell> &it, const ByteArgs &a, 
             const unsigned m = starts(0);
             if ((uint32_t)lane >= carry && (uint32_t)lane < total) {
                 const uint2 e = smem_at<uint2>(before + 8u * (unsigned)__popc(m & le));
-                s_n = (int)e.x;
+                s_n = e.x;
                 q_n = (int)__ldg(ents + (e.y + lane));
             }
             before += 8u * (unsigned)__popc(m);
         }
         uint32_t cb = 0;
         for (; cb + 32 <= total; cb += 32) {       // full batches
-            const int s_h = s_n, q = q_n;
+            const unsigned at = s_n;
+            const int q = q_n;
             {
                 // lanes past the last hit read entries past its cell (the
                 // entries end with padding); they are not applied
                 const unsigned m = starts(cb + 32);
                 const uint2 e = smem_at<uint2>(before + 8u * (unsigned)__popc(m & le));
-                s_n = (int)e.x;
+                s_n = e.x;
                 q_n = (int)__ldg(ents + (e.y + cb + 32 + lane));
                 before += 8u * (unsigned)__popc(m);
             }
-            apply_hits<true>(it, W, true, s_h, q);
+            apply_hits<true>(it, W, true, at, q);
             if (W.n_tasks >= kFlushAt || W.n_blk >= 32) {
                 do                                 // keep room for one more batch
                     W = flush(it, a, W, false);
@@ -539,6 +567,7 @@ __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
         const HbgGroup G = a.groups[g];
         const uint32_t *packed = a.packed + (size_t)g * HBG_NUM_CELLS;
         const uint16_t *ents = a.entries + G.entry_base;
+        const unsigned len = sizeof(Cell) == 2 ? (unsigned)G.diag_len : (unsigned)byte_table_len(G.glen + window);
         // lane k holds the k-th subject of the warp's chunk
         const uint8_t *ds = nullptr;
         int dS = 0, dj = 0, ck = 0, cc = 0;
@@ -573,13 +602,13 @@ __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
                 code = code == K::kPending - 1 ? K::kFlag : code + 1;
                 if (++since >= K::kPending - K::kFlag - 1 || rel > K::kMaxPos) {
                     // the flag codes run out (subjects of a few letters), or the positions
-                    sweep(tab, a.table_len, rel - window, code);
+                    sweep(tab, (int)len, rel - window, code);
                     rel = window;
                     since = 0;
                 }
             }
             Item<Cell> it{(const uint8_t *)(uintptr_t)__shfl_sync(kAll, (unsigned long long)(uintptr_t)ds, ck), S,
-                          __shfl_sync(kAll, dj, ck), tab, mem, (unsigned)G.diag_len - 1u, (unsigned)window - 3u, rel, code, side,
+                          __shfl_sync(kAll, dj, ck), tab, mem, len, (unsigned)window - 3u, rel, code, side,
                           a.letters + G.seq_base, a.ctx_of + G.seq_base, G.first_query};
             process_item(it, a, hd.pv, packed, ents);
             top = S + it.rel;

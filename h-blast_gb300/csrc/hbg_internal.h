@@ -29,6 +29,8 @@ struct HbgGroup {
     int32_t n_queries;
     int32_t placement;    // 0: diagonal table in shared memory, 1: global scratch
     int32_t mode;         // 0: chunk mode (sparse hits), 1: offset mode (dense hits)
+    int32_t max_count;    // entries of the fullest cell
+    int32_t pad;
 };
 
 struct HbgContext {

@@ -88,7 +88,7 @@ struct ByteArgs {
     const HbgContext *contexts;
     const HbgQueryDesc *queries;
     int32_t window;
-    int32_t table_len;            // cells per warp, at least every group's diag_len
+    int32_t table_len;            // cells per warp: diag_len, for 8-bit cells the longest group's byte_table_len
     int32_t n_list;
     int32_t chunk;                // subjects a warp takes at a time, 1..32
     unsigned long long *next;     // per group: subjects taken, zeroed before launch
@@ -99,6 +99,8 @@ struct ByteArgs {
     unsigned long long *q_extended;
     unsigned long long *q_kept;
 };
+// length of an 8-bit table for a group of `letters` letters and gap
+__host__ __device__ constexpr int byte_table_len(int letters) { return (letters + 127) / 128 * 128; }
 size_t byte_smem_bytes(int cell_bytes, int threads, int table_len);
 cudaError_t byte_configure();
 cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threads, cudaStream_t stream);

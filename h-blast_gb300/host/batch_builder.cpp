@@ -300,15 +300,17 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
         }
         uint32_t *cs = b.cells.data() + (size_t)g * HBG_CELL_STRIDE;
         uint32_t *pv = b.pv.data() + (size_t)g * HBG_PV_WORDS;
-        uint32_t acc = 0;
+        uint32_t acc = 0, most = 0;
         for (int32_t w = 0; w < HBG_NUM_CELLS; ++w) {
             cs[w] = acc;
             acc += count[w];
+            most = std::max(most, count[w]);
             if (count[w])
                 pv[w >> 5] |= 1u << (w & 31);
         }
         cs[HBG_NUM_CELLS] = acc;
         group_entries[g] = acc;
+        G.max_count = (int32_t)most;
         // expected hits per subject offset on typical proteins: entries of
         // words over the 20 standard letters, each such word taken as
         // equally likely (1 / 8000)

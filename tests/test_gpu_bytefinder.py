@@ -1,5 +1,5 @@
 """The shared-memory word finder at the edges of its ranges: table sizes (16- and
-8-bit cells, and the first lengths past them), two-hit windows, subject lengths
+8-bit cells, up to the longest query), two-hit windows, subject lengths
 around its chunks, sweeps and position limits, X-drop extremes, and the batches
 it leaves to the general kernel.  Bit-exact against the CPU oracle (integer
 work, tolerance 0)."""
@@ -33,7 +33,8 @@ def database(rng, q, extra=()):
 
 
 @pytest.mark.parametrize("qlen,window", [(3, 40), (24, 40), (25, 40), (700, 5), (700, 4), (700, 64), (700, 65), (2008, 40),
-                                         (2009, 40), (4056, 40), (4057, 40), (8152, 40), (8152, 7), (8153, 40)])
+                                         (2009, 40), (4056, 40), (4057, 40), (8152, 40), (8152, 7), (8153, 40), (16341, 40),
+                                         (16345, 64), (33000, 40), (65000, 64)])
 def test_table_edges(built, qlen, window):
     rng = np.random.default_rng(qlen + window)
     q = synth.random_letters(rng, qlen)
