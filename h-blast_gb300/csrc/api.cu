@@ -566,16 +566,16 @@ int prepare_result(hbg_result *r, int64_t cap) {
     }
     // a failed allocation below leaves the recorded size at 0, so the next
     // search allocates again instead of using a missing buffer
-    if (r->n_counters < 1 + 6 * nq + 2 * ng) {   // first use, or a larger batch
+    if (r->n_counters < 3 + 6 * nq + 2 * ng) {   // first use, or a larger batch
         drop_graph(r);
         dfree(r->d_counters);
         if (r->h_counters)
             cudaFreeHost(r->h_counters);
         r->h_counters = nullptr;
         r->n_counters = 0;
-        CU(dalloc(&r->d_counters, 1 + 6 * nq + 2 * ng));
-        CU(cudaMallocHost((void **)&r->h_counters, (1 + 6 * nq + 2 * ng) * sizeof(unsigned long long)));
-        r->n_counters = 1 + 6 * nq + 2 * ng;
+        CU(dalloc(&r->d_counters, 3 + 6 * nq + 2 * ng));
+        CU(cudaMallocHost((void **)&r->h_counters, (3 + 6 * nq + 2 * ng) * sizeof(unsigned long long)));
+        r->n_counters = 3 + 6 * nq + 2 * ng;
     }
     r->gdiag_len = global_diag_len(h, r->db);
     if (r->gdiag_len > 0 && uses_wordfinder(r)) {
@@ -612,7 +612,7 @@ int prepare_result(hbg_result *r, int64_t cap) {
         CU(dalloc(&r->d_sorted, (size_t)cap));
         CU(dalloc(&r->d_keys, (size_t)cap * 2));
         CU(dalloc(&r->d_vals, (size_t)cap * 2));
-        CU(dalloc(&r->d_hist, (size_t)(256 * hbg::order_max_blocks(cap) + 1)));
+        CU(dalloc(&r->d_hist, (size_t)256 * hbg::kOrderMaxGrid));
         r->cap = cap;
     }
     return HBG_OK;
@@ -770,13 +770,14 @@ int enqueue_search(hbg_result *r) {
     o.q_passed = o.q_end + nq;
     if (o.bits_q + o.bits_s + o.bits_so + o.bits_qo > 64)
         return fail(HBG_ERR_TOO_LONG, "ordering key exceeds 64 bits for this database and batch");
-    CU(hbg::launch_order(o, st));
-    {
-        const int bits = o.bits_q + o.bits_s + o.bits_so + o.bits_qo;
-        r->launches = wf_launches + (hbg::order_max_blocks(r->cap) > 0 ? 3 + 3 * ((bits + 7) / 8) : 0) +
-                      (nq > 0 ? 1 : 0);
-    }
-    CU(hbg::launch_query_hits(db->d_hist, b->d_qcells, (int32_t)nq, r->d_counters + 1 + 2 * nq, st));
+    o.barrier = r->d_counters + 1 + 6 * nq + 2 * ng;
+    o.error = o.barrier + 1;
+    o.db_hist = db->d_hist;
+    o.query_cells = b->d_qcells;
+    o.n_queries = (int32_t)nq;
+    o.lookup_hits = r->d_counters + 1 + 2 * nq;
+    CU(hbg::launch_order(o, hbg::order_grid(r->device), st));
+    r->launches = wf_launches + 1;
     CU(cudaEventRecordWithFlags(r->ev[2], st, ev_flags));
     CU(cudaMemcpyAsync(r->h_counters, r->d_counters, r->n_counters * sizeof(unsigned long long),
                        cudaMemcpyDeviceToHost, st));
@@ -1619,6 +1620,13 @@ int hbg_result_sync(hbg_result *r) {
         n = r->h_counters[0];
         if ((int64_t)n > r->cap)
             return fail(HBG_ERR_STATE, "HSP count changed between identical launches");
+    }
+    {
+        const size_t nq = r->batch->host.queries.size(), ng = r->batch->host.groups.size();
+        if (r->h_counters[2 + 6 * nq + 2 * ng]) {   // a result may be launched again
+            r->launched = false;
+            return fail(HBG_ERR_CUDA, "the ordering pass gave up waiting for its own blocks");
+        }
     }
     r->n_hsps = (int64_t)n;
     CU(cudaEventElapsedTime(&r->wf_ms, r->ev[0], r->ev[1]));

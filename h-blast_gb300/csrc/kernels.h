@@ -106,7 +106,9 @@ cudaError_t byte_configure();
 cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threads, cudaStream_t stream);
 cudaError_t launch_pack_cells(const uint32_t *cells, int32_t n_groups, uint32_t *packed, cudaStream_t stream);
 
-// Ordering pass: sort HSPs by (query, subject, s_off, q_off).
+// Ordering pass: sort HSPs by (query, subject, subject offset, query offset),
+// and count the lookup hits of every query.
+constexpr int kOrderMaxGrid = 512;    // most CTAs of the pass
 struct OrderArgs {
     const hbg_hsp *in;
     hbg_hsp *out;
@@ -114,24 +116,25 @@ struct OrderArgs {
     int64_t cap;
     uint64_t *keys[2];
     uint32_t *vals[2];
-    uint32_t *hist;                   // 256 x max_blocks
+    uint32_t *hist;                   // 256 x kOrderMaxGrid
     int bits_q, bits_s, bits_so, bits_qo;
     // optional (null = skip): per-query first / end index in `out` and the
     // number of subjects with HSPs, each n_queries entries, zeroed beforehand
     unsigned long long *q_first, *q_end, *q_passed;
+    unsigned long long *barrier, *error;   // zeroed beforehand; *error: the grid barrier gave up
+    // lookup_hits[q] = sum_w db_hist[w] * query_cells[q][w]
+    const unsigned long long *db_hist;
+    const uint16_t *query_cells;
+    int32_t n_queries;
+    unsigned long long *lookup_hits;
 };
-int64_t order_max_blocks(int64_t cap);
-cudaError_t launch_order(const OrderArgs &a, cudaStream_t stream);
+int order_grid(int device);
+cudaError_t launch_order(const OrderArgs &a, int grid, cudaStream_t stream);
 
 // Database word histogram: hist[w] += positions whose three letters are
 // non-sentinel and form word w.
 cudaError_t launch_db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist,
                                 cudaStream_t stream);
-
-// lookup_hits[q] = sum_w hist[w] * query_cells[q][w]
-cudaError_t launch_query_hits(const unsigned long long *hist, const uint16_t *query_cells,
-                              int32_t n_queries, unsigned long long *out,
-                              cudaStream_t stream);
 
 }  // namespace hbg
 

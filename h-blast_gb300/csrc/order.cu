@@ -1,13 +1,16 @@
 // order.cu -- the ordering pass and the database/lookup-hit counters.
 //
 // The word finder appends HSPs in whatever order warps finish; H-BLAST fixes
-// its order on the host (memory_defrag, h_blast.cu:1160-1208).  Here a stable
-// LSD radix sort on the device orders them by (query, subject, subject
-// offset, query offset) -- per query and subject, the order in which NCBI's
-// CPU word finder creates them (NF/blast_engine.c:553-576 feeds that list to
-// BlastSaveInitHsp) -- and a gather writes the ordered records.  All sizes are
-// read from device memory, so the pass needs no host round trip.
+// its order on the host (memory_defrag, h_blast.cu:1160-1208).  Here one
+// cooperative kernel orders them by (query, subject, subject offset, query
+// offset) -- per query and subject, the order in which NCBI's CPU word finder
+// creates them (NF/blast_engine.c:553-576 feeds that list to BlastSaveInitHsp)
+// -- writes the ordered records and the per-query ranges, and counts the lookup
+// hits.  All sizes are read from device memory, so the pass needs no host round
+// trip.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "kernels.h"
 
@@ -15,14 +18,15 @@ namespace hbg {
 
 namespace {
 
-constexpr int kSortThreads = 256;          // one thread per digit value
-constexpr int kSortItems = 16;             // per thread per tile
-constexpr int kSortTile = kSortThreads * kSortItems;
-
-__device__ __forceinline__ int64_t live_count(const unsigned long long *count, int64_t cap) {
-    unsigned long long n = *count;
-    return (int64_t)(n < (unsigned long long)cap ? n : (unsigned long long)cap);
-}
+constexpr unsigned kAll = 0xffffffffu;
+constexpr int kOrderThreads = 1024;
+constexpr int kWarps = kOrderThreads / 32;
+// Up to this many HSPs every one is ranked against all others.
+constexpr int kRankMax = 4096;
+constexpr int kItems = 8;                     // per thread and scatter round
+constexpr int kRound = kOrderThreads * kItems;
+constexpr int kPart = 1024;                   // fewest items worth a CTA of the radix sort (8192: 130 us for 16,000, 1024: 73)
+constexpr int kSpinLimit = 1 << 22;           // polls of the grid barrier before it gives up
 
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned r;
@@ -30,170 +34,292 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return r;
 }
 
-__global__ void make_keys(const hbg_hsp *in, const unsigned long long *count, int64_t cap,
-                          uint64_t *keys, uint32_t *vals, int bs, int bso, int bqo) {
-    const int64_t n = live_count(count, cap);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const hbg_hsp h = in[i];
-        uint64_t k = (uint64_t)(uint32_t)h.query;
-        k = (k << bs) | (uint64_t)(uint32_t)h.subject;
-        k = (k << bso) | (uint64_t)(uint32_t)h.s_off;
-        k = (k << bqo) | (uint64_t)(uint32_t)h.q_off;
-        keys[i] = k;
-        vals[i] = (uint32_t)i;
-    }
+struct OrderSmem {
+    union {
+        uint64_t keys[kRankMax];
+        struct {
+            uint32_t cnt[kWarps][256];        // items of a digit in a warp, then before it in the round
+            uint32_t before[4][256], total[4][256];
+        } r;
+    };
+    uint32_t base[256];                       // next place of a digit's items of this CTA
+    uint32_t scan[8];
+    int ok;
+};
+
+__device__ __forceinline__ uint64_t key_of(const OrderArgs &a, const hbg_hsp &h) {
+    uint64_t k = (uint64_t)(uint32_t)h.query;
+    k = (k << a.bits_s) | (uint64_t)(uint32_t)h.subject;
+    k = (k << a.bits_so) | (uint64_t)(uint32_t)h.s_off;
+    return (k << a.bits_qo) | (uint64_t)(uint32_t)h.q_off;
 }
 
-// Per-tile digit histogram, stored digit-major: hist[d * nblk + b].
-__global__ void __launch_bounds__(kSortThreads)
-sort_histogram(const uint64_t *keys, const unsigned long long *count, int64_t cap, int shift,
-               uint32_t *hist) {
-    __shared__ uint32_t h[256];
-    const int64_t n = live_count(count, cap);
-    const int64_t nblk = (n + kSortTile - 1) / kSortTile;
-    if (blockIdx.x >= nblk)
-        return;
-    h[threadIdx.x] = 0;
+// Every one of the first `grid` CTAs of the (cooperative) grid arrives before any leaves.  A wait that
+// exceeds its limit reports through *error and the kernel ends.
+__device__ bool grid_barrier(const OrderArgs &a, OrderSmem &sm, int grid, unsigned long long &target) {
+    target += grid;
+    __threadfence();
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    for (int r = 0; r < kSortItems; ++r) {
-        const int64_t i = base + (int64_t)r * kSortThreads + threadIdx.x;
-        if (i < n)
-            atomicAdd(&h[(keys[i] >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    hist[(int64_t)threadIdx.x * nblk + blockIdx.x] = h[threadIdx.x];
-}
-
-// Exclusive scan of the 256 x nblk histogram in place (one CTA).
-__global__ void __launch_bounds__(1024)
-sort_scan(const unsigned long long *count, int64_t cap, uint32_t *hist) {
-    __shared__ uint32_t part[1024];
-    const int64_t n = live_count(count, cap);
-    const int64_t nblk = (n + kSortTile - 1) / kSortTile;
-    const int64_t total = nblk * 256;
-    if (total == 0)
-        return;
-    const int64_t per = (total + blockDim.x - 1) / blockDim.x;
-    const int64_t b0 = threadIdx.x * per;
-    const int64_t b1 = b0 + per < total ? b0 + per : total;
-    uint32_t sum = 0;
-    for (int64_t i = b0; i < b1; ++i)
-        sum += hist[i];
-    part[threadIdx.x] = sum;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        uint32_t t = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0;
-        __syncthreads();
-        part[threadIdx.x] += t;
-        __syncthreads();
-    }
-    uint32_t run = part[threadIdx.x] - sum;
-    for (int64_t i = b0; i < b1; ++i) {
-        uint32_t v = hist[i];
-        hist[i] = run;
-        run += v;
-    }
-}
-
-// Stable scatter of one tile: elements keep their input order among equal
-// digits (round-major, then warp, then lane).
-__global__ void __launch_bounds__(kSortThreads)
-sort_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout, uint32_t *vout,
-             const unsigned long long *count, int64_t cap, int shift, const uint32_t *hist) {
-    __shared__ uint32_t cnt[kSortThreads / 32][256];
-    __shared__ uint32_t pre[kSortThreads / 32][256];
-    __shared__ uint32_t run[256];
-    __shared__ uint32_t rbase[256];
-    __shared__ uint32_t gofs[256];
-    const int64_t n = live_count(count, cap);
-    const int64_t nblk = (n + kSortTile - 1) / kSortTile;
-    if (blockIdx.x >= nblk)
-        return;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    run[t] = 0;
-    gofs[t] = hist[(int64_t)t * nblk + blockIdx.x];
-    for (int w = 0; w < kSortThreads / 32; ++w)
-        cnt[w][t] = 0;
-    __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    for (int r = 0; r < kSortItems; ++r) {
-        const int64_t i = base + (int64_t)r * kSortThreads + t;
-        const bool valid = i < n;
-        uint64_t k = 0;
-        uint32_t v = 0;
-        int dig = 256 + lane;  // unique non-digit for invalid lanes
-        if (valid) {
-            k = kin[i];
-            v = vin[i];
-            dig = (int)((k >> shift) & 255u);
+    if (threadIdx.x == 0) {
+        sm.ok = 1;
+        atomicAdd(a.barrier, 1ull);
+        int polls = 0;
+        unsigned long long seen;
+        do {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(a.barrier) : "memory");
+        } while (seen < target && ++polls < kSpinLimit);
+        if (seen < target) {
+            sm.ok = 0;
+            atomicExch(a.error, 1ull);
         }
-        const unsigned m = __match_any_sync(0xffffffffu, dig);
-        const int rank = __popc(m & lanemask_lt());
-        if (valid && rank == 0)
-            cnt[warp][dig] = __popc(m);
-        __syncthreads();
-        {
-            uint32_t acc = 0;
-            for (int w = 0; w < kSortThreads / 32; ++w) {
-                pre[w][t] = acc;
-                acc += cnt[w][t];
-                cnt[w][t] = 0;
-            }
-            rbase[t] = run[t];
-            run[t] += acc;
-        }
-        __syncthreads();
-        if (valid) {
-            const uint32_t pos = gofs[dig] + rbase[dig] + pre[warp][dig] + (uint32_t)rank;
-            kout[pos] = k;
-            vout[pos] = v;
-        }
-        __syncthreads();
     }
+    __syncthreads();
+    __threadfence();
+    return sm.ok != 0;
 }
 
-__global__ void gather_hsps(const hbg_hsp *in, const uint32_t *vals,
-                            const unsigned long long *count, int64_t cap, hbg_hsp *out) {
-    const int64_t n = live_count(count, cap);
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = in[vals[i]];
-}
-
-// Per-query ranges of the ordered list (sorted by query, then subject):
-// first[q] and end[q] bound query q's HSPs, passed[q] counts its subjects
-// with at least one HSP.  All three start at zero.  Whole warps step
-// together (warp-uniform loop) so the subject counts can be summed per warp
-// and query before the atomic: the list is sorted, so a warp's lanes mostly
-// share one query.
-__global__ void query_ranges(const hbg_hsp *sorted, const unsigned long long *count, int64_t cap,
-                             unsigned long long *first, unsigned long long *end,
-                             unsigned long long *passed) {
-    const int64_t n = live_count(count, cap);
+// One HSP's place among all n <= kRankMax is the number of smaller keys; keys
+// are distinct (a second hit starts one extension).  The same count for the
+// bounds of its query and of its subject tells whether it is the first or last
+// of them.
+__device__ void rank_all(const OrderArgs &a, OrderSmem &sm, int n) {
     const int lane = threadIdx.x & 31;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x - lane); base < n; base += stride) {
-        const int64_t i = base + lane;
-        const bool valid = i < n;
-        int32_t q = -1;
-        bool fresh = false;
-        if (valid) {
-            q = sorted[i].query;
-            const int32_t s = sorted[i].subject;
-            const bool new_q = i == 0 || sorted[i - 1].query != q;
-            if (new_q)
-                first[q] = (unsigned long long)i;
-            if (i == n - 1 || sorted[i + 1].query != q)
-                end[q] = (unsigned long long)(i + 1);
-            fresh = new_q || sorted[i - 1].subject != s;
+    if ((int)blockIdx.x * kWarps >= n)
+        return;
+    for (int i = threadIdx.x; i < n; i += kOrderThreads)
+        sm.keys[i] = key_of(a, a.in[i]);
+    __syncthreads();
+    const int shift_s = a.bits_so + a.bits_qo, shift_q = shift_s + a.bits_s;
+    for (int i = blockIdx.x * kWarps + (threadIdx.x >> 5); i < n; i += gridDim.x * kWarps) {
+        const uint64_t key = sm.keys[i];
+        // smallest and largest key of this query (one query: its key has no bits)
+        const uint64_t q0 = a.bits_q ? (key >> shift_q) << shift_q : 0ull;
+        const uint64_t q1 = a.bits_q ? q0 | ((1ull << shift_q) - 1ull) : ~0ull;
+        const uint64_t s0 = (key >> shift_s) << shift_s;
+        int below = 0, below_q = 0, upto_q = 0, below_s = 0;
+        for (int j = lane; j < n; j += 32) {
+            const uint64_t k = sm.keys[j];
+            below += k < key;
+            below_q += k < q0;
+            upto_q += k <= q1;
+            below_s += k < s0;
         }
-        const unsigned same = __match_any_sync(0xffffffffu, q);
-        const unsigned cnt = __popc(__ballot_sync(0xffffffffu, fresh) & same);
-        if (valid && cnt && lane == __ffs(same) - 1)
-            atomicAdd(passed + q, (unsigned long long)cnt);
+        below = __reduce_add_sync(kAll, below);
+        below_q = __reduce_add_sync(kAll, below_q);
+        upto_q = __reduce_add_sync(kAll, upto_q);
+        below_s = __reduce_add_sync(kAll, below_s);
+        const int32_t *src = reinterpret_cast<const int32_t *>(a.in + i);
+        int32_t *dst = reinterpret_cast<int32_t *>(a.out + below);
+        if (lane < (int)(sizeof(hbg_hsp) / 4))
+            dst[lane] = src[lane];
+        if (a.q_first && lane == 0) {
+            const int q = a.in[i].query;
+            if (below == below_q)
+                a.q_first[q] = (unsigned long long)below;
+            if (below + 1 == upto_q)
+                a.q_end[q] = (unsigned long long)upto_q;
+            if (below == below_s)
+                atomicAdd(a.q_passed + q, 1ull);
+        }
     }
+}
+
+// Stable LSD radix sort, 8 bits a pass, over the key bits in use.  Each CTA
+// owns a contiguous part of the items; a pass is a digit count per CTA, a grid
+// barrier, the CTA's places from all counts, and the scatter.
+__device__ void radix_all(const OrderArgs &a, OrderSmem &sm, int64_t n) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int grid = (int)min((int64_t)gridDim.x, (n + kPart - 1) / kPart);
+    if ((int)blockIdx.x >= grid)
+        return;
+    const int64_t part = (n + grid - 1) / grid;
+    const int64_t lo = min(n, part * (int64_t)blockIdx.x), hi = min(n, lo + part);
+    const int bits = a.bits_q + a.bits_s + a.bits_so + a.bits_qo;
+    unsigned long long target = 0;
+    for (int64_t i = lo + t; i < hi; i += kOrderThreads) {
+        a.keys[0][i] = key_of(a, a.in[i]);
+        a.vals[0][i] = (uint32_t)i;
+    }
+    int src = 0;
+    for (int shift = 0; shift < bits; shift += 8) {
+        const uint64_t *kin = a.keys[src];
+        const uint32_t *vin = a.vals[src];
+        if (t < 256)
+            sm.base[t] = 0;
+        __syncthreads();               // (also: this CTA's first keys are written)
+        for (int64_t i0 = lo; i0 < hi; i0 += kOrderThreads) {
+            const int64_t i = i0 + t;
+            const int dig = i < hi ? (int)((__ldcg(kin + i) >> shift) & 255u) : 256 + lane;
+            const unsigned m = __match_any_sync(kAll, dig);
+            if (dig < 256 && (m & lanemask_lt()) == 0)
+                atomicAdd(&sm.base[dig], (uint32_t)__popc(m));
+        }
+        __syncthreads();
+        if (t < 256)
+            a.hist[blockIdx.x * 256 + t] = sm.base[t];
+        if (!grid_barrier(a, sm, grid, target))
+            return;
+        {
+            // places of this CTA's items of digit d: after all items of smaller
+            // digits and after those of digit d in earlier CTAs
+            const int d = t & 255, quarter = t >> 8;
+            uint32_t before = 0, total = 0;
+            for (int c = quarter; c < grid; c += 4) {
+                const uint32_t x = __ldcg(a.hist + c * 256 + d);
+                total += x;
+                before += c < (int)blockIdx.x ? x : 0u;
+            }
+            sm.r.before[quarter][d] = before;
+            sm.r.total[quarter][d] = total;
+            __syncthreads();
+            uint32_t tot = 0, bef = 0, incl = 0;
+            if (t < 256) {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    tot += sm.r.total[k][t];
+                    bef += sm.r.before[k][t];
+                }
+                incl = tot;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t x = __shfl_up_sync(kAll, incl, o);
+                    if (lane >= o)
+                        incl += x;
+                }
+                if (lane == 31)
+                    sm.scan[warp] = incl;
+            }
+            __syncthreads();
+            if (t < 256) {
+                uint32_t x = incl - tot + bef;
+                for (int k = 0; k < warp; ++k)
+                    x += sm.scan[k];
+                sm.base[t] = x;
+            }
+        }
+        uint64_t *kout = a.keys[src ^ 1];
+        uint32_t *vout = a.vals[src ^ 1];
+        for (int64_t r0 = lo; r0 < hi; r0 += kRound) {
+            for (int i = t; i < kWarps * 256; i += kOrderThreads)
+                (&sm.r.cnt[0][0])[i] = 0;
+            __syncthreads();
+            uint64_t key[kItems];
+            uint32_t val[kItems], rank[kItems];
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                const int64_t i = r0 + (warp * kItems + k) * 32 + lane;
+                const bool on = i < hi;
+                key[k] = on ? __ldcg(kin + i) : 0;
+                val[k] = on ? __ldcg(vin + i) : 0;
+                const int dig = on ? (int)((key[k] >> shift) & 255u) : 256 + lane;
+                const unsigned m = __match_any_sync(kAll, dig);
+                const unsigned below = m & lanemask_lt();
+                rank[k] = on ? sm.r.cnt[warp][dig] + (uint32_t)__popc(below) : 0xffffffffu;
+                __syncwarp();
+                if (on && below == 0)
+                    sm.r.cnt[warp][dig] += (uint32_t)__popc(m);
+                __syncwarp();
+            }
+            __syncthreads();
+            if (t < 256) {
+                uint32_t acc = sm.base[t];
+#pragma unroll 4
+                for (int w = 0; w < kWarps; ++w) {
+                    const uint32_t x = sm.r.cnt[w][t];
+                    sm.r.cnt[w][t] = acc;
+                    acc += x;
+                }
+                sm.base[t] = acc;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kItems; ++k)
+                if (rank[k] != 0xffffffffu) {
+                    const uint32_t pos = sm.r.cnt[warp][(key[k] >> shift) & 255u] + rank[k];
+                    kout[pos] = key[k];
+                    vout[pos] = val[k];
+                }
+            __syncthreads();
+        }
+        if (!grid_barrier(a, sm, grid, target))
+            return;
+        src ^= 1;
+    }
+    // the ordered records, and per query the range of its HSPs and the number
+    // of subjects with at least one; whole warps step together, so that the
+    // subject counts are summed per warp and query before the atomic
+    const uint64_t *keys = a.keys[src];
+    const uint32_t *vals = a.vals[src];
+    const int shift_s = a.bits_so + a.bits_qo, shift_q = shift_s + a.bits_s;
+    auto query_of = [&](uint64_t key) { return a.bits_q ? (int)(key >> shift_q) : 0; };
+    for (int64_t i0 = lo; i0 < hi; i0 += kOrderThreads) {
+        const int64_t i = i0 + t;
+        const bool on = i < hi;
+        int q = -1;
+        bool fresh = false;
+        if (on) {
+            const uint64_t key = __ldcg(keys + i);
+            const uint64_t prev = i > 0 ? __ldcg(keys + i - 1) : 0, next = i + 1 < n ? __ldcg(keys + i + 1) : 0;
+            a.out[i] = a.in[__ldcg(vals + i)];
+            q = query_of(key);
+            const bool new_q = i == 0 || query_of(prev) != q;
+            if (a.q_first) {
+                if (new_q)
+                    a.q_first[q] = (unsigned long long)i;
+                if (i == n - 1 || query_of(next) != q)
+                    a.q_end[q] = (unsigned long long)(i + 1);
+            }
+            fresh = new_q || (prev >> shift_s) != (key >> shift_s);
+        }
+        if (a.q_first) {
+            const unsigned same = __match_any_sync(kAll, q);
+            const unsigned cnt = __popc(__ballot_sync(kAll, fresh) & same);
+            if (on && cnt && lane == __ffs(same) - 1)
+                atomicAdd(a.q_passed + q, (unsigned long long)cnt);
+        }
+    }
+}
+
+// Lookup hits of a query: database count of each word times the entries the
+// query has in its cell.
+__device__ void count_hits(const OrderArgs &a, OrderSmem &sm) {
+    for (int q = blockIdx.x; q < a.n_queries; q += gridDim.x) {
+        const uint16_t *qc = a.query_cells + (size_t)q * HBG_NUM_CELLS;
+        unsigned long long acc = 0;
+        for (int w = threadIdx.x; w < HBG_NUM_CELLS; w += kOrderThreads) {
+            const unsigned c = __ldg(qc + w);
+            if (c)
+                acc += __ldg(a.db_hist + w) * (unsigned long long)c;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            acc += __shfl_down_sync(kAll, acc, o);
+        if ((threadIdx.x & 31) == 0)
+            sm.keys[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int k = 1; k < kWarps; ++k)
+                acc += sm.keys[k];
+            a.lookup_hits[q] = acc;
+        }
+        __syncthreads();
+    }
+}
+
+// The ordering pass in one launch, bound by its grid barriers (two per 8 bits of
+// the key) until the items are many.  A dozen HSPs 9 us, 570 11 us, 50,000
+// 120 us, 1.4 M 397 us; as 25 launches of separate passes 107, 130, 237 and
+// 893 us.  Ranking against all others is the quicker way up to about 4096
+// (a fourth of the work at each halving; 15 us there), and needs no barrier.
+__global__ void __launch_bounds__(kOrderThreads, 1) order_kernel(OrderArgs a) {
+    __shared__ OrderSmem sm;
+    count_hits(a, sm);
+    const unsigned long long c = *a.count;
+    const int64_t n = (int64_t)(c < (unsigned long long)a.cap ? c : (unsigned long long)a.cap);
+    if (n <= kRankMax)
+        rank_all(a, sm, (int)n);
+    else
+        radix_all(a, sm, n);
 }
 
 __global__ void __launch_bounds__(256)
@@ -214,50 +340,18 @@ db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist) {
             atomicAdd(hist + i, (unsigned long long)hsm[i]);
 }
 
-__global__ void __launch_bounds__(256)
-query_hits(const unsigned long long *hist, const uint16_t *qcells, unsigned long long *out) {
-    __shared__ unsigned long long part[256];
-    const uint16_t *qc = qcells + (size_t)blockIdx.x * HBG_NUM_CELLS;
-    unsigned long long acc = 0;
-    for (int w = threadIdx.x; w < HBG_NUM_CELLS; w += blockDim.x)
-        acc += hist[w] * (unsigned long long)qc[w];
-    part[threadIdx.x] = acc;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < (unsigned)o)
-            part[threadIdx.x] += part[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        out[blockIdx.x] = part[0];
-}
-
 }  // namespace
 
-int64_t order_max_blocks(int64_t cap) { return (cap + kSortTile - 1) / kSortTile; }
+int order_grid(int device) {
+    int sms = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    return std::min(sms, kOrderMaxGrid);
+}
 
-cudaError_t launch_order(const OrderArgs &a, cudaStream_t stream) {
-    const int bits = a.bits_q + a.bits_s + a.bits_so + a.bits_qo;
-    const int64_t maxblk = order_max_blocks(a.cap);
-    if (maxblk == 0)
-        return cudaSuccess;
-    const int gblocks = (int)(maxblk * kSortItems < 65535 ? maxblk * kSortItems : 65535);
-    make_keys<<<gblocks, 256, 0, stream>>>(a.in, a.count, a.cap, a.keys[0], a.vals[0],
-                                           a.bits_s, a.bits_so, a.bits_qo);
-    int src = 0;
-    for (int shift = 0; shift < bits; shift += 8) {
-        sort_histogram<<<(unsigned)maxblk, kSortThreads, 0, stream>>>(a.keys[src], a.count,
-                                                                      a.cap, shift, a.hist);
-        sort_scan<<<1, 1024, 0, stream>>>(a.count, a.cap, a.hist);
-        sort_scatter<<<(unsigned)maxblk, kSortThreads, 0, stream>>>(
-            a.keys[src], a.vals[src], a.keys[src ^ 1], a.vals[src ^ 1], a.count, a.cap, shift,
-            a.hist);
-        src ^= 1;
-    }
-    gather_hsps<<<gblocks, 256, 0, stream>>>(a.in, a.vals[src], a.count, a.cap, a.out);
-    if (a.q_first)
-        query_ranges<<<gblocks, 256, 0, stream>>>(a.out, a.count, a.cap, a.q_first, a.q_end, a.q_passed);
-    return cudaGetLastError();
+cudaError_t launch_order(const OrderArgs &a, int grid, cudaStream_t stream) {
+    OrderArgs args = a;
+    void *params[] = {&args};
+    return cudaLaunchCooperativeKernel((const void *)order_kernel, dim3((unsigned)grid), dim3(kOrderThreads), params, 0, stream);
 }
 
 cudaError_t launch_db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist,
@@ -271,14 +365,6 @@ cudaError_t launch_db_histogram(const uint8_t *db, int64_t n, unsigned long long
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     db_histogram<<<sms > 0 ? sms : 1, 256, smem, stream>>>(db, n, hist);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_query_hits(const unsigned long long *hist, const uint16_t *query_cells,
-                              int32_t n_queries, unsigned long long *out, cudaStream_t stream) {
-    if (n_queries <= 0)
-        return cudaSuccess;
-    query_hits<<<n_queries, 256, 0, stream>>>(hist, query_cells, out);
     return cudaGetLastError();
 }
 
