@@ -568,6 +568,13 @@ __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
         const uint32_t *packed = a.packed + (size_t)g * HBG_NUM_CELLS;
         const uint16_t *ents = a.entries + G.entry_base;
         const unsigned len = sizeof(Cell) == 2 ? (unsigned)G.diag_len : (unsigned)byte_table_len(G.glen + window);
+        if (sizeof(Cell) == 1) {
+            // sweeps move the base of this group's cells alone: start it clean
+            for (unsigned i = lane; i < len / 4; i += 32)
+                smem_at<uint32_t>(tab + 4 * i) = 0;
+            __syncwarp();
+            top = since = 0;
+        }
         // lane k holds the k-th subject of the warp's chunk
         const uint8_t *ds = nullptr;
         int dS = 0, dj = 0, ck = 0, cc = 0;

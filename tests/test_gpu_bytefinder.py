@@ -110,3 +110,16 @@ def test_table_with_repeated_offsets(built):
     assert len(one.hsps) > 0
     assert np.array_equal(one.hsps, two.hsps)
     check(one, [pq], res, off)
+
+
+def test_groups_of_different_lengths(built):
+    """8-bit tables of one launch have their groups' lengths, and a warp goes
+    from group to group with what the last one left in its table: here from a
+    long masked group, soon done, to a shorter one and on to a long one."""
+    rng = np.random.default_rng(21)
+    qs = [np.concatenate([np.full(5500, 21, np.uint8), synth.random_letters(rng, 2500)])]
+    qs += [synth.random_letters(rng, n) for n in (4100, 8100)]
+    db = synth.make_db(rng, 15000, 300, 0.6, 30, 3000, 0.01, qs[1:], 100, 0.5)
+    pqs = [hblast.ProteinQuery.blastp(q) for q in qs]
+    check(hblast.search(hblast.Database(db.residues, db.offsets), hblast.Batch.proteins(pqs)), pqs, db.residues,
+          db.offsets, threads=16)
