@@ -207,6 +207,88 @@ struct LaunchShape {
 };
 constexpr int kMaxLaunchClasses = 32;
 
+// What a search keeps on the host side beside its device buffers: events and
+// the pinned copy of its counters.  Making and freeing them took 250 us of a
+// small search, so a database keeps a few for its next searches.
+struct HostKit {
+    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+    unsigned long long *counters = nullptr;
+    size_t n = 0;                 // counters it has room for
+};
+class KitPool {
+  public:
+    explicit KitPool(int device) : device_(device) {}
+    ~KitPool() {
+        DeviceScope ds(device_);
+        for (HostKit &k : idle_)
+            drop(k);
+        if (upload_)
+            cudaStreamDestroy(upload_);
+    }
+    // A stream for copies that must not wait for the caller's work.
+    cudaError_t upload_stream(cudaStream_t *out) {
+        std::lock_guard<std::mutex> lock(mu_);
+        cudaError_t e = upload_ ? cudaSuccess : cudaStreamCreateWithFlags(&upload_, cudaStreamNonBlocking);
+        *out = upload_;
+        return e;
+    }
+    // A kit with room for n counters.
+    cudaError_t take(size_t n, HostKit *out) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            if (!idle_.empty()) {
+                *out = idle_.back();
+                idle_.pop_back();
+            }
+        }
+        cudaError_t e = cudaSuccess;
+        for (cudaEvent_t &ev : out->ev)
+            if (e == cudaSuccess && !ev)
+                e = cudaEventCreate(&ev);
+        if (e == cudaSuccess && out->n < n) {
+            cudaFreeHost(out->counters);
+            out->counters = nullptr;
+            out->n = 0;
+            n = std::max<size_t>(n, 1024);
+            e = cudaMallocHost((void **)&out->counters, n * sizeof(unsigned long long));
+            if (e == cudaSuccess)
+                out->n = n;
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            drop(*out);
+        }
+        return e;
+    }
+    // Give back a kit that no GPU work still uses.
+    void give(HostKit &k) {
+        {
+            std::lock_guard<std::mutex> lock(mu_);
+            if (k.n > 0 && k.n <= kMost && idle_.size() < kKept) {
+                idle_.push_back(k);
+                k = HostKit();
+                return;
+            }
+        }
+        drop(k);
+    }
+
+  private:
+    static constexpr size_t kKept = 4, kMost = 1 << 17;   // kits, and counters of one (1 MiB)
+    static void drop(HostKit &k) {
+        for (cudaEvent_t &ev : k.ev)
+            if (ev)
+                cudaEventDestroy(ev);
+        if (k.counters)
+            cudaFreeHost(k.counters);
+        k = HostKit();
+    }
+    int device_;
+    std::mutex mu_;
+    std::vector<HostKit> idle_;
+    cudaStream_t upload_ = nullptr;
+};
+
 struct hbg_db {
     uint64_t id = g_next_object_id++;
     int device = 0;
@@ -215,6 +297,7 @@ struct hbg_db {
     int64_t letters_len = 0;
     int32_t max_len = 0;
     std::vector<int32_t> sched_len;   // subject lengths in scheduling order (descending)
+    std::shared_ptr<KitPool> kits;    // also held by the database's results
     uint8_t *d_letters = nullptr;
     int64_t *d_off = nullptr;
     int32_t *d_len = nullptr;
@@ -227,6 +310,7 @@ struct hbg_batch {
     uint64_t id = g_next_object_id++;
     hbg::HostBatch host;
     int device = -1;
+    uint8_t *d_arena = nullptr;        // one block that holds all of the following
     HbgGroup *d_groups = nullptr;
     HbgContext *d_ctx = nullptr;
     HbgQueryDesc *d_queries = nullptr;
@@ -271,9 +355,9 @@ struct hbg_result {
     uint32_t *d_vals = nullptr;
     uint32_t *d_hist = nullptr;
     int64_t sort_cap = 0;
-    cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     // host
-    unsigned long long *h_counters = nullptr;  // pinned
+    std::shared_ptr<KitPool> kits;
+    HostKit kit;                               // events, pinned counters
     size_t n_counters = 0;
     std::vector<hbg_query_stats> stats;
     std::vector<int64_t> q_first, q_count;
@@ -297,32 +381,21 @@ int64_t batch_device_bytes(const hbg::HostBatch &h) {
 }
 
 void free_batch_device(hbg_batch *b) {
-    dfree_idle(b->d_groups);
-    dfree_idle(b->d_ctx);
-    dfree_idle(b->d_queries);
-    if (b->d_letters)
-        b->d_letters -= kFrontPad;
-    dfree_idle(b->d_letters);
-    dfree_idle(b->d_ctx_of);
-    dfree_idle(b->d_cells);
-    dfree_idle(b->d_entries);
-    dfree_idle(b->d_pv);
-    dfree_idle(b->d_qcells);
-    dfree_idle(b->d_group_list);
-    dfree_idle(b->d_packed);
+    dfree_idle(b->d_arena);
 }
 
-int upload_batch_buffers(hbg_batch *b, int device);
+int upload_batch_buffers(hbg_batch *b, const hbg_db *db);
 
 // Upload at the first search; a failed upload gives back what it allocated,
 // so the batch can be searched again later.
-int upload_batch(hbg_batch *b, int device) {
+int upload_batch(hbg_batch *b, const hbg_db *db) {
+    const int device = db->device;
     if (b->device == device)
         return HBG_OK;
     if (b->device >= 0)
         return fail(HBG_ERR_STATE, "batch already resident on another device");
     DeviceScope ds(device);
-    const int rc = upload_batch_buffers(b, device);
+    const int rc = upload_batch_buffers(b, db);
     if (rc != HBG_OK) {
         cudaDeviceSynchronize();   // copies already issued may still read the host vectors
         free_batch_device(b);
@@ -355,28 +428,9 @@ int byte_cell(const hbg_batch *b, int32_t g) {
     return G.diag_len <= kByteTable16 ? 2 : 1;
 }
 
-int upload_batch_buffers(hbg_batch *b, int device) {
+int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
     const hbg::HostBatch &h = b->host;
-    CU(dalloc(&b->d_groups, h.groups.size()));
-    CU(dalloc(&b->d_ctx, h.contexts.size()));
-    CU(dalloc(&b->d_queries, h.queries.size()));
-    CU(alloc_letters(&b->d_letters, h.letters.size() + 64));
-    CU(dalloc(&b->d_ctx_of, h.ctx_of.size() + 16));
-    CU(dalloc(&b->d_cells, h.cells.size()));
-    CU(dalloc(&b->d_entries, h.entries.size() + 64));   // byte_kernel reads up to 31 past a cell
-    CU(dalloc(&b->d_pv, h.pv.size()));
-    CU(dalloc(&b->d_qcells, h.query_cells.size()));
-    CU(dalloc(&b->d_packed, h.groups.size() * HBG_NUM_CELLS));
-    CU(cudaMemcpy(b->d_groups, h.groups.data(), h.groups.size() * sizeof(HbgGroup), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_ctx, h.contexts.data(), h.contexts.size() * sizeof(HbgContext), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_queries, h.queries.data(), h.queries.size() * sizeof(HbgQueryDesc), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_letters, h.letters.data(), h.letters.size(), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_ctx_of, h.ctx_of.data(), h.ctx_of.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_cells, h.cells.data(), h.cells.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    if (!h.entries.empty())
-        CU(cudaMemcpy(b->d_entries, h.entries.data(), h.entries.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_pv, h.pv.data(), h.pv.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(b->d_qcells, h.query_cells.data(), h.query_cells.size() * sizeof(uint16_t), cudaMemcpyHostToDevice));
+    std::vector<int32_t> list;
     {
         // launch classes: (mode, table size); groups with shared tables are
         // launched by table size, so a short query's warps reserve only the
@@ -393,7 +447,6 @@ int upload_batch_buffers(hbg_batch *b, int device) {
         }
         std::stable_sort(keyed.begin(), keyed.end(),
                          [](const auto &x, const auto &y) { return x.first < y.first; });
-        std::vector<int32_t> list;
         b->classes.clear();
         for (size_t i = 0; i < keyed.size(); ++i) {
             const bool global = h.groups[keyed[i].second].placement != 0;
@@ -409,13 +462,60 @@ int upload_batch_buffers(hbg_batch *b, int device) {
         }
         if ((int)b->classes.size() > kMaxLaunchClasses)
             return fail(HBG_ERR_INVALID, "too many launch classes");
-        CU(dalloc(&b->d_group_list, list.size()));
-        CU(cudaMemcpy(b->d_group_list, list.data(), list.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
-    CU(hbg::launch_pack_cells(b->d_cells, (int32_t)h.groups.size(), b->d_packed, 0));
-    CU(cudaStreamSynchronize(0));   // the search may run on any stream
+    // one block, one copy: the arrays in turn, 256-byte aligned; then the
+    // packed cells, made on the device.  (Ten copies of their own took 80 us.)
+    std::vector<std::pair<size_t, std::pair<const void *, size_t>>> parts;   // place, source, bytes
+    size_t at = 0;
+    auto place = [&](const void *src, size_t bytes, size_t before, size_t after) {
+        const size_t p = at + before;
+        parts.push_back({p, {src, bytes}});
+        at = (p + bytes + after + 255) / 256 * 256;
+        return p;
+    };
+    // letters: kFrontPad zeros before (extensions read whole blocks), 64 after
+    const size_t o_groups = place(h.groups.data(), h.groups.size() * sizeof(HbgGroup), 0, 0);
+    const size_t o_ctx = place(h.contexts.data(), h.contexts.size() * sizeof(HbgContext), 0, 0);
+    const size_t o_queries = place(h.queries.data(), h.queries.size() * sizeof(HbgQueryDesc), 0, 0);
+    const size_t o_letters = place(h.letters.data(), h.letters.size(), kFrontPad, 64);
+    const size_t o_ctx_of = place(h.ctx_of.data(), h.ctx_of.size() * sizeof(int32_t), 0, 64);
+    const size_t o_cells = place(h.cells.data(), h.cells.size() * sizeof(uint32_t), 0, 0);
+    // byte_kernel reads up to 31 entries past a cell
+    const size_t o_entries = place(h.entries.data(), h.entries.size() * sizeof(uint16_t), 0, 128);
+    const size_t o_pv = place(h.pv.data(), h.pv.size() * sizeof(uint32_t), 0, 0);
+    const size_t o_qcells = place(h.query_cells.data(), h.query_cells.size() * sizeof(uint16_t), 0, 0);
+    const size_t o_list = place(list.data(), list.size() * sizeof(int32_t), 0, 0);
+    const size_t upload = at;
+    std::unique_ptr<uint8_t[]> stage(new (std::nothrow) uint8_t[upload]);
+    if (!stage)
+        return fail(HBG_ERR_NOMEM, "host allocation");
+    size_t done = 0;
+    for (const auto &p : parts) {
+        memset(stage.get() + done, 0, p.first - done);
+        if (p.second.second)
+            memcpy(stage.get() + p.first, p.second.first, p.second.second);
+        done = p.first + p.second.second;
+    }
+    memset(stage.get() + done, 0, upload - done);
+    CU(dalloc(&b->d_arena, upload + h.groups.size() * HBG_NUM_CELLS * sizeof(uint32_t)));
+    b->d_groups = reinterpret_cast<HbgGroup *>(b->d_arena + o_groups);
+    b->d_ctx = reinterpret_cast<HbgContext *>(b->d_arena + o_ctx);
+    b->d_queries = reinterpret_cast<HbgQueryDesc *>(b->d_arena + o_queries);
+    b->d_letters = b->d_arena + o_letters;
+    b->d_ctx_of = reinterpret_cast<int32_t *>(b->d_arena + o_ctx_of);
+    b->d_cells = reinterpret_cast<uint32_t *>(b->d_arena + o_cells);
+    b->d_entries = reinterpret_cast<uint16_t *>(b->d_arena + o_entries);
+    b->d_pv = reinterpret_cast<uint32_t *>(b->d_arena + o_pv);
+    b->d_qcells = reinterpret_cast<uint16_t *>(b->d_arena + o_qcells);
+    b->d_group_list = reinterpret_cast<int32_t *>(b->d_arena + o_list);
+    b->d_packed = reinterpret_cast<uint32_t *>(b->d_arena + upload);
+    cudaStream_t st = nullptr;
+    CU(db->kits->upload_stream(&st));
+    CU(cudaMemcpyAsync(b->d_arena, stage.get(), upload, cudaMemcpyHostToDevice, st));
+    CU(hbg::launch_pack_cells(b->d_cells, (int32_t)h.groups.size(), b->d_packed, st));
+    CU(cudaStreamSynchronize(st));   // the search may run on any stream
     b->device_bytes = batch_device_bytes(h);
-    b->device = device;
+    b->device = db->device;
     return HBG_OK;
 }
 
@@ -444,50 +544,11 @@ int32_t class_tile_subjects(const hbg_batch *b, int32_t n_subj, const hbg_db *db
     return (int32_t)std::max<int64_t>(8, std::min<int64_t>(128, want));
 }
 
-// CTA size and grid of each launch class: the CTA is halved until its
-// per-warp tables fit the shared-memory carve-out; the grid is one wave at
-// the occupancy that leaves (or the caller's num_blocksx).
-int plan_launches(const hbg_batch *b, const hbg_gpu_options &o, int device, std::vector<LaunchShape> *out) {
-    int optin = 0, sms = 1;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    out->clear();
-    for (const LaunchClass &lc : b->classes) {
-        // num_threadsx is the largest CTA size: per class take the size (halving
-        // down to 64) that keeps the most warps resident per SM -- large diagonal
-        // tables fill shared memory, and smaller CTAs pack it better
-        // with several groups per pass (team > 1) the CTA keeps at least one
-        // warp per group
-        int best_t = 0, best_per = 0, best_warps = -1;
-        for (int t = o.num_threadsx; t >= 32; t = t > 64 ? ((t / 2) + 31) / 32 * 32 : 0) {
-            const int team = std::min(b->team, t / 32);
-            if (team < b->team && best_t > 0)
-                break;
-            if (hbg::wordfinder_smem_bytes(t, lc.smem_diag, team) > (size_t)optin)
-                continue;
-            int per = 0;
-            if (hbg::wordfinder_occupancy(lc.mode, t, lc.smem_diag, team, &per) != cudaSuccess || per < 1)
-                per = 1;
-            if (per * (t / 32) > best_warps) {
-                best_t = t;
-                best_per = per;
-                best_warps = per * (t / 32);
-            }
-            if (o.num_blocksx > 0)
-                break;                 // a fixed grid keeps the caller's CTA size when it fits
-        }
-        if (best_t == 0)
-            return fail(HBG_ERR_TOO_LONG, "group diagonal tables exceed shared memory");
-        const int blocks = o.num_blocksx > 0 ? o.num_blocksx : sms * best_per;
-        out->push_back(LaunchShape{best_t, blocks, std::min(b->team, best_t / 32), 0, 0, 0});
-    }
-    return HBG_OK;
-}
-
 // Which classes byte_kernel takes, with which CTA, and the subjects that stay
 // with wordfinder_kernel: those whose positions do not fit its cells.
 void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, int device,
                 std::vector<LaunchShape> *shapes) {
+    shapes->assign(b->classes.size(), LaunchShape{32, 1, 1, 0, 0, 0});
     hbg_gpu_options std_opt;
     hbg_default_gpu_options(&std_opt);
     if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx || b->tuned || b->team > 1 ||
@@ -515,6 +576,51 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
     }
 }
 
+// CTA size and grid of each launch class that wordfinder_kernel has a part of: the CTA is halved until its
+// per-warp tables fit the shared-memory carve-out; the grid is one wave at
+// the occupancy that leaves (or the caller's num_blocksx).
+int plan_launches(const hbg_batch *b, const hbg_gpu_options &o, int device, std::vector<LaunchShape> *out) {
+    int optin = 0, sms = 1;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    for (size_t c = 0; c < b->classes.size(); ++c) {
+        const LaunchClass &lc = b->classes[c];
+        LaunchShape &sh = (*out)[c];
+        if (sh.byte_threads > 0 && sh.n_long == 0)
+            continue;
+        // num_threadsx is the largest CTA size: per class take the size (halving
+        // down to 64) that keeps the most warps resident per SM -- large diagonal
+        // tables fill shared memory, and smaller CTAs pack it better
+        // with several groups per pass (team > 1) the CTA keeps at least one
+        // warp per group
+        int best_t = 0, best_per = 0, best_warps = -1;
+        for (int t = o.num_threadsx; t >= 32; t = t > 64 ? ((t / 2) + 31) / 32 * 32 : 0) {
+            const int team = std::min(b->team, t / 32);
+            if (team < b->team && best_t > 0)
+                break;
+            if (hbg::wordfinder_smem_bytes(t, lc.smem_diag, team) > (size_t)optin)
+                continue;
+            int per = 0;
+            if (hbg::wordfinder_occupancy(lc.mode, t, lc.smem_diag, team, &per) != cudaSuccess || per < 1)
+                per = 1;
+            if (per * (t / 32) > best_warps) {
+                best_t = t;
+                best_per = per;
+                best_warps = per * (t / 32);
+            }
+            if (o.num_blocksx > 0)
+                break;                 // a fixed grid keeps the caller's CTA size when it fits
+        }
+        if (best_t == 0)
+            return fail(HBG_ERR_TOO_LONG, "group diagonal tables exceed shared memory");
+        const int blocks = o.num_blocksx > 0 ? o.num_blocksx : sms * best_per;
+        sh.threads = best_t;
+        sh.blocks = blocks;
+        sh.team = std::min(b->team, best_t / 32);
+    }
+    return HBG_OK;
+}
+
 void drop_graph(hbg_result *r) {
     if (r->graph_exec)
         cudaGraphExecDestroy(r->graph_exec);
@@ -536,15 +642,8 @@ void free_result_device(hbg_result *r) {
     dfree_idle(r->d_keys);
     dfree_idle(r->d_vals);
     dfree_idle(r->d_hist);
-    for (auto &e : r->ev)
-        if (e) {
-            cudaEventDestroy(e);
-            e = nullptr;
-        }
-    if (r->h_counters) {
-        cudaFreeHost(r->h_counters);
-        r->h_counters = nullptr;
-    }
+    if (r->kits)
+        r->kits->give(r->kit);
 }
 
 // Some class or subject of this search goes to wordfinder_kernel.
@@ -559,22 +658,17 @@ bool uses_wordfinder(const hbg_result *r) {
 int prepare_result(hbg_result *r, int64_t cap) {
     const hbg::HostBatch &h = r->batch->host;
     const size_t nq = h.queries.size(), ng = h.groups.size();
-    if (!r->d_tile) {
+    if (!r->d_tile)
         CU(dalloc(&r->d_tile, kMaxLaunchClasses));
-        for (auto &e : r->ev)
-            CU(cudaEventCreate(&e));
-    }
     // a failed allocation below leaves the recorded size at 0, so the next
     // search allocates again instead of using a missing buffer
     if (r->n_counters < 3 + 6 * nq + 2 * ng) {   // first use, or a larger batch
         drop_graph(r);
         dfree(r->d_counters);
-        if (r->h_counters)
-            cudaFreeHost(r->h_counters);
-        r->h_counters = nullptr;
+        r->kits->give(r->kit);
         r->n_counters = 0;
         CU(dalloc(&r->d_counters, 3 + 6 * nq + 2 * ng));
-        CU(cudaMallocHost((void **)&r->h_counters, (3 + 6 * nq + 2 * ng) * sizeof(unsigned long long)));
+        CU(r->kits->take(3 + 6 * nq + 2 * ng, &r->kit));
         r->n_counters = 3 + 6 * nq + 2 * ng;
     }
     r->gdiag_len = global_diag_len(h, r->db);
@@ -714,7 +808,7 @@ int enqueue_search(hbg_result *r) {
     CU(cudaStreamIsCapturing(st, &cap_status));
     const unsigned ev_flags =
         cap_status == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
-    CU(cudaEventRecordWithFlags(r->ev[0], st, ev_flags));
+    CU(cudaEventRecordWithFlags(r->kit.ev[0], st, ev_flags));
     int wf_launches = 0;
     if (db->n > 0)   // the caller has run wordfinder_configure (not a stream operation)
         for (size_t c = 0; c < b->classes.size(); ++c) {
@@ -748,7 +842,7 @@ int enqueue_search(hbg_result *r) {
             a.smem_diag = lc.smem_diag;
             CU(hbg::launch_wordfinder(a, lc.mode, r->shapes[c].blocks, r->shapes[c].threads, st));
         }
-    CU(cudaEventRecordWithFlags(r->ev[1], st, ev_flags));
+    CU(cudaEventRecordWithFlags(r->kit.ev[1], st, ev_flags));
 
     hbg::OrderArgs o;
     memset(&o, 0, sizeof(o));
@@ -778,8 +872,8 @@ int enqueue_search(hbg_result *r) {
     o.lookup_hits = r->d_counters + 1 + 2 * nq;
     CU(hbg::launch_order(o, hbg::order_grid(r->device), st));
     r->launches = wf_launches + 1;
-    CU(cudaEventRecordWithFlags(r->ev[2], st, ev_flags));
-    CU(cudaMemcpyAsync(r->h_counters, r->d_counters, r->n_counters * sizeof(unsigned long long),
+    CU(cudaEventRecordWithFlags(r->kit.ev[2], st, ev_flags));
+    CU(cudaMemcpyAsync(r->kit.counters, r->d_counters, r->n_counters * sizeof(unsigned long long),
                        cudaMemcpyDeviceToHost, st));
     return HBG_OK;
 }
@@ -788,7 +882,6 @@ int enqueue_search(hbg_result *r) {
 // stream with the same buffers replays a CUDA graph of the whole sequence
 // (captured on its second launch) instead of ~30 separate launches.
 int launch_search(hbg_result *r) {
-    CU(hbg::wordfinder_configure());
     const bool graphable = r->stream != nullptr && r->launch_count > 0;
     const long long key[6] = {(long long)r->batch_id, (long long)r->cap,
                               ((long long)r->shape_opt.num_blocksx << 32) | (unsigned)r->shape_opt.num_threadsx,
@@ -899,6 +992,7 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
     if (!db)
         return fail(HBG_ERR_NOMEM, "host allocation");
     db->device = device;
+    db->kits = std::make_shared<KitPool>(device);
     DeviceScope ds(db->device);
     auto bail = [&](int code) {
         free_letters(db->d_letters);
@@ -1526,7 +1620,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     if (!valid_opts(&o))
         return fail(HBG_ERR_INVALID, "num_threadsx must be a multiple of 32 in 32..256");
     DeviceScope ds(db->device);
-    int rc = upload_batch(batch, db->device);
+    int rc = upload_batch(batch, db);
     if (rc != HBG_OK)
         return rc;
     hbg_result *r = *out;
@@ -1551,6 +1645,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
         r->batch = batch;
         r->batch_id = batch->id;
         r->device = db->device;
+        r->kits = db->kits;
     }
     r->opt = o;
     r->stream = (cudaStream_t)stream;
@@ -1559,13 +1654,13 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
             delete r;
         return fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
     }
+    plan_bytes(batch, db, o, db->device, &r->shapes);
     rc = plan_launches(batch, o, db->device, &r->shapes);
     if (rc != HBG_OK) {
         if (!*out)
             delete r;
         return rc;
     }
-    plan_bytes(batch, db, o, db->device, &r->shapes);
     r->shape_opt = o;
     r->blocks = 0;
     r->threads = 32;
@@ -1603,7 +1698,7 @@ int hbg_result_sync(hbg_result *r) {
         return HBG_OK;
     DeviceScope ds(r->device);
     CU(cudaStreamSynchronize(r->stream));
-    unsigned long long n = r->h_counters[0];
+    unsigned long long n = r->kit.counters[0];
     if ((int64_t)n > r->cap) {
         // the HSP buffer was too small: relaunch once with the exact size.  If
         // that cannot be set up, nothing of this search runs any more and the
@@ -1617,20 +1712,20 @@ int hbg_result_sync(hbg_result *r) {
             return rc;
         }
         CU(cudaStreamSynchronize(r->stream));
-        n = r->h_counters[0];
+        n = r->kit.counters[0];
         if ((int64_t)n > r->cap)
             return fail(HBG_ERR_STATE, "HSP count changed between identical launches");
     }
     {
         const size_t nq = r->batch->host.queries.size(), ng = r->batch->host.groups.size();
-        if (r->h_counters[2 + 6 * nq + 2 * ng]) {   // a result may be launched again
+        if (r->kit.counters[2 + 6 * nq + 2 * ng]) {   // a result may be launched again
             r->launched = false;
             return fail(HBG_ERR_CUDA, "the ordering pass gave up waiting for its own blocks");
         }
     }
     r->n_hsps = (int64_t)n;
-    CU(cudaEventElapsedTime(&r->wf_ms, r->ev[0], r->ev[1]));
-    CU(cudaEventElapsedTime(&r->ord_ms, r->ev[1], r->ev[2]));
+    CU(cudaEventElapsedTime(&r->wf_ms, r->kit.ev[0], r->kit.ev[1]));
+    CU(cudaEventElapsedTime(&r->ord_ms, r->kit.ev[1], r->kit.ev[2]));
     r->synced = true;
     return HBG_OK;
 }
@@ -1644,14 +1739,14 @@ int hbg_result_wait(hbg_result *r) {
     // the ordered HSPs stay on the device (read with hbg_result_hsps); the
     // ordering pass left per-query ranges and subject counts beside the counters
     const size_t nq = r->batch->host.queries.size(), ng = r->batch->host.groups.size();
-    const unsigned long long *rng = r->h_counters + 1 + 3 * nq + ng;
+    const unsigned long long *rng = r->kit.counters + 1 + 3 * nq + ng;
     r->stats.assign(nq, hbg_query_stats{0, 0, 0, 0});
     r->q_first.assign(nq, 0);
     r->q_count.assign(nq, 0);
     for (size_t q = 0; q < nq; ++q) {
-        r->stats[q].init_extends = (int64_t)r->h_counters[1 + q];
-        r->stats[q].good_init_extends = (int64_t)r->h_counters[1 + nq + q];
-        r->stats[q].lookup_hits = (int64_t)r->h_counters[1 + 2 * nq + q];
+        r->stats[q].init_extends = (int64_t)r->kit.counters[1 + q];
+        r->stats[q].good_init_extends = (int64_t)r->kit.counters[1 + nq + q];
+        r->stats[q].lookup_hits = (int64_t)r->kit.counters[1 + 2 * nq + q];
         r->stats[q].subjects_passed = (int64_t)rng[2 * nq + q];
         r->q_first[q] = (int64_t)rng[q];
         r->q_count[q] = (int64_t)rng[nq + q] - (int64_t)rng[q];
@@ -1839,10 +1934,10 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     CU(hbg::wordfinder_configure());
     CU(hbg::byte_configure());
     std::vector<LaunchShape> shapes;   // host-side only; no device allocation
+    plan_bytes(batch, db, o, db->device, &shapes);
     rc = plan_launches(batch, o, db->device, &shapes);
     if (rc != HBG_OK)
         return rc;
-    plan_bytes(batch, db, o, db->device, &shapes);
     cudaStream_t st = (cudaStream_t)stream;
     unsigned char *base = (unsigned char *)scratch;
     unsigned int *tile = (unsigned int *)base;

@@ -51,22 +51,22 @@ class NeighbourCache {
         return lists_[(a << 10) | (b << 5) | c];
     }
 
-    // Enumerate the neighbourhoods of the flagged words not seen before, in
+    // Enumerate the neighbourhoods of those words not seen before, in
     // parallel.  Builds running at the same time take turns here; a list,
     // once written, never changes.
     template <typename ParallelFor>
-    void prepare(const std::vector<uint8_t> &need, ParallelFor &&pfor) {
+    void prepare(const std::vector<int32_t> &words, ParallelFor &&pfor) {
         std::lock_guard<std::mutex> lock(mu_);
         std::vector<int32_t> keys;
-        for (int32_t k = 0; k < HBG_NUM_CELLS; ++k)
-            if (need[k] && !done_[k])
+        for (int32_t k : words)
+            if (!done_[k]) {
+                done_[k] = 1;                 // listed once
                 keys.push_back(k);
+            }
         pfor((int64_t)keys.size(), [&](int64_t i) {
             const int32_t k = keys[i];
             enumerate((uint8_t)(k >> 10), (uint8_t)((k >> 5) & 31), (uint8_t)(k & 31), &lists_[k]);
         });
-        for (int32_t k : keys)
-            done_[k] = 1;
     }
 
   private:
@@ -270,16 +270,17 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
         return c0 >= 0 && gc[p + 1] == c0 && gc[p + 2] == c0;
     };
     {
-        std::vector<uint8_t> need(HBG_NUM_CELLS, 0);
+        std::vector<int32_t> words;
+        words.reserve(b.letters.size());
         for (int32_t g = 0; g < n_groups; ++g) {
             const HbgGroup &G = b.groups[g];
             const uint8_t *gs = b.letters.data() + G.seq_base;
             const int32_t *gc = b.ctx_of.data() + G.seq_base;
             for (int32_t p = 0; p + HBG_WORD_SIZE <= G.glen; ++p)
                 if (valid(gc, p))
-                    need[(gs[p] << 10) | (gs[p + 1] << 5) | gs[p + 2]] = 1;
+                    words.push_back((gs[p] << 10) | (gs[p + 1] << 5) | gs[p + 2]);
         }
-        nb.prepare(need, parallel_for);
+        nb.prepare(words, parallel_for);
     }
     std::vector<uint32_t> group_entries(n_groups, 0);
     parallel_for(n_groups, [&](int64_t gi) {
@@ -315,11 +316,14 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
         // words over the 20 standard letters, each such word taken as
         // equally likely (1 / 8000)
         static const uint8_t kStd[20] = {1, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18, 19, 20, 22};
-        uint64_t std_entries = 0;
-        for (int x = 0; x < 20; ++x)
-            for (int y = 0; y < 20; ++y)
-                for (int z = 0; z < 20; ++z)
-                    std_entries += count[(kStd[x] << 10) | (kStd[y] << 5) | kStd[z]];
+        uint64_t std_entries = acc;            // an upper bound, enough for most groups
+        if ((double)std_entries / 8000.0 >= mode_hits) {
+            std_entries = 0;
+            for (int x = 0; x < 20; ++x)
+                for (int y = 0; y < 20; ++y)
+                    for (int z = 0; z < 20; ++z)
+                        std_entries += count[(kStd[x] << 10) | (kStd[y] << 5) | kStd[z]];
+        }
         G.mode = (double)std_entries / 8000.0 >= mode_hits ? 1 : 0;
     });
     int64_t entry_pos = 0;
