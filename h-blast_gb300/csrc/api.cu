@@ -146,22 +146,9 @@ void dfree_idle(T *&p) {
     p = nullptr;
 }
 
-// Letter buffers have zeros before their first letter, and callers add 64
-// after the last: extensions read whole blocks.
+// Zeros before the first letter of a letter buffer; 64 follow the last:
+// extensions read whole blocks.
 constexpr size_t kFrontPad = 64;
-cudaError_t alloc_letters(uint8_t **p, size_t n) {
-    cudaError_t e = dalloc(p, n + kFrontPad);
-    if (e != cudaSuccess)
-        return e;
-    e = cudaMemset(*p, 0, n + kFrontPad);
-    *p += kFrontPad;
-    return e;
-}
-void free_letters(uint8_t *&p) {
-    if (p)
-        p -= kFrontPad;
-    dfree(p);
-}
 
 // Device guard: make `dev` current for the scope.
 struct DeviceScope {
@@ -298,6 +285,7 @@ struct hbg_db {
     int32_t max_len = 0;
     std::vector<int32_t> sched_len;   // subject lengths in scheduling order (descending)
     std::shared_ptr<KitPool> kits;    // also held by the database's results
+    uint8_t *d_arena = nullptr;       // one block that holds all of the following
     uint8_t *d_letters = nullptr;
     int64_t *d_off = nullptr;
     int32_t *d_len = nullptr;
@@ -976,6 +964,24 @@ int db_device(const hbg_gpu_options *opt, hbg_gpu_options *o) {
     return HBG_OK;
 }
 
+// Subjects by descending length, equal lengths in database order.
+std::vector<int32_t> schedule(const std::vector<int32_t> &len, int32_t max_len) {
+    std::vector<int32_t> order(len.size());
+    if (max_len > (1 << 20)) {
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(), [&](int32_t x, int32_t y) { return len[x] > len[y]; });
+        return order;
+    }
+    std::vector<int32_t> at((size_t)max_len + 2, 0);   // at[k]: next place of length max_len - k
+    for (int32_t l : len)
+        ++at[(size_t)(max_len - l) + 1];
+    for (size_t k = 1; k < at.size(); ++k)
+        at[k] += at[k - 1];
+    for (size_t i = 0; i < len.size(); ++i)
+        order[at[(size_t)(max_len - len[i])]++] = (int32_t)i;
+    return order;
+}
+
 // Allocate the resident database for a validated layout (subject i at
 // device offset off[i], len[i] letters, sentinels between), let `fill` copy
 // the letters (it returns "" or an error), then the offsets, the
@@ -983,10 +989,7 @@ int db_device(const hbg_gpu_options *opt, hbg_gpu_options *o) {
 template <typename Fill>
 int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std::vector<int32_t> &len,
               int64_t total, int32_t max_len, int64_t letters_len, Fill &&fill, hbg_db **out) {
-    std::vector<int32_t> order(n);
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t x, int32_t y) { return len[x] > len[y]; });
+    const std::vector<int32_t> order = schedule(len, max_len);
 
     hbg_db *db = new (std::nothrow) hbg_db;
     if (!db)
@@ -995,11 +998,7 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
     db->kits = std::make_shared<KitPool>(device);
     DeviceScope ds(db->device);
     auto bail = [&](int code) {
-        free_letters(db->d_letters);
-        dfree(db->d_off);
-        dfree(db->d_len);
-        dfree(db->d_order);
-        dfree(db->d_hist);
+        dfree(db->d_arena);
         delete db;
         return code;
     };
@@ -1010,11 +1009,18 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
             return bail(fail(e_ == cudaErrorMemoryAllocation ? HBG_ERR_NOMEM : HBG_ERR_CUDA, \
                              std::string(#call) + ": " + cudaGetErrorString(e_)));  \
     } while (0)
-    CUB(alloc_letters(&db->d_letters, (size_t)letters_len));
-    CUB(dalloc(&db->d_off, (size_t)n));
-    CUB(dalloc(&db->d_len, (size_t)n));
-    CUB(dalloc(&db->d_order, (size_t)n));
-    CUB(dalloc(&db->d_hist, HBG_NUM_CELLS));
+    // one block: letters (with zeros before them and after), offsets, lengths,
+    // schedule, histogram
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t o_off = up(kFrontPad + (size_t)letters_len), o_len = up(o_off + sizeof(int64_t) * n),
+                 o_order = up(o_len + sizeof(int32_t) * n), o_hist = up(o_order + sizeof(int32_t) * n);
+    CUB(dalloc(&db->d_arena, o_hist + sizeof(unsigned long long) * HBG_NUM_CELLS));
+    db->d_letters = db->d_arena + kFrontPad;
+    db->d_off = reinterpret_cast<int64_t *>(db->d_arena + o_off);
+    db->d_len = reinterpret_cast<int32_t *>(db->d_arena + o_len);
+    db->d_order = reinterpret_cast<int32_t *>(db->d_arena + o_order);
+    db->d_hist = reinterpret_cast<unsigned long long *>(db->d_arena + o_hist);
+    CUB(cudaMemset(db->d_arena, 0, kFrontPad + (size_t)letters_len));
     {
         int code = HBG_OK;
         std::string err = fill(db->d_letters, &code);
@@ -1045,6 +1051,10 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
 std::string cuda_msg(const char *what, cudaError_t e, int *code) {
     *code = e == cudaErrorMemoryAllocation ? HBG_ERR_NOMEM : HBG_ERR_CUDA;
     return std::string(what) + ": " + cudaGetErrorString(e);
+}
+
+std::string bad_letter(int32_t subject) {
+    return "subject " + std::to_string(subject) + ": letter outside NCBIstdaa 1..27";
 }
 
 // Volumes of a BLAST database with their place in the resident layout:
@@ -1098,21 +1108,20 @@ int hbg_db_open(const uint8_t *residues, const int64_t *offsets, int32_t n,
     int rc = db_device(opt, &o);
     if (rc != HBG_OK)
         return rc;
-    // validate and lay out: one sentinel before every subject and after the last
+    // lay out: one sentinel before every subject and after the last
     std::vector<int64_t> off(n);
     std::vector<int32_t> len(n);
     int64_t pos = 1, total = 0;
     int32_t max_len = 0;
     for (int32_t i = 0; i < n; ++i) {
-        int64_t L = offsets[i + 1] - offsets[i];
-        if (L < 0 || L > HBG_MAX_SUBJECT_LEN)
-            return fail(L < 0 ? HBG_ERR_INVALID : HBG_ERR_TOO_LONG,
-                        "subject " + std::to_string(i) + ": bad length");
-        const uint8_t *s = residues + offsets[i];
-        for (int64_t k = 0; k < L; ++k)
-            if (s[k] == 0 || s[k] >= HBG_ALPHABET)
-                return fail(HBG_ERR_INVALID, "subject " + std::to_string(i) +
-                                                 ": letter outside NCBIstdaa 1..27");
+        const int64_t L = offsets[i + 1] - offsets[i];
+        if (L < 0 || L > HBG_MAX_SUBJECT_LEN) {
+            for (int32_t j = 0; j < i; ++j)         // an earlier subject's fault comes first
+                for (int64_t k = offsets[j]; k < offsets[j + 1]; ++k)
+                    if (residues[k] == 0 || residues[k] >= HBG_ALPHABET)
+                        return fail(HBG_ERR_INVALID, bad_letter(j));
+            return fail(L < 0 ? HBG_ERR_INVALID : HBG_ERR_TOO_LONG, "subject " + std::to_string(i) + ": bad length");
+        }
         off[i] = pos;
         len[i] = (int32_t)L;
         pos += L + 1;
@@ -1120,23 +1129,43 @@ int hbg_db_open(const uint8_t *residues, const int64_t *offsets, int32_t n,
         max_len = std::max<int32_t>(max_len, (int32_t)L);
     }
     const int64_t letters_len = pos + 64;
-    // copy subjects with their sentinels through a staging buffer of ~64 MiB
+    // the letters go up as they lie, 64 MiB at a time, and are checked and
+    // spread out on the device
     auto fill = [&](uint8_t *d_letters, int *code) -> std::string {
-        int32_t i = 0;
-        std::vector<uint8_t> stage;
-        while (i < n) {
-            const int64_t start_dev = off[i] - 1;
-            stage.clear();
-            stage.push_back(0);
-            while (i < n && (int64_t)stage.size() < (64 << 20)) {
-                const uint8_t *s = residues + offsets[i];
-                stage.insert(stage.end(), s, s + len[i]);
-                stage.push_back(0);
-                ++i;
-            }
-            cudaError_t e = cudaMemcpy(d_letters + start_dev, stage.data(), stage.size(), cudaMemcpyHostToDevice);
-            if (e != cudaSuccess)
-                return cuda_msg("cudaMemcpy (subjects)", e, code);
+        if (total == 0)
+            return std::string();
+        const int64_t piece = std::min<int64_t>(total, (int64_t)64 << 20);
+        uint8_t *d_raw = nullptr;
+        int64_t *d_first = nullptr;
+        int32_t *d_bad = nullptr;
+        int32_t bad = INT32_MAX;
+        cudaError_t e = dalloc(&d_raw, (size_t)piece);
+        if (e == cudaSuccess)
+            e = dalloc(&d_first, (size_t)n + 1);
+        if (e == cudaSuccess)
+            e = dalloc(&d_bad, 1);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(d_first, offsets, sizeof(int64_t) * ((size_t)n + 1), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess)
+            e = cudaMemcpy(d_bad, &bad, sizeof(bad), cudaMemcpyHostToDevice);
+        for (int64_t at = 0; at < total && e == cudaSuccess; at += piece) {
+            const int64_t m = std::min<int64_t>(piece, total - at);
+            e = cudaMemcpy(d_raw, residues + offsets[0] + at, (size_t)m, cudaMemcpyHostToDevice);
+            if (e == cudaSuccess)
+                e = hbg::launch_spread_letters(d_raw, offsets[0] + at, m, d_first, n, d_letters, d_bad, 0);
+        }
+        if (e == cudaSuccess)
+            e = cudaMemcpy(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost);
+        else
+            cudaDeviceSynchronize();                // nothing may still use the buffers
+        dfree_idle(d_raw);
+        dfree_idle(d_first);
+        dfree_idle(d_bad);
+        if (e != cudaSuccess)
+            return cuda_msg("laying out the subjects", e, code);
+        if (bad != INT32_MAX) {
+            *code = HBG_ERR_INVALID;
+            return bad_letter(bad);
         }
         return std::string();
     };
@@ -1294,11 +1323,7 @@ int hbg_db_close(hbg_db *db) {
     if (!db)
         return fail(HBG_ERR_INVALID, "null db");
     DeviceScope ds(db->device);
-    free_letters(db->d_letters);
-    dfree(db->d_off);
-    dfree(db->d_len);
-    dfree(db->d_order);
-    dfree(db->d_hist);
+    dfree(db->d_arena);
     delete db;
     return HBG_OK;
 }

@@ -131,6 +131,13 @@ struct OrderArgs {
 int order_grid(int device);
 cudaError_t launch_order(const OrderArgs &a, int grid, cudaStream_t stream);
 
+// Letters of subjects that lie back to back (subject i at [first[i],
+// first[i + 1]) of the caller's numbering), `count` of them from letter `from`
+// on, into the resident layout: one zero before every subject and after the
+// last.  *bad = min(*bad, subject with a letter outside 1..27).
+cudaError_t launch_spread_letters(const uint8_t *raw, int64_t from, int64_t count, const int64_t *first, int32_t n,
+                                  uint8_t *out, int32_t *bad, cudaStream_t stream);
+
 // Database word histogram: hist[w] += positions whose three letters are
 // non-sentinel and form word w.
 cudaError_t launch_db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist,

@@ -322,6 +322,41 @@ __global__ void __launch_bounds__(kOrderThreads, 1) order_kernel(OrderArgs a) {
         radix_all(a, sm, n);
 }
 
+// A warp spreads 1024 consecutive letters, a lane every 32nd: the subject of
+// the first by bisection, the others from there.  Bound by the copy to the
+// device: 18 M letters in 50,000 subjects open in 0.56 ms, 359 M in 1 M subjects
+// in 10.3 ms; 13.2 and 288 ms with the checks and the staging on the host.
+constexpr int kSpread = 1024;
+__global__ void __launch_bounds__(256)
+spread_letters(const uint8_t *raw, int64_t from, int64_t count, const int64_t *first, int32_t n, uint8_t *out,
+               int32_t *bad) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x / 32);
+    for (int64_t c = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 32; c * kSpread < count; c += warps) {
+        const int64_t begin = from + c * kSpread, end = min(from + count, begin + kSpread);
+        // the last subject that starts at or before `begin`
+        int32_t lo = 0, hi = n;
+        while (hi - lo > 1) {
+            const int32_t mid = lo + (hi - lo) / 2;
+            if (first[mid] <= begin)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        int32_t i = lo;
+        int64_t next = first[i + 1];
+        const int64_t shift = 1 - first[0];
+        for (int64_t p = begin + lane; p < end; p += 32) {
+            while (p >= next)
+                next = first[++i + 1];
+            const uint8_t a = raw[p - from];
+            out[p + shift + i] = a;
+            if (a == 0 || a >= HBG_ALPHABET)
+                atomicMin(bad, i);
+        }
+    }
+}
+
 __global__ void __launch_bounds__(256)
 db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist) {
     extern __shared__ unsigned int hsm[];
@@ -352,6 +387,13 @@ cudaError_t launch_order(const OrderArgs &a, int grid, cudaStream_t stream) {
     OrderArgs args = a;
     void *params[] = {&args};
     return cudaLaunchCooperativeKernel((const void *)order_kernel, dim3((unsigned)grid), dim3(kOrderThreads), params, 0, stream);
+}
+
+cudaError_t launch_spread_letters(const uint8_t *raw, int64_t from, int64_t count, const int64_t *first, int32_t n,
+                                  uint8_t *out, int32_t *bad, cudaStream_t stream) {
+    const int64_t ctas = (count + 8 * kSpread - 1) / (8 * kSpread);
+    spread_letters<<<(unsigned)std::min<int64_t>(ctas, 65535), 256, 0, stream>>>(raw, from, count, first, n, out, bad);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist,
