@@ -310,10 +310,13 @@ struct hbg_batch {
     uint16_t *d_qcells = nullptr;
     int32_t *d_group_list = nullptr;   // groups ordered by launch class
     uint32_t *d_packed = nullptr;      // cells of byte_kernel
+    uint2 *d_stats = nullptr;          // per group: entries, fullest cell
+    uint16_t *d_more = nullptr;        // entries, when they did not fit the block
     std::vector<LaunchClass> classes;
+    std::mutex tables_mu;              // host tables are built when first asked for
+    bool caller_tables = false;        // the tables are the caller's (in `host`)
     bool repeated_entries = false;     // a caller's lookup table lists an offset twice in a cell
     bool tuned = false;                // the caller chose tiles or table placement (hbg_batch_tune)
-    int64_t device_bytes = 0;
     int32_t tile_subjects = 0;   // 0 = automatic (hbg_batch_tune)
     int64_t tile_bytes = 0;      // > 0: tiles of about this many subject letters (hbg_batch_schedule)
     int32_t team = 1;            // groups searched together per pass over a subject (hbg_batch_schedule)
@@ -361,18 +364,32 @@ struct hbg_result {
 
 namespace {
 
-int64_t batch_device_bytes(const hbg::HostBatch &h) {
+int64_t batch_device_bytes(const hbg::HostBatch &h, int64_t entries) {
+    const int64_t ng = (int64_t)h.groups.size(), nq = (int64_t)h.queries.size();
     return (int64_t)(h.groups.size() * sizeof(HbgGroup) + h.contexts.size() * sizeof(HbgContext) +
-                     h.queries.size() * sizeof(HbgQueryDesc) + h.letters.size() + h.ctx_of.size() * 4 +
-                     h.cells.size() * 4 + h.entries.size() * 2 + h.pv.size() * 4 + h.query_cells.size() * 2 +
-                     h.groups.size() * HBG_NUM_CELLS * 4);
+                     h.queries.size() * sizeof(HbgQueryDesc) + h.letters.size() + h.ctx_of.size() * 4) +
+           ng * (HBG_CELL_STRIDE + HBG_PV_WORDS + HBG_NUM_CELLS) * 4 + entries * 2 + nq * HBG_NUM_CELLS * 2;
 }
 
 void free_batch_device(hbg_batch *b) {
     dfree_idle(b->d_arena);
+    dfree_idle(b->d_more);
 }
 
 int upload_batch_buffers(hbg_batch *b, const hbg_db *db);
+
+// Host tables, built when a caller first asks for them.
+void ensure_tables(const hbg_batch *batch) {
+    hbg_batch *b = const_cast<hbg_batch *>(batch);
+    std::lock_guard<std::mutex> lock(b->tables_mu);
+    if (b->host.cells.empty())
+        hbg::build_tables(&b->host);
+}
+int64_t batch_entries(const hbg_batch *batch) {
+    hbg_batch *b = const_cast<hbg_batch *>(batch);
+    std::lock_guard<std::mutex> lock(b->tables_mu);
+    return hbg::count_entries(b->host);
+}
 
 // Upload at the first search; a failed upload gives back what it allocated,
 // so the batch can be searched again later.
@@ -409,71 +426,114 @@ constexpr int kByteMinWarps = 2;
 int byte_cell(const hbg_batch *b, int32_t g) {
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
-    const uint32_t *cs = h.cells.data() + (size_t)g * HBG_CELL_STRIDE;
-    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow ||
-        G.max_count > hbg::kByteMaxCount || cs[HBG_NUM_CELLS] >= (uint32_t)hbg::kByteMaxEntries || b->repeated_entries)
+    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.max_count > hbg::kByteMaxCount ||
+        G.n_entries >= hbg::kByteMaxEntries || b->repeated_entries)
         return 0;
     return G.diag_len <= kByteTable16 ? 2 : 1;
 }
 
-int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
+// The launch classes of a batch and its groups in class order.
+int make_classes(hbg_batch *b, std::vector<int32_t> *list) {
     const hbg::HostBatch &h = b->host;
-    std::vector<int32_t> list;
-    {
-        // launch classes: (mode, table size); groups with shared tables are
-        // launched by table size, so a short query's warps reserve only the
-        // shared memory its table needs (the rest is L1 for cells and entries:
-        // one 350-aa query vs 10 M subjects 8 % faster than with 2048-entry
-        // tables for every group); global-table groups form their own class
-        std::vector<std::pair<std::array<int, 3>, int32_t>> keyed;
-        for (int32_t g = 0; g < (int32_t)h.groups.size(); ++g) {
-            const HbgGroup &G = h.groups[g];
-            const int size = G.placement ? 64 : std::max<int>(64, G.diag_len);
-            // byte_kernel's table, with the cell size in the low bits
-            const int cell = byte_cell(b, g);
-            keyed.push_back({{G.mode, size, cell ? 4 * std::max<int>(64, G.diag_len) + cell : 0}, g});
-        }
-        std::stable_sort(keyed.begin(), keyed.end(),
-                         [](const auto &x, const auto &y) { return x.first < y.first; });
-        b->classes.clear();
-        for (size_t i = 0; i < keyed.size(); ++i) {
-            const bool global = h.groups[keyed[i].second].placement != 0;
-            if (i == 0 || keyed[i].first != keyed[i - 1].first)
-                b->classes.push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
-                                                 keyed[i].first[2] & 3, keyed[i].first[2] / 4});
-            LaunchClass &lc = b->classes.back();
-            lc.count++;
-            if (lc.cell == 1)              // the longest group's exact table
-                lc.table_len = std::max(lc.count == 1 ? 0 : lc.table_len,
-                                        hbg::byte_table_len(h.groups[keyed[i].second].glen + h.window));
-            list.push_back(keyed[i].second);
-        }
-        if ((int)b->classes.size() > kMaxLaunchClasses)
-            return fail(HBG_ERR_INVALID, "too many launch classes");
+    // launch classes: (mode, table size); groups with shared tables are
+    // launched by table size, so a short query's warps reserve only the
+    // shared memory its table needs (the rest is L1 for cells and entries:
+    // one 350-aa query vs 10 M subjects 8 % faster than with 2048-entry
+    // tables for every group); global-table groups form their own class
+    std::vector<std::pair<std::array<int, 3>, int32_t>> keyed;
+    for (int32_t g = 0; g < (int32_t)h.groups.size(); ++g) {
+        const HbgGroup &G = h.groups[g];
+        const int size = G.placement ? 64 : std::max<int>(64, G.diag_len);
+        // byte_kernel's table, with the cell size in the low bits
+        const int cell = byte_cell(b, g);
+        keyed.push_back({{G.mode, size, cell ? 4 * std::max<int>(64, G.diag_len) + cell : 0}, g});
     }
-    // one block, one copy: the arrays in turn, 256-byte aligned; then the
-    // packed cells, made on the device.  (Ten copies of their own took 80 us.)
+    std::stable_sort(keyed.begin(), keyed.end(),
+                     [](const auto &x, const auto &y) { return x.first < y.first; });
+    list->clear();
+    b->classes.clear();
+    for (size_t i = 0; i < keyed.size(); ++i) {
+        const bool global = h.groups[keyed[i].second].placement != 0;
+        if (i == 0 || keyed[i].first != keyed[i - 1].first)
+            b->classes.push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
+                                             keyed[i].first[2] & 3, keyed[i].first[2] / 4});
+        LaunchClass &lc = b->classes.back();
+        lc.count++;
+        if (lc.cell == 1)              // the longest group's exact table
+            lc.table_len = std::max(lc.count == 1 ? 0 : lc.table_len,
+                                    hbg::byte_table_len(h.groups[keyed[i].second].glen + h.window));
+        list->push_back(keyed[i].second);
+    }
+    if ((int)b->classes.size() > kMaxLaunchClasses)
+        return fail(HBG_ERR_INVALID, "too many launch classes");
+    return HBG_OK;
+}
+
+// Entries the device block has room for, per letter of the batch: random
+// proteins have 17 at threshold 11 (30 at 10); more take a block of their own.
+constexpr int64_t kEntriesPerLetter = 40;
+
+int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
+    hbg::HostBatch &h = b->host;
+    const size_t ng = h.groups.size(), nq = h.queries.size();
+    std::vector<hbg::TableSegment> segs;
+    for (size_t g = 0; g < ng; ++g) {
+        HbgGroup &G = h.groups[g];
+        G.seg_base = (int32_t)segs.size();
+        for (int32_t q = G.first_query; q < G.first_query + G.n_queries; ++q) {
+            const int32_t at = h.queries[q].start, end = at + h.queries[q].len - HBG_WORD_SIZE + 1;
+            for (int32_t p = at; p == at || p < end; p += hbg::kTableSegment)
+                segs.push_back({(int32_t)g, q, p, std::min(end, p + hbg::kTableSegment)});
+        }
+        G.n_segs = (int32_t)segs.size() - G.seg_base;
+    }
+    const bool on_device = !b->caller_tables && h.cells.empty() && hbg::tables_fit((int64_t)segs.size());
+    if (!on_device)
+        ensure_tables(b);
+    std::vector<int32_t> list;
+    int rc = make_classes(b, &list);             // again below if a cell turns out too full
+    if (rc != HBG_OK)
+        return rc;
+    // one block, one copy: the arrays in turn, 256-byte aligned, then what the
+    // device makes itself.  (Ten copies of their own took 80 us.)
     std::vector<std::pair<size_t, std::pair<const void *, size_t>>> parts;   // place, source, bytes
     size_t at = 0;
     auto place = [&](const void *src, size_t bytes, size_t before, size_t after) {
         const size_t p = at + before;
-        parts.push_back({p, {src, bytes}});
+        if (src)
+            parts.push_back({p, {src, bytes}});
         at = (p + bytes + after + 255) / 256 * 256;
         return p;
     };
+    const size_t b_cells = ng * HBG_CELL_STRIDE * sizeof(uint32_t), b_pv = ng * HBG_PV_WORDS * sizeof(uint32_t),
+                 b_qcells = nq * HBG_NUM_CELLS * sizeof(uint16_t);
     // letters: kFrontPad zeros before (extensions read whole blocks), 64 after
-    const size_t o_groups = place(h.groups.data(), h.groups.size() * sizeof(HbgGroup), 0, 0);
+    const size_t o_groups = place(h.groups.data(), ng * sizeof(HbgGroup), 0, 0);
     const size_t o_ctx = place(h.contexts.data(), h.contexts.size() * sizeof(HbgContext), 0, 0);
-    const size_t o_queries = place(h.queries.data(), h.queries.size() * sizeof(HbgQueryDesc), 0, 0);
+    const size_t o_queries = place(h.queries.data(), nq * sizeof(HbgQueryDesc), 0, 0);
     const size_t o_letters = place(h.letters.data(), h.letters.size(), kFrontPad, 64);
     const size_t o_ctx_of = place(h.ctx_of.data(), h.ctx_of.size() * sizeof(int32_t), 0, 64);
-    const size_t o_cells = place(h.cells.data(), h.cells.size() * sizeof(uint32_t), 0, 0);
-    // byte_kernel reads up to 31 entries past a cell
-    const size_t o_entries = place(h.entries.data(), h.entries.size() * sizeof(uint16_t), 0, 128);
-    const size_t o_pv = place(h.pv.data(), h.pv.size() * sizeof(uint32_t), 0, 0);
-    const size_t o_qcells = place(h.query_cells.data(), h.query_cells.size() * sizeof(uint16_t), 0, 0);
     const size_t o_list = place(list.data(), list.size() * sizeof(int32_t), 0, 0);
+    const size_t o_segs = place(segs.data(), segs.size() * sizeof(hbg::TableSegment), 0, 0);
+    size_t o_cells = 0, o_pv = 0, o_qcells = 0, o_entries = 0;
+    if (!on_device) {
+        o_cells = place(h.cells.data(), b_cells, 0, 0);
+        o_pv = place(h.pv.data(), b_pv, 0, 0);
+        o_qcells = place(h.query_cells.data(), b_qcells, 0, 0);
+        o_entries = place(h.entries.data(), h.entries.size() * sizeof(uint16_t), 0, 128);
+    }
     const size_t upload = at;
+    const int64_t cap = std::max<int64_t>(1024, kEntriesPerLetter * (int64_t)h.letters.size());
+    // byte_kernel reads up to 31 entries past a cell
+    if (on_device) {
+        o_cells = place(nullptr, b_cells, 0, 0);
+        o_pv = place(nullptr, b_pv, 0, 0);
+        o_qcells = place(nullptr, b_qcells, 0, 0);
+        o_entries = place(nullptr, (size_t)cap * sizeof(uint16_t), 0, 128);
+    }
+    const size_t o_packed = place(nullptr, ng * HBG_NUM_CELLS * sizeof(uint32_t), 0, 0);
+    const size_t o_stats = place(nullptr, ng * sizeof(uint2), 0, 0);
+    const size_t o_counts = place(nullptr, on_device ? segs.size() * HBG_NUM_CELLS * sizeof(uint32_t) : 0, 0, 0);
     std::unique_ptr<uint8_t[]> stage(new (std::nothrow) uint8_t[upload]);
     if (!stage)
         return fail(HBG_ERR_NOMEM, "host allocation");
@@ -485,24 +545,55 @@ int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
         done = p.first + p.second.second;
     }
     memset(stage.get() + done, 0, upload - done);
-    CU(dalloc(&b->d_arena, upload + h.groups.size() * HBG_NUM_CELLS * sizeof(uint32_t)));
+    CU(dalloc(&b->d_arena, at));
     b->d_groups = reinterpret_cast<HbgGroup *>(b->d_arena + o_groups);
     b->d_ctx = reinterpret_cast<HbgContext *>(b->d_arena + o_ctx);
     b->d_queries = reinterpret_cast<HbgQueryDesc *>(b->d_arena + o_queries);
     b->d_letters = b->d_arena + o_letters;
     b->d_ctx_of = reinterpret_cast<int32_t *>(b->d_arena + o_ctx_of);
+    b->d_group_list = reinterpret_cast<int32_t *>(b->d_arena + o_list);
     b->d_cells = reinterpret_cast<uint32_t *>(b->d_arena + o_cells);
-    b->d_entries = reinterpret_cast<uint16_t *>(b->d_arena + o_entries);
     b->d_pv = reinterpret_cast<uint32_t *>(b->d_arena + o_pv);
     b->d_qcells = reinterpret_cast<uint16_t *>(b->d_arena + o_qcells);
-    b->d_group_list = reinterpret_cast<int32_t *>(b->d_arena + o_list);
-    b->d_packed = reinterpret_cast<uint32_t *>(b->d_arena + upload);
+    b->d_entries = reinterpret_cast<uint16_t *>(b->d_arena + o_entries);
+    b->d_packed = reinterpret_cast<uint32_t *>(b->d_arena + o_packed);
+    b->d_stats = reinterpret_cast<uint2 *>(b->d_arena + o_stats);
     cudaStream_t st = nullptr;
     CU(db->kits->upload_stream(&st));
     CU(cudaMemcpyAsync(b->d_arena, stage.get(), upload, cudaMemcpyHostToDevice, st));
-    CU(hbg::launch_pack_cells(b->d_cells, (int32_t)h.groups.size(), b->d_packed, st));
+    if (!on_device) {
+        CU(hbg::launch_pack_cells(b->d_cells, (int32_t)ng, b->d_packed, st));
+    } else {
+        hbg::TableArgs t{b->d_groups, reinterpret_cast<const hbg::TableSegment *>(b->d_arena + o_segs), b->d_letters,
+                         b->d_ctx_of, h.threshold, b->d_cells, b->d_packed, b->d_pv, b->d_entries, cap, b->d_qcells,
+                         b->d_stats, reinterpret_cast<uint32_t *>(b->d_arena + o_counts)};
+        const int32_t n_segs = (int32_t)segs.size();
+        std::vector<uint2> stats(ng);
+        CU(hbg::launch_tables(t, (int32_t)ng, n_segs, false, st));
+        CU(cudaMemcpyAsync(stats.data(), b->d_stats, ng * sizeof(uint2), cudaMemcpyDeviceToHost, st));
+        CU(cudaStreamSynchronize(st));
+        int64_t total = 0;
+        bool again = false;
+        for (size_t g = 0; g < ng; ++g) {
+            total += stats[g].x;
+            h.groups[g].n_entries = (int32_t)stats[g].x;
+            h.groups[g].max_count = (int32_t)stats[g].y;
+            again = again || (int32_t)stats[g].y > hbg::kByteMaxCount || (int32_t)stats[g].x >= hbg::kByteMaxEntries;
+        }
+        if (total > cap) {
+            CU(dalloc(&b->d_more, (size_t)total + 64));
+            b->d_entries = t.entries = b->d_more;
+            t.entries_cap = total;
+            CU(hbg::launch_tables(t, (int32_t)ng, n_segs, true, st));
+        }
+        if (again) {
+            rc = make_classes(b, &list);
+            if (rc != HBG_OK)
+                return rc;
+            CU(cudaMemcpyAsync(b->d_group_list, list.data(), list.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+        }
+    }
     CU(cudaStreamSynchronize(st));   // the search may run on any stream
-    b->device_bytes = batch_device_bytes(h);
     b->device = db->device;
     return HBG_OK;
 }
@@ -1496,6 +1587,8 @@ int hbg_batch_create_from_smallbone(const hbg_query *query, const hbg_word_param
     h.pv = pv;
     h.query_cells = qc;
     h.groups[0].entry_base = 0;
+    h.groups[0].n_entries = (int32_t)ents.size();
+    (*out)->caller_tables = true;
     return HBG_OK;
 bad:
     hbg_batch_destroy(*out);
@@ -1508,6 +1601,7 @@ int hbg_batch_lookup_table(const hbg_batch *b, int32_t g, uint32_t *cells, uint1
                            int32_t *n_queries, int32_t *query_start) {
     if (!b || !n_entries || g < 0 || g >= (int32_t)b->host.groups.size())
         return fail(HBG_ERR_INVALID, "hbg_batch_lookup_table: bad argument");
+    ensure_tables(b);
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
     const uint32_t *cs = h.cells.data() + (size_t)g * HBG_CELL_STRIDE;
@@ -1606,9 +1700,9 @@ int hbg_batch_info(const hbg_batch *b, int32_t *nq, int32_t *ng, int64_t *qlen, 
         *qlen = t;
     }
     if (entries)
-        *entries = (int64_t)b->host.entries.size();
+        *entries = batch_entries(b);
     if (device_bytes)
-        *device_bytes = batch_device_bytes(b->host);
+        *device_bytes = batch_device_bytes(b->host, batch_entries(b));
     return HBG_OK;
 }
 
@@ -1618,9 +1712,7 @@ int hbg_mem_required(const hbg_db *db, const hbg_batch *b, int64_t cap, int64_t 
     if (cap == 0)
         cap = default_capacity(db, b);
     const hbg::HostBatch &h = b->host;
-    int64_t batch_bytes = (int64_t)(h.letters.size() + h.ctx_of.size() * 4 + h.cells.size() * 4 +
-                                    h.entries.size() * 2 + h.pv.size() * 4 + h.query_cells.size() * 2 +
-                                    h.groups.size() * HBG_NUM_CELLS * 4);
+    const int64_t batch_bytes = batch_device_bytes(h, batch_entries(b));
     int64_t per_hsp = 2 * (int64_t)sizeof(hbg_hsp) + 2 * 8 + 2 * 4;
     int64_t gdiag = 0;
     if (global_diag_len(h, db) > 0) {

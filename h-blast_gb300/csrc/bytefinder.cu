@@ -632,14 +632,6 @@ __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
 
 namespace {
 
-// The cells of every group in one word each: first entry | count << 22.
-__global__ void __launch_bounds__(256)
-pack_cells(const uint32_t *cells, uint32_t *packed) {
-    const uint32_t *cs = cells + (size_t)blockIdx.y * HBG_CELL_STRIDE;
-    const int w = blockIdx.x * 256 + threadIdx.x;
-    packed[(size_t)blockIdx.y * HBG_NUM_CELLS + w] = cs[w] | ((cs[w + 1] - cs[w]) << 22);
-}
-
 const void *byte_kernel_of(int cell_bytes) {
     return cell_bytes == 1 ? (const void *)byte_kernel<uint8_t> : (const void *)byte_kernel<uint16_t>;
 }
@@ -667,15 +659,6 @@ cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threa
     void *params[] = {&args};
     return cudaLaunchKernel(byte_kernel_of(cell_bytes), dim3((unsigned)blocks), dim3((unsigned)threads), params,
                             byte_smem_bytes(cell_bytes, threads, a.table_len), stream);
-}
-
-cudaError_t launch_pack_cells(const uint32_t *cells, int32_t n_groups, uint32_t *packed, cudaStream_t stream) {
-    for (int32_t g0 = 0; g0 < n_groups; g0 += 65535) {   // grid.y limit
-        const int32_t n = n_groups - g0 < 65535 ? n_groups - g0 : 65535;
-        pack_cells<<<dim3(HBG_NUM_CELLS / 256, n), 256, 0, stream>>>(cells + (size_t)g0 * HBG_CELL_STRIDE,
-                                                                     packed + (size_t)g0 * HBG_NUM_CELLS);
-    }
-    return cudaGetLastError();
 }
 
 }  // namespace hbg

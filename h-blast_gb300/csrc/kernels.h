@@ -104,6 +104,31 @@ __host__ __device__ constexpr int byte_table_len(int letters) { return (letters 
 size_t byte_smem_bytes(int cell_bytes, int threads, int table_len);
 cudaError_t byte_configure();
 cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threads, cudaStream_t stream);
+
+// The lookup tables of a batch (tables.cu): from letters, contexts and queries
+// to cells, presence vectors, packed cells, entries and per-query cell counts.
+struct TableSegment {             // letters of one query, up to kTableSegment words
+    int32_t group, query;         // of the batch
+    int32_t begin, end;           // group-local offsets of its words
+};
+constexpr int kTableSegment = 512;
+struct TableArgs {
+    HbgGroup *groups;             // entry_base is written
+    const TableSegment *segs;     // in query order; a group's are seg_base ..
+    const uint8_t *letters;
+    const int32_t *ctx_of;
+    int32_t threshold;
+    uint32_t *cells;
+    uint32_t *packed;
+    uint32_t *pv;
+    uint16_t *entries;
+    int64_t entries_cap;          // a group whose entries would pass it is not filled
+    uint16_t *query_cells;
+    uint2 *stats;                 // per group: entries, fullest cell
+    uint32_t *counts;             // scratch: HBG_NUM_CELLS per segment
+};
+bool tables_fit(int64_t n_segs);
+cudaError_t launch_tables(const TableArgs &a, int32_t n_groups, int32_t n_segs, bool fill_only, cudaStream_t stream);
 cudaError_t launch_pack_cells(const uint32_t *cells, int32_t n_groups, uint32_t *packed, cudaStream_t stream);
 
 // Ordering pass: sort HSPs by (query, subject, subject offset, query offset),

@@ -257,31 +257,63 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
         seq_pos += glen;
     }
 
-    // --- lookup tables: count, then fill ---
-    NeighbourCache &nb = neighbour_cache(threshold);
+    b.mode_hits = mode_hits;
+    if (mode_hits < kOffsetModeHits)             // the hit mode depends on the tables
+        build_tables(out);
+    return std::string();
+}
+
+namespace {
+
+// A word is stored when its three letters lie inside one context.
+bool valid(const int32_t *gc, int32_t p) {
+    const int32_t c0 = gc[p];
+    return c0 >= 0 && gc[p + 1] == c0 && gc[p + 2] == c0;
+}
+
+// The neighbourhoods of every word in the batch, enumerated in parallel.
+NeighbourCache &prepared_cache(const HostBatch &b) {
+    NeighbourCache &nb = neighbour_cache(b.threshold);
+    std::vector<int32_t> words;
+    words.reserve(b.letters.size());
+    for (const HbgGroup &G : b.groups) {
+        const uint8_t *gs = b.letters.data() + G.seq_base;
+        const int32_t *gc = b.ctx_of.data() + G.seq_base;
+        for (int32_t p = 0; p + HBG_WORD_SIZE <= G.glen; ++p)
+            if (valid(gc, p))
+                words.push_back((gs[p] << 10) | (gs[p + 1] << 5) | gs[p + 2]);
+    }
+    nb.prepare(words, parallel_for);
+    return nb;
+}
+
+}  // namespace
+
+int64_t count_entries(const HostBatch &b) {
+    if (!b.cells.empty())
+        return (int64_t)b.entries.size();
+    const NeighbourCache &nb = prepared_cache(b);
+    int64_t n = 0;
+    for (const HbgGroup &G : b.groups) {
+        const uint8_t *gs = b.letters.data() + G.seq_base;
+        const int32_t *gc = b.ctx_of.data() + G.seq_base;
+        for (int32_t p = 0; p + HBG_WORD_SIZE <= G.glen; ++p)
+            if (valid(gc, p))
+                n += (int64_t)nb.get(gs[p], gs[p + 1], gs[p + 2]).size();
+    }
+    return n;
+}
+
+// Count, then fill, per group (in parallel: groups own disjoint cells, queries
+// and entries).
+void build_tables(HostBatch *out) {
+    HostBatch &b = *out;
+    const int32_t n_groups = (int32_t)b.groups.size();
+    const double mode_hits = b.mode_hits;
+    const NeighbourCache &nb = prepared_cache(b);
     b.cells.assign((size_t)n_groups * HBG_CELL_STRIDE, 0);
     b.pv.assign((size_t)n_groups * HBG_PV_WORDS, 0);
-    b.query_cells.assign(qs.size() * (size_t)HBG_NUM_CELLS, 0);
-    // the neighbourhoods of every word in the batch, enumerated in parallel;
-    // then per group (in parallel: groups own disjoint cells, queries and
-    // entries) count, prefix, and fill
-    auto valid = [&](const int32_t *gc, int32_t p) {
-        const int32_t c0 = gc[p];
-        return c0 >= 0 && gc[p + 1] == c0 && gc[p + 2] == c0;
-    };
-    {
-        std::vector<int32_t> words;
-        words.reserve(b.letters.size());
-        for (int32_t g = 0; g < n_groups; ++g) {
-            const HbgGroup &G = b.groups[g];
-            const uint8_t *gs = b.letters.data() + G.seq_base;
-            const int32_t *gc = b.ctx_of.data() + G.seq_base;
-            for (int32_t p = 0; p + HBG_WORD_SIZE <= G.glen; ++p)
-                if (valid(gc, p))
-                    words.push_back((gs[p] << 10) | (gs[p + 1] << 5) | gs[p + 2]);
-        }
-        nb.prepare(words, parallel_for);
-    }
+    b.query_cells.assign(b.queries.size() * (size_t)HBG_NUM_CELLS, 0);
     std::vector<uint32_t> group_entries(n_groups, 0);
     parallel_for(n_groups, [&](int64_t gi) {
         const int32_t g = (int32_t)gi;
@@ -311,6 +343,7 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
         }
         cs[HBG_NUM_CELLS] = acc;
         group_entries[g] = acc;
+        G.n_entries = (int32_t)acc;
         G.max_count = (int32_t)most;
         // expected hits per subject offset on typical proteins: entries of
         // words over the 20 standard letters, each such word taken as
@@ -324,7 +357,8 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
                     for (int z = 0; z < 20; ++z)
                         std_entries += count[(kStd[x] << 10) | (kStd[y] << 5) | kStd[z]];
         }
-        G.mode = (double)std_entries / 8000.0 >= mode_hits ? 1 : 0;
+        if (mode_hits < kOffsetModeHits)
+            G.mode = (double)std_entries / 8000.0 >= mode_hits ? 1 : 0;
     });
     int64_t entry_pos = 0;
     for (int32_t g = 0; g < n_groups; ++g) {
@@ -349,7 +383,6 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
                 ge[cursor[w]++] = (uint16_t)p;
         }
     });
-    return std::string();
 }
 
 // --- six-frame translation ------------------------------------------------

@@ -47,6 +47,7 @@ struct HostBatch {
     std::vector<HbgQueryDesc> queries;
     std::vector<uint8_t> letters;        // all groups, gaps included
     std::vector<int32_t> ctx_of;         // per letter, -1 outside contexts
+    // lookup tables: empty until build_tables
     std::vector<uint32_t> cells;         // groups x HBG_CELL_STRIDE
     std::vector<uint16_t> entries;       // group-local query offsets
     std::vector<uint32_t> pv;            // groups x HBG_PV_WORDS
@@ -54,6 +55,7 @@ struct HostBatch {
     int32_t max_query_len = 0;
     int32_t max_diag_len = 0;            // over groups with global placement
     int32_t smem_diag_len = 64;          // per-warp shared table: max over shared-placed groups
+    double mode_hits = 0;                // offset-mode threshold
 };
 
 // One query already in NCBI concatenated form.
@@ -63,12 +65,18 @@ struct QueryIn {
     std::vector<int32_t> ctx_off, ctx_len, xdrop, cutoff;
 };
 
+// Packs the queries into groups; the lookup tables come later (build_tables).
 // Returns an empty string on success, else the reason.
 // max_group_len 0 = default; mode_hits < 0 = default offset-mode threshold,
 // 0 = offset mode for every group, a huge value = chunk mode for every group.
 std::string build_batch(const std::vector<QueryIn> &queries, int32_t threshold,
                         int32_t window, int32_t max_group_len, HostBatch *out,
                         double mode_hits = -1.0);
+
+// The lookup tables of a batch on the host; searches build theirs on the device.
+void build_tables(HostBatch *b);
+// Lookup entries the tables hold, without building them.
+int64_t count_entries(const HostBatch &b);
 
 // Standard-code six-frame translation (frames +1,+2,+3,-1,-2,-3, one sentinel
 // between frames).  Returns the concatenated letters; fills offsets/lengths.

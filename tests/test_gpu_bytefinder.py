@@ -123,3 +123,24 @@ def test_groups_of_different_lengths(built):
     pqs = [hblast.ProteinQuery.blastp(q) for q in qs]
     check(hblast.search(hblast.Database(db.residues, db.offsets), hblast.Batch.proteins(pqs)), pqs, db.residues,
           db.offsets, threads=16)
+
+
+@pytest.mark.parametrize("threshold,qlens", [(8, (300,)), (9, (700, 40, 3, 2)), (11, (33, 34, 35, 1500)), (14, (64, 65)),
+                                             (30, (50,)), (-400, (3, 5))])
+def test_device_built_tables(built, threshold, qlens):
+    """Lookup tables built on the device, from thresholds whose entries outgrow
+    the block they are given (-400: every word of 28 letters is a neighbour) to
+    none at all: hits, extensions and HSPs as the oracle finds them."""
+    rng = np.random.default_rng(threshold + 1000)
+    qs = [synth.random_letters(rng, n) for n in qlens]
+    res, off = database(rng, qs[0] if len(qs[0]) > 10 else synth.random_letters(rng, 90))
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 20) for q in qs]
+    got = hblast.search(hblast.Database(res, off), hblast.Batch.proteins(pqs, threshold=threshold))
+    for k, q in enumerate(qs):
+        ref, subj, cnt = oracle.search(oracle.Query.blastp(q, 16, 20), res, off, threshold=threshold)
+        h = got.hsps[got.hsps["query"] == k]
+        assert len(h) == len(ref) and np.array_equal(h["subject"], subj)
+        for f in ("q_start", "s_start", "q_off", "s_off", "len", "score"):
+            assert np.array_equal(h[f], ref[f]), f
+        st = got.stats[k]
+        assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
