@@ -410,9 +410,9 @@ int upload_batch(hbg_batch *b, const hbg_db *db) {
 }
 
 // Longest diagonal tables byte_kernel keeps in 16-bit cells: 4096 entries leave
-// room for 22 warps per SM (9.2 ms for a 4056-letter query against 400,000
-// subjects; 8-bit cells, 24 warps: 10.3 ms, the sweeps cut its rounds of
-// extensions short).  Longer tables take 8-bit cells (8152 letters against
+// room for 22 warps per SM (a 4056-letter query against 400,000 subjects: 9.2
+// ms; 8-bit cells, 24 warps: 10.3 ms, the sweeps cut its rounds of extensions
+// short).  Longer tables take 8-bit cells (8152 letters against
 // 200,000 subjects: 9.5 ms, 12.2 ms with 16-bit cells and 12 warps).
 constexpr int kByteTable16 = 4096;
 // Fewest warps per SM it is used with.  Against 20,000 subjects, ms here and

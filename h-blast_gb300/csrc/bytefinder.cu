@@ -25,11 +25,13 @@
 // The rules are NCBI aa_ungapped.c's two-hit state machine (H-BLAST
 // h_blast_kernel.cu:672-871); the extension is in extend.h.
 //
-// What bounds it: issued instructions (3.0 of 4 per cycle).  One 4056-letter
-// query against 400,000 subjects (1.22e9 hits): 9.2 ms, 1.33e11 hits/s, 13.9 ms
-// with wordfinder_kernel; of about 250 warp instructions per batch of 32 hits
-// the extensions take 85, the batch itself 50, shared diagonals 35, scanning
-// and locating 45.  DRAM traffic is the subject letters once per group.
+// What bounds it: issued instructions (3.0 of 4 per cycle); 24 warps of 80
+// registers (32 of 64 spill: 2 % faster for one 350-letter query against 400,000
+// subjects, 20 % slower against 20,000, where a warp's latency counts).  One 4056-letter
+// query against 400,000 subjects (1.22e9 hits): 8.9 ms, 1.37e11 hits/s, 13.9 ms
+// with wordfinder_kernel; of 223 warp instructions per batch of 32 hits the
+// extensions take 93 (75 of them the walks), shared diagonals 22, scanning,
+// locating and the common case 107.  DRAM traffic is the subject letters once per group.
 #include <cuda_runtime.h>
 #include <stddef.h>
 
@@ -242,11 +244,13 @@ __device__ __forceinline__ void apply_hits(const Item<Cell> &it, Queues &W, bool
     const bool shared = t != pos;
     const bool hard = v >= K::kFlag ||
                       (shared && ((unsigned)(t - pos + 1) > 2u || trig || (unsigned)(t - v - 3) < it.span));
+    bool store = (Full || act) && (shared ? reset && pos < t : nv != pos);
     if (__any_sync(kAll, hard)) {
         apply_chains(it, W, Full || act, d, s_h, q, v, nv, diff, trig);
-    } else if ((Full || act) && (shared ? reset && pos < t : nv != pos)) {
-        cell = (Cell)nv;
+        store = false;
     }
+    if (store)
+        cell = (Cell)nv;
     trig = (Full || act) && trig;
     const unsigned tm = __ballot_sync(kAll, trig);
     if (trig)
@@ -268,6 +272,7 @@ __device__ __noinline__ Queues flush(const Item<Cell> it, const ByteArgs &a, Que
     using K = Cells<Cell>;
     Head &hd = *reinterpret_cast<Head *>(g_byte_smem);
     const int lane = threadIdx.x & 31;
+    const Letters subject = letters_of(it.s), group = letters_of(it.gseq);
     do {
         const int first = (!drain && W.n_tasks > 32) ? W.n_tasks - 32 : 0;
         for (int t0 = first; t0 < W.n_tasks; t0 += 32) {
@@ -279,8 +284,8 @@ __device__ __noinline__ Queues flush(const Item<Cell> it, const ByteArgs &a, Que
                 const HbgContext C = a.contexts[ci];
                 const HbgQueryDesc Q = a.queries[C.query];
                 const int ql = q - Q.start;
-                const Ext e = extend_two_hit(hd.matrix, it.s, it.S, it.gseq + Q.start, Q.len, s_h - (int)task.y + 3, s_h,
-                                             ql, C.x_dropoff);
+                const Ext e = extend_two_hit(hd.matrix, subject, it.S, group, Q.start, Q.len, s_h - (int)task.y + 3, s_h, ql,
+                                             C.x_dropoff);
                 atomicAdd(&hd.q_ext[C.query - it.first_query], 1u);
                 if (e.score >= C.cutoff) {
                     atomicAdd(&hd.q_kept[C.query - it.first_query], 1u);
@@ -646,8 +651,8 @@ cudaError_t byte_configure() {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    for (int c = 1; c <= 2; ++c) {
-        cudaError_t e = cudaFuncSetAttribute(byte_kernel_of(c), cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+    for (const void *k : {byte_kernel_of(1), byte_kernel_of(2)}) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (e != cudaSuccess)
             return e;
     }

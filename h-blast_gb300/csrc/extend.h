@@ -23,15 +23,23 @@ __device__ __forceinline__ void load_scores(Score *m, const int8_t *blosum, int 
     m[i] = (Score)(kScoreScale * blosum[i] - 1);
 }
 
-// scaled sum -> prefix score, for 1..15 letters taken
-__device__ __forceinline__ int unscaled(int x) { return (x + kScoreScale - 1) >> 4; }
+// A sequence by an aligned base (the same in all lanes of a warp) and 32-bit
+// offsets from it; the base lies 64 letters before the first one, so that the
+// blocks that reach past the start have offsets too.
+struct Letters {
+    const uint32_t *base;
+    unsigned first;                          // offset of letter 0
+};
+__device__ __forceinline__ Letters letters_of(const uint8_t *p) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p) - 64;
+    return Letters{reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3), 64u + (unsigned)(a & 3)};
+}
 
-// Eight letters from p (any alignment), as two words: three aligned 32-bit
-// loads and two funnel shifts.  Reads the aligned words that hold the letters.
-__device__ __forceinline__ uint2 load8(const uint8_t *p) {
-    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
-    const uint32_t sh = (uint32_t)a * 8;     // funnel shifts take it modulo 32
+// Eight letters from offset `at` (any alignment), as two words: three aligned
+// 32-bit loads and two funnel shifts.  Reads the aligned words that hold them.
+__device__ __forceinline__ uint2 load8(const uint32_t *base, unsigned at) {
+    const uint32_t *w = base + (at >> 2);
+    const uint32_t sh = at * 8;              // funnel shifts take it modulo 32
     const uint32_t w0 = __ldg(w), w1 = __ldg(w + 1), w2 = __ldg(w + 2);
     return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
 }
@@ -78,27 +86,12 @@ __device__ __forceinline__ void walk8(Walk &w, const int *x, int taken, int drop
     const int top = max8(p), low = min8(p);
     w.score = p[7] + 8;
     *adv = 8;
-    // 16 (largest prefix) is in top + 1 .. top + 8, 16 (smallest) in low + 1 .. low + 8
-    const bool up = top + 8 >= w.best + kScoreScale;
-    if (!up) {
-        // nothing better in this block, so the best so far decides about the end
-        if (Right) {
-            const int limit = max(w.best - drop, 0);
-            if (low < limit || low <= 0) {
-#pragma unroll
-                for (int i = 7; i >= 0; --i)
-                    *adv = p[i] < limit ? i : *adv;
-                w.stop = *adv < 8;
-            }
-        } else {
-            w.stop = w.best - unscaled(low) * kScoreScale >= drop;
-        }
-    } else if (max(w.best, top + 8) - low < drop && (!Right || low > 0)) {
-        // the walk cannot end in this block
-        const int b = unscaled(top) * kScoreScale;
-        w.best_len = taken + (b - top);
-        w.best = b;
-    } else {
+    // 16 (largest prefix) is in top + 1 .. top + 8, so it beats the best if top
+    // + 8 reaches the next score; 16 (a prefix) <= limit if and only if its sum
+    // is below limit, for any limit that is a multiple of 16
+    const bool up = top >= w.best + (kScoreScale - 8);
+    if (up && (top - low >= drop - 8 || (Right && low <= 0))) {
+        // better, and perhaps the end: letter by letter
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int c = p[i] + i + 1;
@@ -108,6 +101,18 @@ __device__ __forceinline__ void walk8(Walk &w, const int *x, int taken, int drop
             const bool end = !w.stop && i >= skip && ((Right && c <= 0) || w.best - c >= drop);
             *adv = end ? i : *adv;
             w.stop = w.stop || end;
+        }
+    } else {
+        // nothing better: the best so far decides about the end; better: no end
+        const int limit = Right ? max(w.best - drop, 0) : w.best - drop;
+        const int b = (top + kScoreScale - 1) & -kScoreScale;
+        w.stop = !up && low < limit;
+        w.best_len = up ? taken + (b - top) : w.best_len;
+        w.best = up ? b : w.best;
+        if (Right && w.stop) {
+#pragma unroll
+            for (int i = 7; i >= 0; --i)
+                *adv = p[i] < limit ? i : *adv;
         }
     }
 }
@@ -126,20 +131,21 @@ struct Ext {
     bool right;
 };
 
-// The extension of a second hit (word at s_h, q_h) whose first hit's word ends
-// before s_left: the best prefix of the word, the walk to the left from its
+// The extension of a second hit (word at s_h, q_h; the query's letters start at
+// q_start of G) whose first hit's word ends before s_left: the best prefix of the word, the walk to the left from its
 // end, and the walk to the right if the left one reached the first hit.  The
 // first block of the left walk holds the word.  Reads up to 8 letters before
 // and 11 after the sequences' ends (the letter buffers are padded).
-__device__ __forceinline__ Ext extend_two_hit(const Score *m, const uint8_t *s, int s_len, const uint8_t *q, int q_len,
-                                              int s_left, int s_h, int q_h, int dropoff) {
+__device__ __forceinline__ Ext extend_two_hit(const Score *m, const Letters &S, int s_len, const Letters &G, int q_start,
+                                              int q_len, int s_left, int s_h, int q_h, int dropoff) {
+    const unsigned s0 = S.first + (unsigned)s_h - 5u, q0 = G.first + (unsigned)(q_start + q_h) - 5u;
     const int drop = kScoreScale * dropoff;
     Walk w{0, 0, 0, false};
     int x[8], y[8], adv;
     const int n_left = min(s_h, q_h) + 3;    // letters up to the end of the word
     int skip, k = 0;
     {
-        const uint2 sw = load8(s + s_h - 5), qw = load8(q + q_h - 5);
+        const uint2 sw = load8(S.base, s0), qw = load8(G.base, q0);
         score4(m, qw.x, sw.x, y);
         score4(m, qw.y, sw.y, y + 4);
         // prefixes of the word, as 16 (score) - (letters): the largest, first one wins
@@ -157,7 +163,7 @@ __device__ __forceinline__ Ext extend_two_hit(const Score *m, const uint8_t *s, 
         walk8<false>(w, x, 0, drop, skip, &adv);
     }
     for (k = 8; !w.stop && k < n_left; k += 8) {
-        const uint2 sw = load8(s + s_h - 5 - k), qw = load8(q + q_h - 5 - k);
+        const uint2 sw = load8(S.base, s0 - (unsigned)k), qw = load8(G.base, q0 - (unsigned)k);
         score4(m, qw.x, sw.x, y);
         score4(m, qw.y, sw.y, y + 4);
 #pragma unroll
@@ -180,7 +186,8 @@ __device__ __forceinline__ Ext extend_two_hit(const Score *m, const uint8_t *s, 
         w.stop = false;
         int i = 0;
         while (!w.stop && i < n) {
-            const uint2 sw = load8(s + s_r + i), qw = load8(q + q_r + i);
+            const uint2 sw = load8(S.base, s0 + 8u - (unsigned)skip + (unsigned)i),
+                        qw = load8(G.base, q0 + 8u - (unsigned)skip + (unsigned)i);
             score4(m, qw.x, sw.x, x);
             score4(m, qw.y, sw.y, x + 4);
             cut8(x, n - i);

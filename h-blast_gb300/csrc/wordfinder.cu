@@ -241,7 +241,7 @@ __device__ void flush(const Item<Cell> &it, const WordFinderArgs &a, Slot &sh, W
                 const HbgContext C = a.contexts[ci];
                 const HbgQueryDesc Q = a.queries[C.query];
                 const int ql = q - Q.start;
-                const Ext e = extend_two_hit(score_matrix(), it.s, it.S, it.gseq + Q.start, Q.len,
+                const Ext e = extend_two_hit(score_matrix(), letters_of(it.s), it.S, letters_of(it.gseq), Q.start, Q.len,
                                              wq.task_left[i], s_h, ql, C.x_dropoff);
                 atomicAdd(&sh.q_ext[C.query - it.first_query], 1u);
                 if (e.score >= C.cutoff) {
