@@ -21,8 +21,10 @@ namespace {
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kOrderThreads = 1024;
 constexpr int kWarps = kOrderThreads / 32;
-// Up to this many HSPs every one is ranked against all others.
-constexpr int kRankMax = 4096;
+// Up to kRankMax HSPs every one is ranked against all others; up to kRankAlone
+// the same counts give the per-query ranges, and no CTA waits for another.
+constexpr int kRankAlone = 1024;
+constexpr int kRankMax = 16384;
 constexpr int kItems = 8;                     // per thread and scatter round
 constexpr int kRound = kOrderThreads * kItems;
 constexpr int kPart = 1024;                   // fewest items worth a CTA of the radix sort (8192: 130 us for 16,000, 1024: 73)
@@ -35,6 +37,9 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 }
 
 struct OrderSmem {
+    uint32_t base[256];                       // next place of a digit's items of this CTA
+    uint32_t scan[8];
+    int ok, pad;
     union {
         uint64_t keys[kRankMax];
         struct {
@@ -42,10 +47,8 @@ struct OrderSmem {
             uint32_t before[4][256], total[4][256];
         } r;
     };
-    uint32_t base[256];                       // next place of a digit's items of this CTA
-    uint32_t scan[8];
-    int ok;
 };
+extern __shared__ __align__(16) unsigned char g_order_smem[];
 
 __device__ __forceinline__ uint64_t key_of(const OrderArgs &a, const hbg_hsp &h) {
     uint64_t k = (uint64_t)(uint32_t)h.query;
@@ -78,11 +81,11 @@ __device__ bool grid_barrier(const OrderArgs &a, OrderSmem &sm, int grid, unsign
     return sm.ok != 0;
 }
 
-// One HSP's place among all n <= kRankMax is the number of smaller keys; keys
+// An HSP's place among all n <= kRankAlone is the number of smaller keys; keys
 // are distinct (a second hit starts one extension).  The same count for the
 // bounds of its query and of its subject tells whether it is the first or last
 // of them.
-__device__ void rank_all(const OrderArgs &a, OrderSmem &sm, int n) {
+__device__ void rank_alone(const OrderArgs &a, OrderSmem &sm, int n) {
     const int lane = threadIdx.x & 31;
     if ((int)blockIdx.x * kWarps >= n)
         return;
@@ -121,6 +124,57 @@ __device__ void rank_all(const OrderArgs &a, OrderSmem &sm, int n) {
             if (below == below_s)
                 atomicAdd(a.q_passed + q, 1ull);
         }
+    }
+}
+
+// The same for n <= kRankMax, two HSPs to a warp at a time; the ranges come from
+// the ordered records, after a barrier.
+__device__ void rank_all(const OrderArgs &a, OrderSmem &sm, int n) {
+    const int lane = threadIdx.x & 31;
+    for (int i = threadIdx.x; i < n; i += kOrderThreads)
+        sm.keys[i] = key_of(a, a.in[i]);
+    __syncthreads();
+    const int step = gridDim.x * kWarps;
+    for (int i = blockIdx.x * kWarps + (threadIdx.x >> 5); i < n; i += 2 * step) {
+        const int i2 = i + step < n ? i + step : i;
+        const uint64_t key = sm.keys[i], key2 = sm.keys[i2];
+        int below = 0, below2 = 0;
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) {
+            const uint64_t k = sm.keys[j];
+            below += k < key;
+            below2 += k < key2;
+        }
+        below = __reduce_add_sync(kAll, below);
+        below2 = __reduce_add_sync(kAll, below2);
+        if (lane < (int)(sizeof(hbg_hsp) / 4)) {
+            reinterpret_cast<int32_t *>(a.out + below)[lane] = reinterpret_cast<const int32_t *>(a.in + i)[lane];
+            reinterpret_cast<int32_t *>(a.out + below2)[lane] = reinterpret_cast<const int32_t *>(a.in + i2)[lane];
+        }
+    }
+    if (!a.q_first)
+        return;
+    unsigned long long target = 0;
+    if (!grid_barrier(a, sm, gridDim.x, target))
+        return;
+    for (int i0 = blockIdx.x * kOrderThreads; i0 < n; i0 += gridDim.x * kOrderThreads) {
+        const int i = i0 + threadIdx.x;
+        const bool on = i < n;
+        int q = -1;
+        bool fresh = false;
+        if (on) {
+            q = __ldcg(&a.out[i].query);
+            const bool new_q = i == 0 || __ldcg(&a.out[i - 1].query) != q;
+            if (new_q)
+                a.q_first[q] = (unsigned long long)i;
+            if (i == n - 1 || __ldcg(&a.out[i + 1].query) != q)
+                a.q_end[q] = (unsigned long long)(i + 1);
+            fresh = new_q || __ldcg(&a.out[i - 1].subject) != __ldcg(&a.out[i].subject);
+        }
+        const unsigned same = __match_any_sync(kAll, q);
+        const unsigned cnt = __popc(__ballot_sync(kAll, fresh) & same);
+        if (on && cnt && lane == __ffs(same) - 1)
+            atomicAdd(a.q_passed + q, (unsigned long long)cnt);
     }
 }
 
@@ -306,17 +360,19 @@ __device__ void count_hits(const OrderArgs &a, OrderSmem &sm) {
     }
 }
 
-// The ordering pass in one launch, bound by its grid barriers (two per 8 bits of
-// the key) until the items are many.  A dozen HSPs 9 us, 570 11 us, 50,000
-// 120 us, 1.4 M 397 us; as 25 launches of separate passes 107, 130, 237 and
-// 893 us.  Ranking against all others is the quicker way up to about 4096
-// (a fourth of the work at each halving; 15 us there), and needs no barrier.
+// The ordering pass in one launch.  A dozen HSPs 9 us, 570 10 us, 9155 27 us
+// (sorted: 72), 16,000 64 us, 50,000 115 us, 1.4 M 397 us; as 25 launches of
+// separate passes 107, 130, 214, -, 237 and 893 us.  The sort is bound by its
+// grid barriers and block-wide steps (ten us per 8 bits of the key) until the
+// items are many.
 __global__ void __launch_bounds__(kOrderThreads, 1) order_kernel(OrderArgs a) {
-    __shared__ OrderSmem sm;
+    OrderSmem &sm = *reinterpret_cast<OrderSmem *>(g_order_smem);
     count_hits(a, sm);
     const unsigned long long c = *a.count;
     const int64_t n = (int64_t)(c < (unsigned long long)a.cap ? c : (unsigned long long)a.cap);
-    if (n <= kRankMax)
+    if (n <= kRankAlone)
+        rank_alone(a, sm, (int)n);
+    else if (n <= kRankMax)
         rank_all(a, sm, (int)n);
     else
         radix_all(a, sm, n);
@@ -386,7 +442,11 @@ int order_grid(int device) {
 cudaError_t launch_order(const OrderArgs &a, int grid, cudaStream_t stream) {
     OrderArgs args = a;
     void *params[] = {&args};
-    return cudaLaunchCooperativeKernel((const void *)order_kernel, dim3((unsigned)grid), dim3(kOrderThreads), params, 0, stream);
+    cudaError_t e = cudaFuncSetAttribute(order_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(OrderSmem));
+    if (e != cudaSuccess)
+        return e;
+    return cudaLaunchCooperativeKernel((const void *)order_kernel, dim3((unsigned)grid), dim3(kOrderThreads), params,
+                                       sizeof(OrderSmem), stream);
 }
 
 cudaError_t launch_spread_letters(const uint8_t *raw, int64_t from, int64_t count, const int64_t *first, int32_t n,

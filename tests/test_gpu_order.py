@@ -11,7 +11,8 @@ from hblast import synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("k,nq", [(1, 1), (31, 1), (4095, 1), (4096, 1), (4097, 1), (1365, 3), (1366, 3), (8193, 1), (3001, 7),
+@pytest.mark.parametrize("k,nq", [(1, 1), (31, 1), (1024, 1), (1025, 1), (341, 3), (342, 3), (4863, 1), (4865, 2), (16383, 1),
+                                  (16384, 1), (16385, 1), (8192, 2), (3001, 7),
                                   (70001, 2), (1300003, 1)])
 def test_order_of_known_hsps(built, k, nq):
     q = synth.random_letters(np.random.default_rng(3), 60)
