@@ -1,4 +1,4 @@
-// extend.h -- the ungapped X-drop extension shared by the word-finder kernels
+// extend.h -- the ungapped X-drop extension of byte_kernel (bytefinder.cu)
 // (s_BlastAaExtendTwoHit/Left/Right; H-BLAST h_blast_kernel.cu:1069-1540, with
 // the left walk also taken when min(s, q) == 0 as NCBI does).
 #ifndef HBG_EXTEND_H
@@ -202,12 +202,6 @@ __device__ __forceinline__ Ext extend_two_hit(const Score *m, const Letters &S, 
     e.len = left_d + rlen;
     e.score = (e.right ? w.best : left_score) / kScoreScale;
     return e;
-}
-
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned r;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(r));
-    return r;
 }
 
 }  // namespace

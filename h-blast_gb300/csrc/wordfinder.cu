@@ -25,11 +25,11 @@
 // scratch for groups (or subjects) too long for it.
 //
 // The per-hit rule is the two-hit state machine of NCBI aa_ungapped.c, which
-// H-BLAST restates at h_blast_kernel.cu:672-871; the extension is in
-// extend.h.
+// H-BLAST restates at h_blast_kernel.cu:672-871; the extension is
+// s_BlastAaExtendTwoHit/Left/Right (h_blast_kernel.cu:1069-1540), with the
+// left walk also taken when min(s, q) == 0 as NCBI does.
 #include <cuda_runtime.h>
 
-#include "extend.h"
 #include "kernels.h"
 
 namespace hbg {
@@ -50,7 +50,7 @@ __constant__ int8_t c_blosum[28 * 32] = {
 extern __shared__ __align__(16) unsigned char g_smem[];
 
 struct __align__(16) Head {
-    Score matrix[28 * 32];    // scaled BLOSUM62, query letter x 32 + subject letter
+    int8_t matrix[28 * 32];   // BLOSUM62, query letter x 32 + subject letter
     long long tile;
     long long pad;
 };
@@ -64,8 +64,149 @@ struct __align__(16) Slot {
     int group;                   // group index, -1 when the tile has none for this slot
 };
 
-__device__ __forceinline__ const Score *score_matrix() { return reinterpret_cast<const Head *>(g_smem)->matrix; }
+__device__ __forceinline__ const int8_t *score_matrix() { return reinterpret_cast<const Head *>(g_smem)->matrix; }
 
+// This kernel walks four letters at a time, byte_kernel eight (extend.h): the
+// longer walk needs registers that four CTAs per SM do not leave (64 a thread;
+// 280 bytes of spills instead of 28).  Word finder, ms, with this walk and with
+// the longer one: 4056 letters against 400,000 subjects 13.97 / 14.84, 350
+// letters with window 100 2.55 / 2.73, six groups of 500 letters searched four
+// to a pass over 100,000 subjects 12.9 / 14.5; only 20,000 letters against 20,000
+// subjects is better off with the longer one, 26.4 / 25.7.
+__device__ __forceinline__ int sc(const int8_t *m, int q, int s) { return m[q * 32 + s]; }
+
+// Four letters from p (any alignment): two aligned 32-bit loads and a funnel
+// shift.  Reads up to 7 bytes past p; the database and batch letter buffers
+// carry 64 bytes of tail padding, and walks only take blocks that start at or
+// after the sequence start.
+__device__ __forceinline__ uint32_t load4(const uint8_t *p) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+    return __funnelshift_r(__ldg(w), __ldg(w + 1), (uint32_t)(a & 3) * 8);
+}
+
+// X-drop walk to the left from (s_off, q_off) inclusive, at most
+// min(s_off, q_off) + 1 letters; returns the best score, *len = letters in
+// the best walk.  Letters are read four at a time; every letter is checked.
+__device__ int extend_left(const int8_t *m, const uint8_t *s, const uint8_t *q, int s_off,
+                           int q_off, int dropoff, int *len) {
+    const int n = min(s_off, q_off);
+    int best_i = n + 1;
+    int score = 0, maxscore = 0;
+    int k = 0;             // letters taken: the next is (s_off - k, q_off - k), index i = n - k
+    bool stop = false;
+    while (!stop && k + 3 <= n) {
+        const uint32_t sw = load4(s + s_off - k - 3);
+        const uint32_t qw = load4(q + q_off - k - 3);
+        // four letters without branches: letters after a stop change nothing
+#pragma unroll
+        for (int j = 3; j >= 0; --j) {
+            const int ns = score + sc(m, (qw >> (8 * j)) & 255u, (sw >> (8 * j)) & 255u);
+            const bool better = !stop && ns > maxscore;
+            best_i = better ? n - k - (3 - j) : best_i;
+            maxscore = better ? ns : maxscore;
+            stop = stop || maxscore - ns >= dropoff;
+            score = ns;
+        }
+        k += 4;
+    }
+    for (; !stop && k <= n; ++k) {
+        score += sc(m, q[q_off - k], s[s_off - k]);
+        if (score > maxscore) {
+            maxscore = score;
+            best_i = n - k;
+        }
+        if (maxscore - score >= dropoff)
+            stop = true;
+    }
+    *len = n - best_i + 1;
+    return maxscore;
+}
+
+// X-drop walk to the right from (s_off, q_off) that also stops when the
+// running score is <= 0; *s_last_off = the last subject offset examined
+// (s_off + n when the walk reaches a sequence end).
+__device__ int extend_right(const int8_t *m, const uint8_t *s, int s_len, const uint8_t *q,
+                            int q_len, int s_off, int q_off, int dropoff, int maxscore,
+                            int *len, int *s_last_off) {
+    const int n = min(s_len - s_off, q_len - q_off);
+    int best_i = -1;
+    int score = maxscore;
+    int i = 0;
+    bool stop = false;
+    while (!stop && i + 3 < n) {
+        const uint32_t sw = load4(s + s_off + i);
+        const uint32_t qw = load4(q + q_off + i);
+        int adv = 4;           // letters before the stopping one
+#pragma unroll
+        for (int jj = 0; jj < 4; ++jj) {
+            const int ns = score + sc(m, (qw >> (8 * jj)) & 255u, (sw >> (8 * jj)) & 255u);
+            const bool better = !stop && ns > maxscore;
+            best_i = better ? i + jj : best_i;
+            maxscore = better ? ns : maxscore;
+            const bool end = !stop && (ns <= 0 || maxscore - ns >= dropoff);
+            adv = end ? jj : adv;
+            stop = stop || end;
+            score = stop ? score : ns;
+        }
+        i += adv;
+    }
+    for (; !stop && i < n; ++i) {
+        score += sc(m, q[q_off + i], s[s_off + i]);
+        if (score > maxscore) {
+            maxscore = score;
+            best_i = i;
+        }
+        if (score <= 0 || maxscore - score >= dropoff)
+            break;
+    }
+    *len = best_i + 1;
+    *s_last_off = s_off + i;
+    return maxscore;
+}
+
+struct Ext {
+    int q_start, s_start, len, score, s_last_off;
+    bool right;
+};
+
+__device__ Ext extend_two_hit(const int8_t *m, const uint8_t *s, int s_len, const uint8_t *q,
+                              int q_len, int s_left_off, int s_right_off, int q_right_off,
+                              int dropoff) {
+    Ext e;
+    int right_d = 0, best = 0, acc = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        acc += sc(m, q[q_right_off + i], s[s_right_off + i]);
+        if (acc > best) {
+            best = acc;
+            right_d = i + 1;
+        }
+    }
+    q_right_off += right_d;
+    s_right_off += right_d;
+    int left_d = 0;
+    int left_score = extend_left(m, s, q, s_right_off - 1, q_right_off - 1, dropoff, &left_d);
+    int right_score = 0, rlen = 0;
+    e.s_last_off = s_right_off;
+    e.right = false;
+    if (left_d >= s_right_off - s_left_off) {
+        e.right = true;
+        right_score = extend_right(m, s, s_len, q, q_len, s_right_off, q_right_off, dropoff,
+                                   left_score, &rlen, &e.s_last_off);
+    }
+    e.q_start = q_right_off - left_d;
+    e.s_start = s_right_off - left_d;
+    e.len = left_d + rlen;
+    e.score = max(left_score, right_score);
+    return e;
+}
+
+__device__ __forceinline__ unsigned lanemask_lt() {
+    unsigned r;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(r));
+    return r;
+}
 // ---------------------------------------------------------------------------
 // Diagonal cells.  NCBI's DiagStruct keeps a 31-bit last hit and a 1-bit flag
 // against an offset that grows by subject length + window per subject.  The
@@ -241,7 +382,7 @@ __device__ void flush(const Item<Cell> &it, const WordFinderArgs &a, Slot &sh, W
                 const HbgContext C = a.contexts[ci];
                 const HbgQueryDesc Q = a.queries[C.query];
                 const int ql = q - Q.start;
-                const Ext e = extend_two_hit(score_matrix(), letters_of(it.s), it.S, letters_of(it.gseq), Q.start, Q.len,
+                const Ext e = extend_two_hit(score_matrix(), it.s, it.S, it.gseq + Q.start, Q.len,
                                              wq.task_left[i], s_h, ql, C.x_dropoff);
                 atomicAdd(&sh.q_ext[C.query - it.first_query], 1u);
                 if (e.score >= C.cutoff) {
@@ -612,7 +753,7 @@ __global__ void __launch_bounds__(256, (Mode & 1) == 0 ? 4 : 1) wordfinder_kerne
         a.gdiag ? a.gdiag + ((size_t)blockIdx.x * nwarps + warp) * (size_t)a.gdiag_len : nullptr;
 
     for (int i = threadIdx.x; i < 28 * 32; i += blockDim.x)
-        load_scores(hd.matrix, c_blosum, i);
+        hd.matrix[i] = c_blosum[i];
     for (int i = threadIdx.x; i < team; i += blockDim.x)
         slots[i].group = -1;
     for (int i = lane; i < a.smem_diag; i += 32)
