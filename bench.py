@@ -502,11 +502,11 @@ def main():
     alg_bytes = ssum + 8 * db.n + HSP_BYTES * n_hsps
     achieved = alg_bytes / wf_avg / 1e9
     traffic = None
-    tfile = ROOT / "profiles" / "wordfinder_traffic.json"
+    tfile = ROOT / "profiles" / "bytefinder_traffic.json"
     if tfile.exists():
         try:
             tj = json.loads(tfile.read_text())
-            if tj.get("config") == args.config:
+            if tj.get("config") == args.config and not (args.mode == 1 or args.subjects or args.group_len):
                 traffic = tj.get("dram_bytes_per_launch")
         except ValueError:
             pass
@@ -539,22 +539,23 @@ def main():
     e2e = None
     if not args.no_e2e:
         times = []
-        h2d = d2h = 0
+        d2h = 0
         for i in range(1 + max(1, args.steps // 3)):
             torch.cuda.synchronize()
             t0 = time.perf_counter()
             b2 = batch_of(pqs)
             r2 = hblast.search(gdb, b2, opts, hsp_capacity=max(int(n_hsps * 1.1) + 1024, 1 << 20), stream=sptr)
-            h2d = b2.info()["device_bytes"]
             b2.close()
             torch.cuda.synchronize()
             if i > 0:
                 times.append(time.perf_counter() - t0)
             d2h = HSP_BYTES * len(r2.hsps) + 8 * (1 + 4 * len(pqs))
+        # copied: a letter and a context index per query letter (the lookup tables are built on the device)
+        h2d = 5 * binfo["total_query_len"]
         te = sum(times) / len(times)
         e2e = {"value": units_per_step * world / te, "unit": UNIT, "h2d_bytes_per_step": int(h2d),
                "d2h_bytes_per_step": int(d2h), "ms_per_step": te * 1e3,
-               "path": "hbg_batch_create (host lookup tables) + hbg_search + hbg_result_wait"}
+               "path": "hbg_batch_create + hbg_search (lookup tables on the device) + hbg_result_wait"}
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline:
@@ -581,7 +582,7 @@ def main():
             "clocks": ck,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
-                         "kernel": "wordfinder_kernel", "kernel_ms": wf_avg * 1e3,
+                         "kernel": "wordfinder_kernel" if args.mode == 1 else "byte_kernel", "kernel_ms": wf_avg * 1e3,
                          "algorithmic_bytes": int(alg_bytes)},
             "lookup_hits_per_s": hits / wf_avg, "extensions_per_s": ext / wf_avg,
             "hsps": n_hsps, "ordering_ms": sum(ord_ms) / len(ord_ms),

@@ -21,16 +21,12 @@ namespace hbg {
 // beat them by 13-23 % (4096 to 32768 entries, BLASTP and six-frame BLASTX).
 constexpr int32_t kSmemDiagMax = 2048;
 // Default group length (letters, gaps included): 4056, the longest whose
-// table is 4096 entries of 16-bit cells in global memory (8 KB a warp, 40 MB
-// for all resident warps, which stay in L2).  On the 64-query batched workload
-// (GB300, word-finder ms for 2,000,000 subjects): 4056 letters 936 (16 scans
-// of the database); 6000 906, 7000 905, 8152 909 (8192-entry tables: 80 MB,
-// which L2 no longer holds -- DRAM writes of evicted table lines rise from
-// 6.4 GB to 92 GB per 500,000 subjects, ~15x, for 3 % less time); 10000 942,
-// 12000 975, 16344 1159; 2008-letter groups with shared tables are slower
-// still (37 scans).  Since each subject's hits are carried across chunks,
-// 6000-letter groups are within 0.4 % of 4056 (858 vs 862 ms), so the extra
-// traffic buys nothing.
+// table has 4096 entries, which byte_kernel keeps in 16-bit cells with 22 warps
+// per SM.  64 queries of 50..1500 letters against 500,000 subjects, word-finder
+// ms by group length (and scans of the database): 1000 187 (52), 2008 167 (37),
+// 4056 143 (16), 6000 146 (10), 8152 144 (7), 16,000 189 (4).  wordfinder_kernel
+// has the same best range: 2,000,000 subjects, tables in global memory, 4056
+// 862, 6000 858, with 15 times the DRAM writes above 4096 entries.
 constexpr int32_t kDefaultGroupLen = 4056;
 // Groups whose expected hits per subject offset reach this use offset mode
 // (off by default: chunk mode at high occupancy measured faster; the autotuner

@@ -196,8 +196,9 @@ int hbg_db_open_blastdb(const char *path, const hbg_gpu_options *opt, hbg_db **o
 
 /* ---- query batches -------------------------------------------------------- */
 
-/* Build the neighbourhood lookup tables of a batch of protein queries on the
- * host (the work NCBI's BlastAaLookupTableNew/BlastAaLookupIndexQuery do
+/* Pack a batch of protein queries; its neighbourhood lookup tables are built on
+ * the device by the first search, and on the host when a caller asks to see
+ * them (the work NCBI's BlastAaLookupTableNew/BlastAaLookupIndexQuery do
  * before H-BLAST reads the table at h_blast.cu:940-958, with cells sorted as
  * lut_sorting does at h_blast.cu:165-194).  Queries are packed into groups
  * that share one scan of the database; results are identical to searching
@@ -298,7 +299,8 @@ int hbg_batch_tune(hbg_batch *batch, int32_t tile_subjects, int32_t global_table
 int hbg_batch_schedule(hbg_batch *batch, int32_t warps_per_subject, int64_t tile_bytes);
 
 int hbg_batch_destroy(hbg_batch *batch);
-/* Sizes of a batch; device_bytes is what its upload copies host-to-device. */
+/* Sizes of a batch; device_bytes is what its letters and
+ * lookup tables take on the device. */
 int hbg_batch_info(const hbg_batch *batch, int32_t *n_queries, int32_t *n_groups,
                    int64_t *total_query_len, int64_t *lookup_entries, int64_t *device_bytes);
 
@@ -313,7 +315,8 @@ int hbg_mem_required(const hbg_db *db, const hbg_batch *batch, int64_t hsp_capac
 /* Launch the word-hit stage of batch against db on stream (a cudaStream_t,
  * NULL = the legacy default stream) and return at once.  Replaces H_BLAST_pre
  * + H_BLAST (h_blast.cu:873-1157).  hsp_capacity bounds the HSP buffer (0 =
- * one slot per subject, at least 1 Mi; H-BLAST sizes it as AVG_HSPS_PER_SEQUENCE
+ * 2e-7 slots per letter of the queries and of the database, at least one per
+ * subject and 1 Mi; H-BLAST sizes it as AVG_HSPS_PER_SEQUENCE
  * slots per subject, NF/functions.cpp:1513-1516);
  * if a search finds more, hbg_result_wait relaunches it once with a buffer of
  * the exact size, so results never depend on the capacity.  *out == NULL
