@@ -19,6 +19,11 @@ namespace {
 constexpr int kScoreScale = 16;
 typedef int16_t Score;
 
+// X-drops are taken up to this.  No walk falls further: it has at most 65,000
+// letter pairs of -128 (a sentinel) to 11, so at most 9.1 million lie between its
+// best score and any other.  The scaled value and sums with it fit 32 bits.
+constexpr int kMaxDrop = 1 << 24;
+
 __device__ __forceinline__ void load_scores(Score *m, const int8_t *blosum, int i) {
     m[i] = (Score)(kScoreScale * blosum[i] - 1);
 }
@@ -139,7 +144,7 @@ struct Ext {
 __device__ __forceinline__ Ext extend_two_hit(const Score *m, const Letters &S, int s_len, const Letters &G, int q_start,
                                               int q_len, int s_left, int s_h, int q_h, int dropoff) {
     const unsigned s0 = S.first + (unsigned)s_h - 5u, q0 = G.first + (unsigned)(q_start + q_h) - 5u;
-    const int drop = kScoreScale * dropoff;
+    const int drop = kScoreScale * min(dropoff, kMaxDrop);
     Walk w{0, 0, 0, false};
     int x[8], y[8], adv;
     const int n_left = min(s_h, q_h) + 3;    // letters up to the end of the word

@@ -144,3 +144,18 @@ def test_device_built_tables(built, threshold, qlens):
             assert np.array_equal(h[f], ref[f]), f
         st = got.stats[k]
         assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
+
+
+@pytest.mark.parametrize("xdrop", [1 << 24, (1 << 24) + 1, (1 << 27) - 1, 1 << 27, 1 << 28, (1 << 28) + 1, 2**31 - 1])
+@pytest.mark.parametrize("qlen", [300, 5000])
+def test_xdrop_without_limit(built, xdrop, qlen):
+    """X-drops so large that no walk ends by them, the plain way to ask for
+    none, with either size of cells."""
+    rng = np.random.default_rng(qlen)
+    parts = [synth.random_letters(rng, n) for n in (40, qlen, 5)]
+    pq = contexts_query(parts, [xdrop, 16, xdrop], [11, 25, 11])
+    res, off = database(rng, parts[0])
+    check(hblast.search(hblast.Database(res, off), hblast.Batch.proteins([pq])), [pq], res, off)
+    pq = contexts_query(parts, [xdrop] * 3, [30] * 3)
+    res, off = database(rng, parts[1])
+    check(hblast.search(hblast.Database(res, off), hblast.Batch.proteins([pq])), [pq], res, off)
