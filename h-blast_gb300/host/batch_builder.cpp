@@ -153,6 +153,8 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
         return "empty batch";
     if (max_group_len <= 0)
         max_group_len = kDefaultGroupLen;
+    // offsets in a group are kept in 16 bits: lookup entries, queued extensions
+    max_group_len = std::min<int32_t>(max_group_len, HBG_MAX_QUERY_LEN);
     if (mode_hits < 0)
         mode_hits = kOffsetModeHits;
     HostBatch &b = *out;

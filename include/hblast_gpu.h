@@ -203,7 +203,8 @@ int hbg_db_open_blastdb(const char *path, const hbg_gpu_options *opt, hbg_db **o
  * lut_sorting does at h_blast.cu:165-194).  Queries are packed into groups
  * that share one scan of the database; results are identical to searching
  * each query alone.  max_group_len 0 = library default; 1 packs one query
- * per group (the plain one-query-per-launch form). */
+ * per group (the plain one-query-per-launch form); values above
+ * HBG_MAX_QUERY_LEN count as that. */
 int hbg_batch_create(const hbg_query *queries, int32_t n_queries,
                      const hbg_word_params *params, int32_t max_group_len,
                      hbg_batch **out);

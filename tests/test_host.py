@@ -103,6 +103,31 @@ def test_group_packing_and_offsets(built):
     assert seen == 6
 
 
+@pytest.mark.parametrize("max_group_len,n,qlen", [(100000, 12, 6000), (65535, 12, 5400), (65536, 2, 40000), (2**31 - 1, 2, 65000)])
+def test_groups_stay_within_16_bit_offsets(built, max_group_len, n, qlen):
+    """A caller's group length beyond what 16-bit entries can address: more
+    groups, with every query's words at its own offsets, ascending in each cell."""
+    rng = np.random.default_rng(n)
+    qs = [synth.random_letters(rng, qlen) for _ in range(n)]
+    b = hblast.Batch.proteins([hblast.ProteinQuery.blastp(x) for x in qs], threshold=19, max_group_len=max_group_len)
+    assert b.info()["n_groups"] >= 2
+    seen = 0
+    for g in range(b.info()["n_groups"]):
+        cells, ents, first, starts = b.lookup_table(g)
+        assert first == seen and starts[-1] + qlen <= 65000
+        seen += len(starts)
+        inner = np.ones(len(ents), bool)
+        inner[cells[:-1][cells[:-1] < len(ents)]] = False            # first entries of cells
+        assert np.all(np.diff(ents.astype(np.int64), prepend=0)[inner] > 0)
+        for k, at in enumerate(starts):
+            mine = (ents >= at) & (ents < at + qlen)
+            cs, es = oracle.lookup_table(oracle.Query.blastp(qs[first + k], 16, 41), 19)
+            word = np.repeat(np.arange(32768), np.diff(cells.astype(np.int64)))
+            assert np.array_equal(ents[mine] - at, es)
+            assert np.array_equal(np.bincount(word[mine], minlength=32768), np.diff(cs.astype(np.int64)))
+    assert seen == n
+
+
 def test_plain_form_one_query_per_group(built):
     rng = np.random.default_rng(2)
     qs = [synth.random_letters(rng, 60) for _ in range(5)]
