@@ -1349,6 +1349,12 @@ int hbg_db_open_blastdb(const char *path, const hbg_gpu_options *opt, hbg_db **o
             if (e == cudaSuccess)
                 e = cudaEventCreateWithFlags(&done[j], cudaEventDisableTiming);
         }
+        // db_create zeroed the letters on the legacy stream, where a search may
+        // still run ahead of it: the copies come after
+        if (e == cudaSuccess)
+            e = cudaEventRecord(done[0], cudaStreamLegacy);
+        if (e == cudaSuccess)
+            e = cudaStreamWaitEvent(st, done[0], 0);
         if (e != cudaSuccess)
             err = cuda_msg("staging buffers", e, code);
         int cur = 0;

@@ -42,6 +42,29 @@ def test_larger_than_staging_pieces(built, tmp_path):
     compare(tmp_path / "big", qs, db)
 
 
+def test_opened_behind_a_running_search(built, tmp_path):
+    """The letters are zeroed on the default stream and copied on another: with a
+    search of 50 ms and more ahead on the default stream, the copies still come last."""
+    qs, big = synth.batched_blastp(seed=6, n_queries=64, n_subjects=200_000)
+    gdb = hblast.Database(big.residues, big.offsets)
+    busy = hblast.Searcher(gdb, hblast.Batch.proteins([hblast.ProteinQuery.blastp(q) for q in qs]))
+    busy.launch()
+    busy.sync()
+    n = 5000
+    blastdb.write_volume(tmp_path / "one", big.residues[:big.offsets[n]], big.offsets[:n + 1])
+    small = hblast.Database(big.residues[:big.offsets[n]], big.offsets[:n + 1])
+    batch = hblast.Batch.proteins([hblast.ProteinQuery.blastp(q) for q in qs[:3]])
+    ref = hblast.search(small, batch)
+    assert len(ref.hsps) > 0
+    for _ in range(3):
+        busy.launch()
+        opened = hblast.Database.from_blastdb(tmp_path / "one")
+        got = hblast.search(opened, batch)
+        busy.sync()
+        assert np.array_equal(got.hsps, ref.hsps) and got.stats == ref.stats
+        opened.close()
+
+
 def test_bad_database_is_an_error(built, tmp_path):
     with pytest.raises(hblast.HblastError, match="neither"):
         hblast.Database.from_blastdb(tmp_path / "absent")
