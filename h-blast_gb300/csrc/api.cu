@@ -192,7 +192,7 @@ struct LaunchShape {
     int byte_blocks;
     int n_long;      // subjects left to wordfinder_kernel: the longest n_long
 };
-constexpr int kMaxLaunchClasses = 32;
+constexpr int kMaxLaunchClasses = 64;
 
 // What a search keeps on the host side beside its device buffers: events and
 // the pinned copy of its counters.  Making and freeing them took 250 us of a
@@ -421,11 +421,14 @@ constexpr int kByteTable16 = 4096;
 constexpr int kByteMinWarps = 2;
 
 // Bytes of a diagonal cell in byte_kernel for a group, 0 when it cannot take
-// the group: its window, table, cell counts or entry count do not fit, or the
-// caller's own table lists an offset twice in a cell (two hits in one place).
+// the group: its window, table, cell counts or entry count do not fit, the
+// caller's own table lists an offset twice in a cell (two hits in one place), or
+// the caller chose offset mode or a launch shape of wordfinder_kernel.
 int byte_cell(const hbg_batch *b, int32_t g) {
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
+    if ((G.mode & 1) || b->tuned || b->team > 1 || b->tile_bytes > 0)
+        return 0;
     if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.max_count > hbg::kByteMaxCount ||
         G.n_entries >= hbg::kByteMaxEntries || b->repeated_entries)
         return 0;
@@ -439,14 +442,19 @@ int make_classes(hbg_batch *b, std::vector<int32_t> *list) {
     // launched by table size, so a short query's warps reserve only the
     // shared memory its table needs (the rest is L1 for cells and entries:
     // one 350-aa query vs 10 M subjects 8 % faster than with 2048-entry
-    // tables for every group); global-table groups form their own class
+    // tables for every group).  Global-table groups of one length form a class
+    // of their own, all of them one class when the caller chose the tiles: a
+    // class alone then has too few.  Five groups of 2500 to 40,000 letters
+    // against 20,000 subjects, ms, together and apart: tiles of 64 subjects 61 /
+    // 105, of 64 KiB 120 / 233; automatic tiles in offset mode 48 / 27, four
+    // groups to a pass 145 / 75.
+    const bool tiles = b->tile_subjects > 0 || b->tile_bytes > 0;
     std::vector<std::pair<std::array<int, 3>, int32_t>> keyed;
     for (int32_t g = 0; g < (int32_t)h.groups.size(); ++g) {
         const HbgGroup &G = h.groups[g];
         const int size = G.placement ? 64 : std::max<int>(64, G.diag_len);
-        // byte_kernel's table, with the cell size in the low bits
-        const int cell = byte_cell(b, g);
-        keyed.push_back({{G.mode, size, cell ? 4 * std::max<int>(64, G.diag_len) + cell : 0}, g});
+        // byte_kernel's table with the cell size in the low bits, longest first
+        keyed.push_back({{G.mode, size, tiles ? 0 : -(4 * std::max<int>(64, G.diag_len) + byte_cell(b, g))}, g});
     }
     std::stable_sort(keyed.begin(), keyed.end(),
                      [](const auto &x, const auto &y) { return x.first < y.first; });
@@ -456,7 +464,7 @@ int make_classes(hbg_batch *b, std::vector<int32_t> *list) {
         const bool global = h.groups[keyed[i].second].placement != 0;
         if (i == 0 || keyed[i].first != keyed[i - 1].first)
             b->classes.push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
-                                             keyed[i].first[2] & 3, keyed[i].first[2] / 4});
+                                             -keyed[i].first[2] & 3, -keyed[i].first[2] / 4});
         LaunchClass &lc = b->classes.back();
         lc.count++;
         if (lc.cell == 1)              // the longest group's exact table
@@ -630,8 +638,7 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
     shapes->assign(b->classes.size(), LaunchShape{32, 1, 1, 0, 0, 0});
     hbg_gpu_options std_opt;
     hbg_default_gpu_options(&std_opt);
-    if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx || b->tuned || b->team > 1 ||
-        b->tile_bytes > 0)
+    if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx)
         return;                                  // the caller chose a launch shape of wordfinder_kernel
     int optin = 0, sms = 1;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
@@ -639,7 +646,7 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
     for (size_t c = 0; c < b->classes.size(); ++c) {
         const LaunchClass &lc = b->classes[c];
         LaunchShape &sh = (*shapes)[c];
-        if (!lc.cell || (lc.mode & 1))
+        if (!lc.cell)
             continue;
         // one CTA per SM, with as many warps as their tables leave room for
         int t = hbg::kByteThreads;
@@ -834,6 +841,62 @@ hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass 
     return t;
 }
 
+// The word finder's launches: byte_kernel for each class it takes, then
+// wordfinder_kernel for the rest.  With smaller CTAs than the default the classes
+// that wordfinder_kernel does not tell apart share one launch, longest groups
+// first: few warps work on a class's last tiles.  Threads 128, ms, together and
+// apart: five groups of 2500 to 40,000 letters against 20,000 subjects 36.9 / 44.2,
+// seven of 300 to 20,000 14.3 / 19.9, six of 3000 and three of 6000 9.4 / 10.3.
+// `a` holds scratch and outputs (tile_counter: one counter per class), `next` a
+// subject counter per group, both zeroed.  The caller has run
+// wordfinder_configure and byte_configure (not stream operations).
+int launch_finders(const hbg_db *db, const hbg_batch *b, const std::vector<LaunchShape> &shapes,
+                   const hbg_gpu_options &opt, hbg::WordFinderArgs a, unsigned long long *next, uint16_t *side,
+                   cudaStream_t st, int *launches) {
+    hbg_gpu_options std_opt;
+    hbg_default_gpu_options(&std_opt);
+    const bool together = opt.num_threadsx < std_opt.num_threadsx;
+    unsigned int *const tiles = a.tile_counter;
+    const size_t n = db->n > 0 ? b->classes.size() : 0;
+    for (size_t c = 0; c < n; ++c) {
+        const LaunchClass &lc = b->classes[c];
+        const LaunchShape &sh = shapes[c];
+        if (sh.byte_threads == 0 || sh.n_long >= db->n)
+            continue;
+        hbg::ByteArgs t = byte_args(db, b, lc, sh);
+        t.next = next;
+        t.side = side;
+        t.hsps = a.hsps;
+        t.hsp_count = a.hsp_count;
+        t.hsp_cap = a.hsp_cap;
+        t.q_extended = a.q_extended;
+        t.q_kept = a.q_kept;
+        CU(hbg::launch_byte(t, lc.cell, sh.byte_blocks, sh.byte_threads, st));
+        ++*launches;
+    }
+    auto subjects = [&](size_t c) { return shapes[c].byte_threads > 0 ? shapes[c].n_long : db->n; };
+    for (size_t c = 0, e; c < n; c = e) {
+        LaunchClass lc = b->classes[c];
+        for (e = c + 1; together && e < n && b->classes[e].mode == lc.mode && b->classes[e].smem_diag == lc.smem_diag &&
+                        subjects(e) == subjects(c); ++e)
+            lc.count += b->classes[e].count;
+        a.n_subj = subjects(c);
+        if (a.n_subj == 0)
+            continue;
+        a.tile_subjects = class_tile_subjects(b, a.n_subj, db, lc, shapes[c].blocks);
+        a.tiles_per_group = (a.n_subj + a.tile_subjects - 1) / a.tile_subjects;
+        a.team = shapes[c].team;
+        a.n_list = lc.count;
+        a.group_list = b->d_group_list + lc.first;
+        a.n_tiles = (int64_t)a.tiles_per_group * ((lc.count + a.team - 1) / a.team);
+        a.tile_counter = tiles + c;
+        a.smem_diag = lc.smem_diag;
+        CU(hbg::launch_wordfinder(a, lc.mode, shapes[c].blocks, shapes[c].threads, st));
+        ++*launches;
+    }
+    return HBG_OK;
+}
+
 // Enqueue one search on r->stream: counter resets, the word finder, the
 // ordering pass, the lookup-hit counters and the copy of the counters to
 // pinned host memory.  No host synchronisation, so it can be captured.
@@ -889,38 +952,9 @@ int enqueue_search(hbg_result *r) {
         cap_status == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     CU(cudaEventRecordWithFlags(r->kit.ev[0], st, ev_flags));
     int wf_launches = 0;
-    if (db->n > 0)   // the caller has run wordfinder_configure (not a stream operation)
-        for (size_t c = 0; c < b->classes.size(); ++c) {
-            const LaunchClass &lc = b->classes[c];
-            const LaunchShape &sh = r->shapes[c];
-            if (sh.byte_threads > 0) {
-                hbg::ByteArgs t = byte_args(db, b, lc, sh);
-                t.next = r->d_counters + 1 + 6 * nq + ng;
-                t.side = r->d_side;
-                t.hsps = a.hsps;
-                t.hsp_count = a.hsp_count;
-                t.hsp_cap = a.hsp_cap;
-                t.q_extended = a.q_extended;
-                t.q_kept = a.q_kept;
-                if (t.n_subj > 0) {
-                    CU(hbg::launch_byte(t, lc.cell, sh.byte_blocks, sh.byte_threads, st));
-                    ++wf_launches;
-                }
-                if (sh.n_long == 0)
-                    continue;
-            }
-            ++wf_launches;
-            a.n_subj = sh.byte_threads > 0 ? sh.n_long : db->n;
-            a.tile_subjects = class_tile_subjects(b, a.n_subj, db, lc, r->shapes[c].blocks);
-            a.tiles_per_group = (a.n_subj + a.tile_subjects - 1) / a.tile_subjects;
-            a.team = r->shapes[c].team;
-            a.n_list = lc.count;
-            a.group_list = b->d_group_list + lc.first;
-            a.n_tiles = (int64_t)a.tiles_per_group * ((lc.count + a.team - 1) / a.team);
-            a.tile_counter = r->d_tile + c;
-            a.smem_diag = lc.smem_diag;
-            CU(hbg::launch_wordfinder(a, lc.mode, r->shapes[c].blocks, r->shapes[c].threads, st));
-        }
+    const int rc = launch_finders(db, b, r->shapes, r->shape_opt, a, r->d_counters + 1 + 6 * nq + ng, r->d_side, st, &wf_launches);
+    if (rc != HBG_OK)
+        return rc;
     CU(cudaEventRecordWithFlags(r->kit.ev[1], st, ev_flags));
 
     hbg::OrderArgs o;
@@ -2101,36 +2135,12 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     a.gdiag = nullptr;
     a.gdiag_len = 0;
     a.smem_diag = h.smem_diag_len;
-    if (db->n > 0) {
-        for (size_t c = 0; c < batch->classes.size(); ++c) {
-            const LaunchClass &lc = batch->classes[c];
-            if (shapes[c].byte_threads > 0) {
-                // 16-bit cells (longer groups are refused above), so no side
-                // table; the group counters serve as subject counters
-                hbg::ByteArgs t = byte_args(db, batch, lc, shapes[c]);
-                t.next = g_hits;
-                t.hsps = a.hsps;
-                t.hsp_count = a.hsp_count;
-                t.hsp_cap = a.hsp_cap;
-                t.q_extended = a.q_extended;
-                t.q_kept = a.q_kept;
-                if (t.n_subj > 0)
-                    CU(hbg::launch_byte(t, lc.cell, shapes[c].byte_blocks, shapes[c].byte_threads, st));
-                if (shapes[c].n_long == 0)
-                    continue;
-            }
-            a.n_subj = shapes[c].byte_threads > 0 ? shapes[c].n_long : db->n;
-            a.tile_subjects = class_tile_subjects(batch, a.n_subj, db, lc, shapes[c].blocks);
-            a.tiles_per_group = (a.n_subj + a.tile_subjects - 1) / a.tile_subjects;
-            a.team = shapes[c].team;
-            a.n_list = lc.count;
-            a.group_list = batch->d_group_list + lc.first;
-            a.n_tiles = (int64_t)a.tiles_per_group * ((lc.count + a.team - 1) / a.team);
-            a.tile_counter = tile + c;
-            a.smem_diag = lc.smem_diag;
-            CU(hbg::launch_wordfinder(a, lc.mode, shapes[c].blocks, shapes[c].threads, st));
-        }
-    }
+    // 16-bit cells (longer groups are refused above), so no side table; the
+    // group counters serve as subject counters
+    int launches = 0;
+    rc = launch_finders(db, batch, shapes, o, a, g_hits, nullptr, st, &launches);
+    if (rc != HBG_OK)
+        return rc;
     // per-query extension and kept counts follow the HSP count in d_counts
     CU(cudaMemcpyAsync(d_counts + 1, q_ext, sizeof(unsigned long long) * (size_t)(2 * nq),
                        cudaMemcpyDeviceToDevice, st));

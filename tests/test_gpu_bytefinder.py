@@ -159,3 +159,36 @@ def test_xdrop_without_limit(built, xdrop, qlen):
     pq = contexts_query(parts, [xdrop] * 3, [30] * 3)
     res, off = database(rng, parts[1])
     check(hblast.search(hblast.Database(res, off), hblast.Batch.proteins([pq])), [pq], res, off)
+
+
+@pytest.mark.parametrize("form,launches", [("tiles", 1), ("tile bytes", 1), ("threads", 1), ("offset", 4), ("team", 4),
+                                           ("window", 4)])
+def test_general_kernel_takes_long_groups_together(built, form, launches):
+    """Groups of every table length, left to the general kernel by the caller's
+    choice or by the window: with chosen tiles or small CTAs those with global
+    tables share one launch."""
+    rng = np.random.default_rng(31)
+    qs = [synth.random_letters(rng, n) for n in (2500, 5000, 9000, 17000)]
+    res, off = database(rng, qs[0])
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 20) for q in qs]
+    gdb = hblast.Database(res, off)
+    window = 70 if form == "window" else 40
+    b = hblast.Batch.proteins(pqs, window=window, max_group_len=1)
+    if form == "tiles":
+        b.tune(64)
+    if form == "tile bytes":
+        b.schedule(1, 65536)
+    if form == "team":
+        b.schedule(3)
+    if form == "offset":
+        b.set_mode(1)
+    s = hblast.Searcher(gdb, b, hblast.default_options(num_threadsx=128) if form == "threads" else None)
+    s.launch()
+    s.wait()
+    assert s.timing()[2] == launches + 1         # and the ordering
+    got = s.result()
+    if window == 40:
+        check(got, pqs, res, off)
+    else:
+        other = hblast.search(gdb, hblast.Batch.proteins(pqs, window=window, max_group_len=1).tune(64))
+        assert len(got.hsps) > 0 and np.array_equal(got.hsps, other.hsps) and got.stats == other.stats
