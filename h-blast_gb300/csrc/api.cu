@@ -654,6 +654,14 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
             t -= 32;
         if (t < 32 * kByteMinWarps)
             continue;
+        // a group's subjects go to the warps of one CTA: with fewer subjects than
+        // warps, groups in great number are better off with wordfinder_kernel,
+        // whose CTAs take several at a time.  Here / there, ms: 1000 groups of 300
+        // letters against 12 subjects 0.227 / 0.169, 25 subjects 0.223 / 0.236;
+        // 1500 of 4000 letters 1.64 / 1.32, 1.62 / 1.87; 300 groups of 1500 letters
+        // against 12 subjects 0.143 / 0.162.
+        if (db->n < t / 32 && lc.count > 4 * sms)
+            continue;
         const int32_t cut = lc.cell == 2 ? 0x7ffe - b->host.window : 0xffff;
         const auto &L = db->sched_len;
         sh.n_long = (int)(std::partition_point(L.begin(), L.end(), [&](int32_t l) { return l > cut; }) - L.begin());
@@ -834,10 +842,12 @@ hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass 
     t.window = b->host.window;
     t.table_len = lc.table_len;
     // the first subjects are the longest: a take of them is at most an eighth
-    // of a warp's share of the letters
-    const int64_t warps = (int64_t)sh.byte_blocks * (sh.byte_threads / 32);
+    // of a warp's share of a group's letters (with more groups than CTAs each
+    // has a CTA to itself; taken as the share of all letters, 5000 one-query
+    // groups against 400 subjects had takes of 12 and took 14.6 ms, now 8.2)
+    const int64_t warps = (int64_t)sh.byte_blocks * (sh.byte_threads / 32), groups = std::min(lc.count, sh.byte_blocks);
     t.chunk = (int32_t)std::max<int64_t>(
-        1, std::min<int64_t>(16, db->n_res * lc.count / (8 * warps * std::max<int32_t>(1, db->max_len))));
+        1, std::min<int64_t>(16, db->n_res * groups / (8 * warps * std::max<int32_t>(1, db->max_len))));
     return t;
 }
 

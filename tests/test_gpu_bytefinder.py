@@ -192,3 +192,28 @@ def test_general_kernel_takes_long_groups_together(built, form, launches):
     else:
         other = hblast.search(gdb, hblast.Batch.proteins(pqs, window=window, max_group_len=1).tune(64))
         assert len(got.hsps) > 0 and np.array_equal(got.hsps, other.hsps) and got.stats == other.stats
+
+
+@pytest.mark.parametrize("n_groups,n_subjects", [(151, 30), (153, 30), (770, 30), (1700, 30), (608, 20), (609, 20), (1700, 2)])
+def test_many_groups_few_subjects(built, n_groups, n_subjects):
+    """More groups than CTAs and than a CTA has threads, against databases of
+    about as many subjects as a CTA has warps: every query as the general kernel
+    has it, and a few as the oracle."""
+    rng = np.random.default_rng(n_groups)
+    qs = [synth.random_letters(rng, int(n)) for n in rng.integers(20, 70, n_groups)]
+    subs = [np.concatenate([synth.mutate(rng, qs[int(i)], 0.8) for i in rng.integers(0, n_groups, 12)]) for _ in range(n_subjects)]
+    off = np.zeros(n_subjects + 1, np.int64)
+    off[1:] = np.cumsum([len(s) for s in subs])
+    res = np.concatenate(subs)
+    gdb = hblast.Database(res, off)
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 25) for q in qs]
+    got = hblast.search(gdb, hblast.Batch.proteins(pqs, max_group_len=1))
+    ref = hblast.search(gdb, hblast.Batch.proteins(pqs, max_group_len=1).tune(8))
+    assert len(got.hsps) > n_subjects and np.array_equal(got.hsps, ref.hsps) and got.stats == ref.stats
+    for k in (0, 1, n_groups // 2, n_groups - 1):
+        hsps, subj, cnt = oracle.search(oracle.Query.blastp(qs[k], 16, 25), res, off)
+        mine = got.for_query(k)
+        assert len(mine) == len(hsps) and np.array_equal(mine["subject"], subj)
+        assert np.array_equal(mine["score"], hsps["score"]) and np.array_equal(mine["s_start"], hsps["s_start"])
+        st = got.stats[k]
+        assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
