@@ -917,8 +917,6 @@ int enqueue_search(hbg_result *r) {
     cudaStream_t st = r->stream;
     CU(cudaMemsetAsync(r->d_counters, 0, r->n_counters * sizeof(unsigned long long), st));
     CU(cudaMemsetAsync(r->d_tile, 0, kMaxLaunchClasses * sizeof(unsigned int), st));
-    if (r->d_gdiag && uses_wordfinder(r))
-        CU(cudaMemsetAsync(r->d_gdiag, 0, (size_t)r->gdiag_entries * sizeof(uint32_t), st));
 
     hbg::WordFinderArgs a;
     memset(&a, 0, sizeof(a));

@@ -46,7 +46,7 @@ struct WordFinderArgs {
     unsigned long long *q_kept;     // per batch query, zeroed
     unsigned long long *g_hits;     // per group lookup hits, zeroed
     // global-memory diagonal tables (groups with placement 1): one slice of
-    // gdiag_len entries per (block, warp), zeroed before launch
+    // gdiag_len entries per (block, warp); warps clear theirs
     uint32_t *gdiag;
     int32_t gdiag_len;
     // entries per warp of the 16-bit shared-memory tables (a multiple of 8)

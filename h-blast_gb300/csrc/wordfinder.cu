@@ -759,11 +759,12 @@ __global__ void __launch_bounds__(256, (Mode & 1) == 0 ? 4 : 1) wordfinder_kerne
     for (int i = lane; i < a.smem_diag; i += 32)
         diag_s[i] = 0;
     const int window = a.window;
-    // the 16-bit shared table starts past its limit so the first item clears it
     // offsets of the three tables a warp may use: its shared 16-bit table,
     // and its global slice seen as 16-bit or as 32-bit cells (switching views
-    // forces the other view to clear before its next use)
-    int32_t dofs_s = CellTraits<uint16_t>::kLimit + 1, dofs_g = window;
+    // forces the other view to clear before its next use); each starts past its
+    // limit, so that its first item clears it -- an earlier launch of the same
+    // search has used the slice
+    int32_t dofs_s = CellTraits<uint16_t>::kLimit + 1, dofs_g = kWrap32;
     int32_t dofs_h = CellTraits<uint16_t>::kLimit + 1;
 
     for (;;) {

@@ -323,3 +323,44 @@ def test_word_parameters(small_db, threshold, window):
             assert np.array_equal(got[g], ref[f]), (k, f)
         st = res.stats[k]
         assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt), k
+
+
+@pytest.mark.parametrize("form", ["default", "tiles", "offset", "mixed", "window", "one warp"])
+@pytest.mark.parametrize("qlens", [(20, 300, 1900), (300, 2500, 5000, 20)])
+def test_long_subjects_in_several_launches(built, form, qlens):
+    """Subjects whose positions need 32-bit cells, searched by several launches
+    one after another (groups of different table lengths, or hit modes) in
+    the same scratch: none sees what an earlier one left in it."""
+    rng = np.random.default_rng(41)
+    qs = [synth.random_letters(rng, n) for n in qlens]
+    subs = []
+    for n in (70000, 66000, 40000, 33000, 500, 100):
+        s = synth.random_letters(rng, n)
+        for at in range(0, n - 100, 300):
+            q = qs[at // 300 % len(qs)]
+            m = min(len(q), 100)
+            s[at:at + m] = synth.mutate(rng, q[:m], 0.7)
+        subs.append(s)
+    off = np.zeros(len(subs) + 1, np.int64)
+    off[1:] = np.cumsum([len(s) for s in subs])
+    res = np.concatenate(subs)
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 30) for q in qs]
+    window = 70 if form == "window" else 40
+    b = hblast.Batch.proteins(pqs, window=window, max_group_len=1)
+    if form == "tiles":
+        b.tune(8)
+    elif form == "offset":
+        b.set_mode(1)
+    elif form == "mixed":
+        b.set_mode(1, 1)
+    # one warp: every launch has the same scratch
+    opts = hblast.default_options(num_blocksx=1, num_threadsx=32) if form == "one warp" else None
+    got = hblast.search(hblast.Database(res, off), b, opts)
+    for k, q in enumerate(qs):
+        ref, subj, cnt = oracle.search(oracle.Query.blastp(q, 16, 30), res, off, window=window, nthreads=8)
+        mine = got.for_query(k)
+        assert len(mine) == len(ref) > 0 and np.array_equal(mine["subject"], subj)
+        for f in ("q_start", "s_start", "q_off", "s_off", "len", "score"):
+            assert np.array_equal(mine[f], ref[f]), (k, f)
+        st = got.stats[k]
+        assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
