@@ -199,6 +199,8 @@ constexpr int kMaxLaunchClasses = 64;
 // small search, so a database keeps a few for its next searches.
 struct HostKit {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+    cudaStream_t side = nullptr;  // for work beside the caller's stream, with the
+    cudaEvent_t fork = nullptr, join = nullptr;   // events around it: made when first needed
     unsigned long long *counters = nullptr;
     size_t n = 0;                 // counters it has room for
 };
@@ -247,6 +249,14 @@ class KitPool {
         }
         return e;
     }
+    // The kit's side stream and its events.
+    static cudaError_t add_side(HostKit *k) {
+        cudaError_t e = k->side ? cudaSuccess : cudaStreamCreateWithFlags(&k->side, cudaStreamNonBlocking);
+        for (cudaEvent_t *ev : {&k->fork, &k->join})
+            if (e == cudaSuccess && !*ev)
+                e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        return e;
+    }
     // Give back a kit that no GPU work still uses.
     void give(HostKit &k) {
         {
@@ -266,6 +276,11 @@ class KitPool {
         for (cudaEvent_t &ev : k.ev)
             if (ev)
                 cudaEventDestroy(ev);
+        for (cudaEvent_t ev : {k.fork, k.join})
+            if (ev)
+                cudaEventDestroy(ev);
+        if (k.side)
+            cudaStreamDestroy(k.side);
         if (k.counters)
             cudaFreeHost(k.counters);
         k = HostKit();
@@ -673,8 +688,9 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
 // CTA size and grid of each launch class that wordfinder_kernel has a part of: the CTA is halved until its
 // per-warp tables fit the shared-memory carve-out; the grid is one wave at
 // the occupancy that leaves (or the caller's num_blocksx).
-int plan_launches(const hbg_batch *b, const hbg_gpu_options &o, int device, std::vector<LaunchShape> *out) {
-    int optin = 0, sms = 1;
+int plan_launches(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, int device,
+                  std::vector<LaunchShape> *out) {
+    int optin = 0, sms = 1, beside = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     for (size_t c = 0; c < b->classes.size(); ++c) {
@@ -711,8 +727,26 @@ int plan_launches(const hbg_batch *b, const hbg_gpu_options &o, int device, std:
         sh.threads = best_t;
         sh.blocks = blocks;
         sh.team = std::min(b->team, best_t / 32);
+        if (sh.byte_threads > 0) {     // a few long subjects: as many CTAs as they make tiles
+            const int32_t tile = class_tile_subjects(b, sh.n_long, db, lc, blocks);
+            sh.blocks = (int)std::min<int64_t>(blocks, (int64_t)((sh.n_long + tile - 1) / tile) * lc.count);
+            beside = std::max(beside, sh.blocks);
+        }
     }
+    // the long subjects are searched beside byte_kernel, which leaves SMs for
+    // them (its CTAs stay to the end and fill theirs)
+    for (LaunchShape &sh : *out)
+        if (sh.byte_threads > 0)
+            sh.byte_blocks = std::max(1, sh.byte_blocks - std::min(beside, sms / 8));
     return HBG_OK;
+}
+
+// byte_kernel and wordfinder_kernel both have a part of the search.
+bool has_long(const hbg_db *db, const std::vector<LaunchShape> &shapes) {
+    for (const LaunchShape &sh : shapes)
+        if (sh.byte_threads > 0 && sh.n_long > 0 && sh.n_long < db->n)
+            return true;
+    return false;
 }
 
 void drop_graph(hbg_result *r) {
@@ -781,6 +815,8 @@ int prepare_result(hbg_result *r, int64_t cap) {
         if (r->shapes[c].byte_threads > 0 && r->batch->classes[c].cell == 1)
             side = std::max<int64_t>(side, (int64_t)r->shapes[c].byte_blocks * (r->shapes[c].byte_threads / 32) *
                                                r->batch->classes[c].table_len);
+    if (has_long(r->db, r->shapes))
+        CU(KitPool::add_side(&r->kit));
     if (side > r->side_entries) {
         drop_graph(r);
         dfree(r->d_side);
@@ -860,9 +896,21 @@ hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass 
 // `a` holds scratch and outputs (tile_counter: one counter per class), `next` a
 // subject counter per group, both zeroed.  The caller has run
 // wordfinder_configure and byte_configure (not stream operations).
+//
+// Subjects too long for byte_kernel's cells are few and one warp walks each, so
+// with `kit` they go on its side stream (without, `next` may be a.g_hits, which
+// byte_kernel must find zeroed: it goes first): one query of 350 letters against
+// 300,000 subjects 1.30 ms, with one subject of 35,000 letters besides 1.60, after
+// the others 2.85; 16 queries of 500 letters against 100,000 4.67, 11.0, 15.8.
 int launch_finders(const hbg_db *db, const hbg_batch *b, const std::vector<LaunchShape> &shapes,
                    const hbg_gpu_options &opt, hbg::WordFinderArgs a, unsigned long long *next, uint16_t *side,
-                   cudaStream_t st, int *launches) {
+                   const HostKit *kit, cudaStream_t st, int *launches) {
+    const bool beside = kit && has_long(db, shapes);
+    cudaStream_t other = beside ? kit->side : st;   // wordfinder_kernel's
+    if (beside) {
+        CU(cudaEventRecord(kit->fork, st));
+        CU(cudaStreamWaitEvent(other, kit->fork, 0));
+    }
     hbg_gpu_options std_opt;
     hbg_default_gpu_options(&std_opt);
     const bool together = opt.num_threadsx < std_opt.num_threadsx;
@@ -901,8 +949,12 @@ int launch_finders(const hbg_db *db, const hbg_batch *b, const std::vector<Launc
         a.n_tiles = (int64_t)a.tiles_per_group * ((lc.count + a.team - 1) / a.team);
         a.tile_counter = tiles + c;
         a.smem_diag = lc.smem_diag;
-        CU(hbg::launch_wordfinder(a, lc.mode, shapes[c].blocks, shapes[c].threads, st));
+        CU(hbg::launch_wordfinder(a, lc.mode, shapes[c].blocks, shapes[c].threads, other));
         ++*launches;
+    }
+    if (beside) {
+        CU(cudaEventRecord(kit->join, other));
+        CU(cudaStreamWaitEvent(st, kit->join, 0));
     }
     return HBG_OK;
 }
@@ -960,7 +1012,8 @@ int enqueue_search(hbg_result *r) {
         cap_status == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     CU(cudaEventRecordWithFlags(r->kit.ev[0], st, ev_flags));
     int wf_launches = 0;
-    const int rc = launch_finders(db, b, r->shapes, r->shape_opt, a, r->d_counters + 1 + 6 * nq + ng, r->d_side, st, &wf_launches);
+    const int rc = launch_finders(db, b, r->shapes, r->shape_opt, a, r->d_counters + 1 + 6 * nq + ng, r->d_side, &r->kit, st,
+                                  &wf_launches);
     if (rc != HBG_OK)
         return rc;
     CU(cudaEventRecordWithFlags(r->kit.ev[1], st, ev_flags));
@@ -1820,7 +1873,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
         return fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
     }
     plan_bytes(batch, db, o, db->device, &r->shapes);
-    rc = plan_launches(batch, o, db->device, &r->shapes);
+    rc = plan_launches(batch, db, o, db->device, &r->shapes);
     if (rc != HBG_OK) {
         if (!*out)
             delete r;
@@ -1845,8 +1898,10 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     if (rc == HBG_OK)
         rc = launch_search(r);
     if (rc != HBG_OK) {
+        cudaStreamSynchronize(r->stream);       // a partly enqueued search may still run
+        if (r->kit.side)
+            cudaStreamSynchronize(r->kit.side);
         if (!*out) {
-            cudaStreamSynchronize(r->stream);   // a partly enqueued search may still run
             free_result_device(r);
             delete r;
         }
@@ -1873,6 +1928,8 @@ int hbg_result_sync(hbg_result *r) {
             rc = launch_search(r);
         if (rc != HBG_OK) {
             cudaStreamSynchronize(r->stream);
+            if (r->kit.side)
+                cudaStreamSynchronize(r->kit.side);
             r->launched = false;
             return rc;
         }
@@ -2100,7 +2157,7 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     CU(hbg::byte_configure());
     std::vector<LaunchShape> shapes;   // host-side only; no device allocation
     plan_bytes(batch, db, o, db->device, &shapes);
-    rc = plan_launches(batch, o, db->device, &shapes);
+    rc = plan_launches(batch, db, o, db->device, &shapes);
     if (rc != HBG_OK)
         return rc;
     cudaStream_t st = (cudaStream_t)stream;
@@ -2146,7 +2203,7 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     // 16-bit cells (longer groups are refused above), so no side table; the
     // group counters serve as subject counters
     int launches = 0;
-    rc = launch_finders(db, batch, shapes, o, a, g_hits, nullptr, st, &launches);
+    rc = launch_finders(db, batch, shapes, o, a, g_hits, nullptr, nullptr, st, &launches);
     if (rc != HBG_OK)
         return rc;
     // per-query extension and kept counts follow the HSP count in d_counts

@@ -217,3 +217,28 @@ def test_many_groups_few_subjects(built, n_groups, n_subjects):
         assert np.array_equal(mine["score"], hsps["score"]) and np.array_equal(mine["s_start"], hsps["s_start"])
         st = got.stats[k]
         assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
+
+
+@pytest.mark.parametrize("qlens,lens", [((300,), (32727,)), ((300, 2000, 4000, 5000), (32726, 32727, 40000, 65535, 65536, 70000)),
+                                        ((5000, 20), (65536,) * 20)])
+@pytest.mark.parametrize("own_stream", [False, True])
+def test_long_subjects_beside_the_others(built, qlens, lens, own_stream):
+    """Subjects too long for the cells are searched on a stream of their own beside
+    the others: the same result from the first launch, a captured one and its replays."""
+    import torch
+    rng = np.random.default_rng(len(qlens))
+    qs = [synth.random_letters(rng, n) for n in qlens]
+    res, off = database(rng, qs[0], lens)
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 30) for q in qs]
+    gdb = hblast.Database(res, off)
+    s = hblast.Searcher(gdb, hblast.Batch.proteins(pqs))
+    stream = torch.cuda.Stream() if own_stream else None
+    first = None
+    for _ in range(4):
+        s.launch(stream.cuda_stream if stream else None)
+        s.wait()
+        got = s.result()
+        if first is None:
+            first = got
+            check(got, pqs, res, off, threads=16)
+        assert np.array_equal(got.hsps, first.hsps) and got.stats == first.stats

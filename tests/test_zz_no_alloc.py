@@ -88,3 +88,27 @@ def test_search_static_rejects_what_needs_global_tables(built):
     d_counts = torch.zeros(3, dtype=torch.int64, device="cuda")
     rc = call_static(gdb, batch, d_hsps, 16, d_counts, torch.cuda.current_stream())
     assert rc == hblast.core.HBG_ERR_TOO_LONG
+
+
+def test_search_static_longest_subject(built):
+    """The longest subject it takes has positions past byte_kernel's cells: two
+    kernels share the counters in its scratch."""
+    import torch
+    rng = np.random.default_rng(33)
+    q = synth.random_letters(rng, 300)
+    subs = [np.concatenate([synth.mutate(rng, q, 0.8), synth.random_letters(rng, n - 300)]) for n in (32727, 32726, 400, 350, 300)]
+    off = np.zeros(6, np.int64)
+    off[1:] = np.cumsum([len(s) for s in subs])
+    gdb = hblast.Database(np.concatenate(subs), off)
+    batch = hblast.Batch.proteins([hblast.ProteinQuery.blastp(q)])
+    ref = hblast.search(gdb, batch)
+    assert set(ref.hsps["subject"]) == set(range(5))
+    d_hsps = torch.zeros(9 * (len(ref.hsps) + 8), dtype=torch.int32, device="cuda")
+    d_counts = torch.zeros(3, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        assert call_static(gdb, batch, d_hsps, len(ref.hsps) + 8, d_counts, torch.cuda.current_stream()) == 0
+        torch.cuda.synchronize()
+        got = d_hsps.cpu().numpy().view(HSP_DTYPE)[:len(ref.hsps)]
+        got = got[np.lexsort((got["q_off"], got["s_off"], got["subject"], got["query"]))]
+        assert d_counts[0] == len(ref.hsps) and np.array_equal(got, ref.hsps)
