@@ -403,7 +403,7 @@ void ensure_tables(const hbg_batch *batch) {
 int64_t batch_entries(const hbg_batch *batch) {
     hbg_batch *b = const_cast<hbg_batch *>(batch);
     std::lock_guard<std::mutex> lock(b->tables_mu);
-    return hbg::count_entries(b->host);
+    return hbg::count_entries(&b->host);
 }
 
 // Upload at the first search; a failed upload gives back what it allocated,

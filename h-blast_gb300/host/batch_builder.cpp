@@ -291,18 +291,90 @@ NeighbourCache &prepared_cache(const HostBatch &b) {
 
 }  // namespace
 
-int64_t count_entries(const HostBatch &b) {
+// Neighbours of every word at a threshold, without listing them: sums of two
+// letters' scores are counted once (at[a][b][v]: pairs (x, y) with score(a, x) +
+// score(b, y) >= v), and a word's neighbours are the pairs that each third
+// letter's score leaves room for.  One table per threshold, kept: 64 KiB, at most
+// 418 of them (lower and higher thresholds count as the ends of the range).
+constexpr int kScoreMin = -128, kScoreMax = 11;
+
+const uint16_t *neighbour_counts(int32_t threshold) {
+    constexpr int kPairMin = 2 * kScoreMin, kPairs = 2 * (kScoreMax - kScoreMin) + 1;
+    typedef std::array<uint16_t, kPairs + 1> Sums;
+    struct Row {
+        std::vector<std::pair<int, int>> values;   // score, letters with it
+    };
+    static std::mutex mu;
+    static std::vector<Row> rows;
+    static std::vector<Sums> at;
+    static std::map<int32_t, std::vector<uint16_t>> tables;
+    threshold = std::min(std::max(threshold, 3 * kScoreMin), 3 * kScoreMax + 1);
+    std::lock_guard<std::mutex> lock(mu);
+    if (at.empty()) {
+        std::vector<Row> r(HBG_ALPHABET);
+        for (int x = 0; x < HBG_ALPHABET; ++x) {
+            std::map<int, int> n;
+            for (int y = 0; y < HBG_ALPHABET; ++y)
+                ++n[kBlosum62[x * 32 + y]];
+            r[x].values.assign(n.begin(), n.end());
+        }
+        std::vector<Sums> sums(HBG_ALPHABET * HBG_ALPHABET, Sums{});
+        for (int x = 0; x < HBG_ALPHABET; ++x)
+            for (int y = 0; y < HBG_ALPHABET; ++y) {
+                Sums &c = sums[x * HBG_ALPHABET + y];
+                for (const auto &u : r[x].values)
+                    for (const auto &v : r[y].values)
+                        c[u.first + v.first - kPairMin] += (uint16_t)(u.second * v.second);
+                for (int k = kPairs - 1; k >= 0; --k)
+                    c[k] = (uint16_t)(c[k] + c[k + 1]);
+            }
+        rows.swap(r);
+        at.swap(sums);
+    }
+    std::vector<uint16_t> &t = tables[threshold];
+    if (t.empty()) {
+        std::vector<uint16_t> n(HBG_NUM_CELLS, 0);
+        for (int x = 0; x < HBG_ALPHABET; ++x)
+            for (int y = 0; y < HBG_ALPHABET; ++y)
+                for (int z = 0; z < HBG_ALPHABET; ++z) {
+                    int sum = 0;
+                    for (const auto &v : rows[z].values) {
+                        const int k = threshold - v.first - kPairMin;
+                        if (k < kPairs)
+                            sum += v.second * at[x * HBG_ALPHABET + y][std::max(k, 0)];
+                    }
+                    n[(x << 10) | (y << 5) | z] = (uint16_t)sum;
+                }
+        t.swap(n);
+    }
+    return t.data();
+}
+
+int64_t count_entries(HostBatch *out) {
+    HostBatch &b = *out;
     if (!b.cells.empty())
         return (int64_t)b.entries.size();
-    const NeighbourCache &nb = prepared_cache(b);
-    int64_t n = 0;
-    for (const HbgGroup &G : b.groups) {
-        const uint8_t *gs = b.letters.data() + G.seq_base;
-        const int32_t *gc = b.ctx_of.data() + G.seq_base;
-        for (int32_t p = 0; p + HBG_WORD_SIZE <= G.glen; ++p)
-            if (valid(gc, p))
-                n += (int64_t)nb.get(gs[p], gs[p + 1], gs[p + 2]).size();
+    if (!b.counted) {
+        const uint16_t *count = neighbour_counts(b.threshold);
+        for (HbgGroup &G : b.groups) {
+            const uint8_t *gs = b.letters.data() + G.seq_base;
+            const int32_t *gc = b.ctx_of.data() + G.seq_base;
+            int64_t n = 0;
+            uint32_t word = 0;
+            int32_t run = 0, before = -1;              // letters of one context so far
+            for (int32_t p = 0; p < G.glen; ++p) {
+                run = gc[p] < 0 ? 0 : (gc[p] == before ? run + 1 : 1);
+                before = gc[p];
+                word = ((word << 5) | gs[p]) & (HBG_NUM_CELLS - 1);
+                n += run >= HBG_WORD_SIZE ? count[word] : 0;
+            }
+            G.n_entries = (int32_t)n;
+        }
+        b.counted = true;
     }
+    int64_t n = 0;
+    for (const HbgGroup &G : b.groups)
+        n += G.n_entries;
     return n;
 }
 

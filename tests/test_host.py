@@ -240,3 +240,22 @@ def test_schedule_validates_before_upload(built):
         with pytest.raises(hblast.HblastError):
             b.schedule(*bad)
     b.close()
+
+
+@pytest.mark.parametrize("threshold", [-1000, -384, -137, -12, 0, 8, 11, 13, 33, 34, 1000])
+def test_entry_count_is_that_of_the_tables(built, threshold):
+    """hbg_batch_info counts entries without building tables: all 27 letters, short
+    queries, several contexts, and thresholds that every word or none reaches."""
+    rng = np.random.default_rng(5)
+    few = threshold < 0                            # up to 21952 entries a letter
+    seqs = [rng.integers(1, 28, size=n).astype(np.uint8) for n in ((2, 3, 4, 40) if few else (1, 2, 3, 4, 700, 3000))]
+    seqs.append(np.array([20, 20, 20, 20], np.uint8))   # the word with the highest score, twice
+    pqs = [hblast.ProteinQuery.blastp(q) for q in seqs]
+    s = np.concatenate([seqs[2], [0], seqs[3], [0], seqs[1]]).astype(np.uint8)
+    o = [0, len(seqs[2]) + 1, len(seqs[2]) + len(seqs[3]) + 2]
+    pqs.append(hblast.ProteinQuery(s, o, [len(seqs[2]), len(seqs[3]), len(seqs[1])], [16] * 3, [41] * 3))
+    b = hblast.Batch.proteins(pqs, threshold=threshold)
+    told = b.info()["lookup_entries"]
+    assert told == sum(len(b.lookup_table(g)[1]) for g in range(b.info()["n_groups"]))
+    assert told == b.info()["lookup_entries"]
+    assert threshold > 33 or told > 0
