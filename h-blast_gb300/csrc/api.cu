@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <exception>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -393,6 +394,17 @@ void free_batch_device(hbg_batch *b) {
 
 int upload_batch_buffers(hbg_batch *b, const hbg_db *db);
 
+// Run host code that allocates or starts threads: what it throws must not leave
+// a C entry point.
+template <typename F>
+int guarded(F &&f) {
+    try {
+        return f();
+    } catch (const std::exception &e) {
+        return fail(HBG_ERR_NOMEM, std::string("host allocation: ") + e.what());
+    }
+}
+
 // Host tables, built when a caller first asks for them.
 void ensure_tables(const hbg_batch *batch) {
     hbg_batch *b = const_cast<hbg_batch *>(batch);
@@ -415,7 +427,7 @@ int upload_batch(hbg_batch *b, const hbg_db *db) {
     if (b->device >= 0)
         return fail(HBG_ERR_STATE, "batch already resident on another device");
     DeviceScope ds(device);
-    const int rc = upload_batch_buffers(b, db);
+    const int rc = guarded([&] { return upload_batch_buffers(b, db); });
     if (rc != HBG_OK) {
         cudaDeviceSynchronize();   // copies already issued may still read the host vectors
         free_batch_device(b);
@@ -1702,7 +1714,12 @@ int hbg_batch_lookup_table(const hbg_batch *b, int32_t g, uint32_t *cells, uint1
                            int32_t *n_queries, int32_t *query_start) {
     if (!b || !n_entries || g < 0 || g >= (int32_t)b->host.groups.size())
         return fail(HBG_ERR_INVALID, "hbg_batch_lookup_table: bad argument");
-    ensure_tables(b);
+    const int rc = guarded([&] {
+        ensure_tables(b);
+        return HBG_OK;
+    });
+    if (rc != HBG_OK)
+        return rc;
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
     const uint32_t *cs = h.cells.data() + (size_t)g * HBG_CELL_STRIDE;
@@ -1800,11 +1817,16 @@ int hbg_batch_info(const hbg_batch *b, int32_t *nq, int32_t *ng, int64_t *qlen, 
             t += q.len;
         *qlen = t;
     }
-    if (entries)
-        *entries = batch_entries(b);
-    if (device_bytes)
-        *device_bytes = batch_device_bytes(b->host, batch_entries(b));
-    return HBG_OK;
+    if (!entries && !device_bytes)
+        return HBG_OK;
+    return guarded([&] {
+        const int64_t n = batch_entries(b);
+        if (entries)
+            *entries = n;
+        if (device_bytes)
+            *device_bytes = batch_device_bytes(b->host, n);
+        return HBG_OK;
+    });
 }
 
 int hbg_mem_required(const hbg_db *db, const hbg_batch *b, int64_t cap, int64_t *bytes) {
@@ -1813,7 +1835,13 @@ int hbg_mem_required(const hbg_db *db, const hbg_batch *b, int64_t cap, int64_t 
     if (cap == 0)
         cap = default_capacity(db, b);
     const hbg::HostBatch &h = b->host;
-    const int64_t batch_bytes = batch_device_bytes(h, batch_entries(b));
+    int64_t batch_bytes = 0;
+    const int rc = guarded([&] {
+        batch_bytes = batch_device_bytes(h, batch_entries(b));
+        return HBG_OK;
+    });
+    if (rc != HBG_OK)
+        return rc;
     int64_t per_hsp = 2 * (int64_t)sizeof(hbg_hsp) + 2 * 8 + 2 * 4;
     int64_t gdiag = 0;
     if (global_diag_len(h, db) > 0) {

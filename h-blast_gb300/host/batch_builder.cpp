@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <exception>
 #include <functional>
 #include <map>
 #include <memory>
@@ -59,14 +60,17 @@ class NeighbourCache {
         std::lock_guard<std::mutex> lock(mu_);
         std::vector<int32_t> keys;
         for (int32_t k : words)
-            if (!done_[k]) {
-                done_[k] = 1;                 // listed once
+            if (!done_[k])
                 keys.push_back(k);
-            }
+        std::sort(keys.begin(), keys.end());  // each listed once
+        keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
         pfor((int64_t)keys.size(), [&](int64_t i) {
             const int32_t k = keys[i];
+            lists_[k].clear();                // of a build that ran out of memory
             enumerate((uint8_t)(k >> 10), (uint8_t)((k >> 5) & 31), (uint8_t)(k & 31), &lists_[k]);
         });
+        for (int32_t k : keys)
+            done_[k] = 1;
     }
 
   private:
@@ -107,7 +111,8 @@ NeighbourCache &neighbour_cache(int32_t threshold) {
 }
 
 // Run body(i) for i in [0, n) on up to 16 host threads (items taken from a
-// shared counter).
+// shared counter), on fewer when no more can be started.  The first exception
+// of a body ends the run and comes out of the call.
 void parallel_for(int64_t n, const std::function<void(int64_t)> &body) {
     const int64_t nt = std::min<int64_t>({n, 16, (int64_t)std::max(1u, std::thread::hardware_concurrency())});
     if (nt <= 1) {
@@ -116,16 +121,30 @@ void parallel_for(int64_t n, const std::function<void(int64_t)> &body) {
         return;
     }
     std::atomic<int64_t> next{0};
+    std::mutex mu;
+    std::exception_ptr first;
     auto run = [&] {
-        for (int64_t i = next++; i < n; i = next++)
-            body(i);
+        try {
+            for (int64_t i = next++; i < n; i = next++)
+                body(i);
+        } catch (...) {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!first)
+                first = std::current_exception();
+            next = n;
+        }
     };
     std::vector<std::thread> th;
-    for (int64_t t = 1; t < nt; ++t)
-        th.emplace_back(run);
+    try {
+        for (int64_t t = 1; t < nt; ++t)
+            th.emplace_back(run);
+    } catch (const std::exception &) {
+    }
     run();
     for (std::thread &x : th)
         x.join();
+    if (first)
+        std::rethrow_exception(first);
 }
 
 int32_t next_pow2(int32_t v) {
@@ -382,6 +401,17 @@ int64_t count_entries(HostBatch *out) {
 // and entries).
 void build_tables(HostBatch *out) {
     HostBatch &b = *out;
+    struct Undo {                      // an exception leaves no half-built tables
+        HostBatch *b;
+        ~Undo() {
+            if (b) {
+                b->cells = std::vector<uint32_t>();
+                b->pv = std::vector<uint32_t>();
+                b->query_cells = std::vector<uint16_t>();
+                b->entries = std::vector<uint16_t>();
+            }
+        }
+    } undo{out};
     const int32_t n_groups = (int32_t)b.groups.size();
     const double mode_hits = b.mode_hits;
     const NeighbourCache &nb = prepared_cache(b);
@@ -457,6 +487,7 @@ void build_tables(HostBatch *out) {
                 ge[cursor[w]++] = (uint16_t)p;
         }
     });
+    undo.b = nullptr;
 }
 
 // --- six-frame translation ------------------------------------------------

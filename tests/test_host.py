@@ -4,6 +4,8 @@ kernel is launched here."""
 import ctypes as C
 import json
 import re
+import subprocess
+import sys
 from pathlib import Path
 
 import numpy as np
@@ -259,3 +261,35 @@ def test_entry_count_is_that_of_the_tables(built, threshold):
     assert told == sum(len(b.lookup_table(g)[1]) for g in range(b.info()["n_groups"]))
     assert told == b.info()["lookup_entries"]
     assert threshold > 33 or told > 0
+
+
+_LITTLE_MEMORY = """
+import resource, sys
+sys.path[:0] = {paths!r}
+import numpy as np, hblast
+from hblast import synth
+q = synth.random_letters(np.random.default_rng(0), 20000)
+b = hblast.Batch.proteins([hblast.ProteinQuery.blastp(q)] * 3, threshold=0, max_group_len=1)
+n = b.info()["lookup_entries"]                       # and the library's first allocations
+used = resource.getpagesize() * int(open("/proc/self/statm").read().split()[0])
+resource.setrlimit(resource.RLIMIT_AS, (used + (192 << 20), resource.RLIM_INFINITY))
+for _ in range(2):
+    try:
+        b.lookup_table(0)
+        sys.exit("the tables fitted")
+    except hblast.HblastError as e:
+        assert e.code == hblast.core.HBG_ERR_NOMEM, e
+resource.setrlimit(resource.RLIMIT_AS, (resource.RLIM_INFINITY, resource.RLIM_INFINITY))
+assert b.info()["lookup_entries"] == n == sum(len(b.lookup_table(g)[1]) for g in range(3))
+cells, ents, _, _ = b.lookup_table(1)
+assert np.all(np.diff(ents[cells[5000]:cells[5001]].astype(int)) > 0)
+print("ok")
+"""
+
+
+def test_tables_without_host_memory_are_an_error(built):
+    """Tables that a caller asks to see are built then, and may not fit: an error
+    code, not an exception through the C entry, and right once there is room."""
+    code = _LITTLE_MEMORY.format(paths=[str(p) for p in (ROOT / "h-blast_gb300", ROOT)])
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout, r.stderr)
