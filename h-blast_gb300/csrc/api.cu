@@ -327,9 +327,9 @@ struct hbg_batch {
     int32_t *d_group_list = nullptr;   // groups ordered by launch class
     uint32_t *d_packed = nullptr;      // cells of byte_kernel
     uint2 *d_stats = nullptr;          // per group: entries, fullest cell
-    uint16_t *d_more = nullptr;        // entries, when they did not fit the block
+    uint32_t *d_counts = nullptr;      // scratch of the table build
     std::vector<LaunchClass> classes;
-    std::mutex tables_mu;              // host tables are built when first asked for
+    std::mutex tables_mu;              // host tables and entry counts are made when first asked for
     bool caller_tables = false;        // the tables are the caller's (in `host`)
     bool repeated_entries = false;     // a caller's lookup table lists an offset twice in a cell
     bool tuned = false;                // the caller chose tiles or table placement (hbg_batch_tune)
@@ -380,16 +380,9 @@ struct hbg_result {
 
 namespace {
 
-int64_t batch_device_bytes(const hbg::HostBatch &h, int64_t entries) {
-    const int64_t ng = (int64_t)h.groups.size(), nq = (int64_t)h.queries.size();
-    return (int64_t)(h.groups.size() * sizeof(HbgGroup) + h.contexts.size() * sizeof(HbgContext) +
-                     h.queries.size() * sizeof(HbgQueryDesc) + h.letters.size() + h.ctx_of.size() * 4) +
-           ng * (HBG_CELL_STRIDE + HBG_PV_WORDS + HBG_NUM_CELLS) * 4 + entries * 2 + nq * HBG_NUM_CELLS * 2;
-}
-
 void free_batch_device(hbg_batch *b) {
     dfree_idle(b->d_arena);
-    dfree_idle(b->d_more);
+    dfree_idle(b->d_counts);
 }
 
 int upload_batch_buffers(hbg_batch *b, const hbg_db *db);
@@ -405,17 +398,96 @@ int guarded(F &&f) {
     }
 }
 
+// A batch on the device: one block, 256-byte aligned parts in it.  First what
+// is copied there (`upload` bytes; with a caller's own tables, these too), then
+// what the device makes.
+struct BatchLayout {
+    std::vector<hbg::TableSegment> segs;       // of the table build
+    int32_t slice = 0;                         // most of them built at a time
+    size_t groups = 0, ctx = 0, queries = 0, letters = 0, ctx_of = 0, list = 0, segments = 0, cells = 0, pv = 0, qcells = 0,
+           entries = 0, packed = 0, stats = 0;
+    size_t upload = 0, total = 0;
+
+    size_t scratch() const { return (size_t)slice * HBG_NUM_CELLS * sizeof(uint32_t); }
+};
+
+// Segments of the table build that are in hand at a time: 128 KiB of scratch
+// each.  A slice is whole groups, and a group of 65,000 letters has at most 191
+// segments.
+constexpr int32_t kSliceSegments = 512;
+
+// The groups of the slice that starts with group g, and its segments.
+int32_t slice_end(const hbg::HostBatch &h, int32_t g, int32_t *n_segs) {
+    int32_t n = 0;
+    for (; g < (int32_t)h.groups.size() && (n == 0 || n + h.groups[g].n_segs <= kSliceSegments); ++g)
+        n += h.groups[g].n_segs;
+    *n_segs = n;
+    return g;
+}
+
+// Counts the batch's entries, cuts it into segments and lays it out (the groups
+// learn their segments and the place of their entries).  Under tables_mu.
+BatchLayout lay_out(hbg_batch *b) {
+    hbg::HostBatch &h = b->host;
+    BatchLayout L;
+    const size_t ng = h.groups.size(), nq = h.queries.size();
+    const size_t n_entries = (size_t)hbg::count_entries(&h);
+    int64_t base = 0;
+    for (size_t g = 0; g < ng; ++g) {
+        HbgGroup &G = h.groups[g];
+        G.entry_base = base;
+        base += G.n_entries;
+        G.seg_base = (int32_t)L.segs.size();
+        for (int32_t q = G.first_query; q < G.first_query + G.n_queries; ++q) {
+            const int32_t at = h.queries[q].start, end = at + h.queries[q].len - HBG_WORD_SIZE + 1;
+            for (int32_t p = at; p == at || p < end; p += hbg::kTableSegment)
+                L.segs.push_back({(int32_t)g, q, p, std::min(end, p + hbg::kTableSegment)});
+        }
+        G.n_segs = (int32_t)L.segs.size() - G.seg_base;
+    }
+    size_t at = 0;
+    auto place = [&](size_t bytes, size_t before = 0, size_t after = 0) {
+        const size_t p = at + before;
+        at = (p + bytes + after + 255) / 256 * 256;
+        return p;
+    };
+    auto tables = [&] {
+        L.cells = place(ng * HBG_CELL_STRIDE * sizeof(uint32_t));
+        L.pv = place(ng * HBG_PV_WORDS * sizeof(uint32_t));
+        L.qcells = place(nq * HBG_NUM_CELLS * sizeof(uint16_t));
+        L.entries = place(n_entries * sizeof(uint16_t), 0, 128);   // byte_kernel reads up to 31 entries past a cell
+    };
+    L.groups = place(ng * sizeof(HbgGroup));
+    L.ctx = place(h.contexts.size() * sizeof(HbgContext));
+    L.queries = place(nq * sizeof(HbgQueryDesc));
+    L.letters = place(h.letters.size(), kFrontPad, 64);            // extensions read whole blocks
+    L.ctx_of = place(h.ctx_of.size() * sizeof(int32_t), 0, 64);
+    L.list = place(ng * sizeof(int32_t));
+    if (b->caller_tables) {
+        L.segs.clear();
+        tables();
+    } else {
+        L.segments = place(L.segs.size() * sizeof(hbg::TableSegment));
+        for (int32_t g = 0, n; g < (int32_t)ng;) {
+            g = slice_end(h, g, &n);
+            L.slice = std::max(L.slice, n);
+        }
+    }
+    L.upload = at;
+    if (!b->caller_tables)
+        tables();
+    L.packed = place(ng * HBG_NUM_CELLS * sizeof(uint32_t));
+    L.stats = place(ng * sizeof(uint2));
+    L.total = at;
+    return L;
+}
+
 // Host tables, built when a caller first asks for them.
 void ensure_tables(const hbg_batch *batch) {
     hbg_batch *b = const_cast<hbg_batch *>(batch);
     std::lock_guard<std::mutex> lock(b->tables_mu);
     if (b->host.cells.empty())
         hbg::build_tables(&b->host);
-}
-int64_t batch_entries(const hbg_batch *batch) {
-    hbg_batch *b = const_cast<hbg_batch *>(batch);
-    std::lock_guard<std::mutex> lock(b->tables_mu);
-    return hbg::count_entries(&b->host);
 }
 
 // Upload at the first search; a failed upload gives back what it allocated,
@@ -463,7 +535,7 @@ int byte_cell(const hbg_batch *b, int32_t g) {
 }
 
 // The launch classes of a batch and its groups in class order.
-int make_classes(hbg_batch *b, std::vector<int32_t> *list) {
+int make_classes(const hbg_batch *b, std::vector<LaunchClass> *classes, std::vector<int32_t> *list) {
     const hbg::HostBatch &h = b->host;
     // launch classes: (mode, table size); groups with shared tables are
     // launched by table size, so a short query's warps reserve only the
@@ -486,149 +558,108 @@ int make_classes(hbg_batch *b, std::vector<int32_t> *list) {
     std::stable_sort(keyed.begin(), keyed.end(),
                      [](const auto &x, const auto &y) { return x.first < y.first; });
     list->clear();
-    b->classes.clear();
+    classes->clear();
     for (size_t i = 0; i < keyed.size(); ++i) {
         const bool global = h.groups[keyed[i].second].placement != 0;
         if (i == 0 || keyed[i].first != keyed[i - 1].first)
-            b->classes.push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
+            classes->push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
                                              -keyed[i].first[2] & 3, -keyed[i].first[2] / 4});
-        LaunchClass &lc = b->classes.back();
+        LaunchClass &lc = classes->back();
         lc.count++;
         if (lc.cell == 1)              // the longest group's exact table
             lc.table_len = std::max(lc.count == 1 ? 0 : lc.table_len,
                                     hbg::byte_table_len(h.groups[keyed[i].second].glen + h.window));
         list->push_back(keyed[i].second);
     }
-    if ((int)b->classes.size() > kMaxLaunchClasses)
+    if ((int)classes->size() > kMaxLaunchClasses)
         return fail(HBG_ERR_INVALID, "too many launch classes");
     return HBG_OK;
 }
 
-// Entries the device block has room for, per letter of the batch: random
-// proteins have 17 at threshold 11 (30 at 10); more take a block of their own.
-constexpr int64_t kEntriesPerLetter = 40;
-
 int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
     hbg::HostBatch &h = b->host;
-    const size_t ng = h.groups.size(), nq = h.queries.size();
-    std::vector<hbg::TableSegment> segs;
-    for (size_t g = 0; g < ng; ++g) {
-        HbgGroup &G = h.groups[g];
-        G.seg_base = (int32_t)segs.size();
-        for (int32_t q = G.first_query; q < G.first_query + G.n_queries; ++q) {
-            const int32_t at = h.queries[q].start, end = at + h.queries[q].len - HBG_WORD_SIZE + 1;
-            for (int32_t p = at; p == at || p < end; p += hbg::kTableSegment)
-                segs.push_back({(int32_t)g, q, p, std::min(end, p + hbg::kTableSegment)});
-        }
-        G.n_segs = (int32_t)segs.size() - G.seg_base;
-    }
-    const bool on_device = !b->caller_tables && h.cells.empty() && hbg::tables_fit((int64_t)segs.size());
-    if (!on_device)
-        ensure_tables(b);
+    const size_t ng = h.groups.size();
+    std::unique_lock<std::mutex> lock(b->tables_mu);
+    const BatchLayout L = lay_out(b);
     std::vector<int32_t> list;
-    int rc = make_classes(b, &list);             // again below if a cell turns out too full
+    int rc = make_classes(b, &b->classes, &list);   // again below if a cell turns out too full
     if (rc != HBG_OK)
         return rc;
-    // one block, one copy: the arrays in turn, 256-byte aligned, then what the
-    // device makes itself.  (Ten copies of their own took 80 us.)
-    std::vector<std::pair<size_t, std::pair<const void *, size_t>>> parts;   // place, source, bytes
-    size_t at = 0;
-    auto place = [&](const void *src, size_t bytes, size_t before, size_t after) {
-        const size_t p = at + before;
-        if (src)
-            parts.push_back({p, {src, bytes}});
-        at = (p + bytes + after + 255) / 256 * 256;
-        return p;
-    };
-    const size_t b_cells = ng * HBG_CELL_STRIDE * sizeof(uint32_t), b_pv = ng * HBG_PV_WORDS * sizeof(uint32_t),
-                 b_qcells = nq * HBG_NUM_CELLS * sizeof(uint16_t);
-    // letters: kFrontPad zeros before (extensions read whole blocks), 64 after
-    const size_t o_groups = place(h.groups.data(), ng * sizeof(HbgGroup), 0, 0);
-    const size_t o_ctx = place(h.contexts.data(), h.contexts.size() * sizeof(HbgContext), 0, 0);
-    const size_t o_queries = place(h.queries.data(), nq * sizeof(HbgQueryDesc), 0, 0);
-    const size_t o_letters = place(h.letters.data(), h.letters.size(), kFrontPad, 64);
-    const size_t o_ctx_of = place(h.ctx_of.data(), h.ctx_of.size() * sizeof(int32_t), 0, 64);
-    const size_t o_list = place(list.data(), list.size() * sizeof(int32_t), 0, 0);
-    const size_t o_segs = place(segs.data(), segs.size() * sizeof(hbg::TableSegment), 0, 0);
-    size_t o_cells = 0, o_pv = 0, o_qcells = 0, o_entries = 0;
-    if (!on_device) {
-        o_cells = place(h.cells.data(), b_cells, 0, 0);
-        o_pv = place(h.pv.data(), b_pv, 0, 0);
-        o_qcells = place(h.query_cells.data(), b_qcells, 0, 0);
-        o_entries = place(h.entries.data(), h.entries.size() * sizeof(uint16_t), 0, 128);
-    }
-    const size_t upload = at;
-    const int64_t cap = std::max<int64_t>(1024, kEntriesPerLetter * (int64_t)h.letters.size());
-    // byte_kernel reads up to 31 entries past a cell
-    if (on_device) {
-        o_cells = place(nullptr, b_cells, 0, 0);
-        o_pv = place(nullptr, b_pv, 0, 0);
-        o_qcells = place(nullptr, b_qcells, 0, 0);
-        o_entries = place(nullptr, (size_t)cap * sizeof(uint16_t), 0, 128);
-    }
-    const size_t o_packed = place(nullptr, ng * HBG_NUM_CELLS * sizeof(uint32_t), 0, 0);
-    const size_t o_stats = place(nullptr, ng * sizeof(uint2), 0, 0);
-    const size_t o_counts = place(nullptr, on_device ? segs.size() * HBG_NUM_CELLS * sizeof(uint32_t) : 0, 0, 0);
-    std::unique_ptr<uint8_t[]> stage(new (std::nothrow) uint8_t[upload]);
+    // one copy (ten of their own took 80 us)
+    std::unique_ptr<uint8_t[]> stage(new (std::nothrow) uint8_t[L.upload]);
     if (!stage)
         return fail(HBG_ERR_NOMEM, "host allocation");
     size_t done = 0;
-    for (const auto &p : parts) {
-        memset(stage.get() + done, 0, p.first - done);
-        if (p.second.second)
-            memcpy(stage.get() + p.first, p.second.first, p.second.second);
-        done = p.first + p.second.second;
+    auto put = [&](size_t at, const void *src, size_t bytes) {     // in ascending order; zeros between
+        memset(stage.get() + done, 0, at - done);
+        if (bytes)
+            memcpy(stage.get() + at, src, bytes);
+        done = at + bytes;
+    };
+    put(L.groups, h.groups.data(), ng * sizeof(HbgGroup));
+    put(L.ctx, h.contexts.data(), h.contexts.size() * sizeof(HbgContext));
+    put(L.queries, h.queries.data(), h.queries.size() * sizeof(HbgQueryDesc));
+    put(L.letters, h.letters.data(), h.letters.size());
+    put(L.ctx_of, h.ctx_of.data(), h.ctx_of.size() * sizeof(int32_t));
+    put(L.list, list.data(), list.size() * sizeof(int32_t));
+    if (b->caller_tables) {
+        put(L.cells, h.cells.data(), h.cells.size() * sizeof(uint32_t));
+        put(L.pv, h.pv.data(), h.pv.size() * sizeof(uint32_t));
+        put(L.qcells, h.query_cells.data(), h.query_cells.size() * sizeof(uint16_t));
+        put(L.entries, h.entries.data(), h.entries.size() * sizeof(uint16_t));
+    } else {
+        put(L.segments, L.segs.data(), L.segs.size() * sizeof(hbg::TableSegment));
     }
-    memset(stage.get() + done, 0, upload - done);
-    CU(dalloc(&b->d_arena, at));
-    b->d_groups = reinterpret_cast<HbgGroup *>(b->d_arena + o_groups);
-    b->d_ctx = reinterpret_cast<HbgContext *>(b->d_arena + o_ctx);
-    b->d_queries = reinterpret_cast<HbgQueryDesc *>(b->d_arena + o_queries);
-    b->d_letters = b->d_arena + o_letters;
-    b->d_ctx_of = reinterpret_cast<int32_t *>(b->d_arena + o_ctx_of);
-    b->d_group_list = reinterpret_cast<int32_t *>(b->d_arena + o_list);
-    b->d_cells = reinterpret_cast<uint32_t *>(b->d_arena + o_cells);
-    b->d_pv = reinterpret_cast<uint32_t *>(b->d_arena + o_pv);
-    b->d_qcells = reinterpret_cast<uint16_t *>(b->d_arena + o_qcells);
-    b->d_entries = reinterpret_cast<uint16_t *>(b->d_arena + o_entries);
-    b->d_packed = reinterpret_cast<uint32_t *>(b->d_arena + o_packed);
-    b->d_stats = reinterpret_cast<uint2 *>(b->d_arena + o_stats);
+    put(L.upload, nullptr, 0);
+    lock.unlock();
+    CU(dalloc(&b->d_arena, L.total));
+    b->d_groups = reinterpret_cast<HbgGroup *>(b->d_arena + L.groups);
+    b->d_ctx = reinterpret_cast<HbgContext *>(b->d_arena + L.ctx);
+    b->d_queries = reinterpret_cast<HbgQueryDesc *>(b->d_arena + L.queries);
+    b->d_letters = b->d_arena + L.letters;
+    b->d_ctx_of = reinterpret_cast<int32_t *>(b->d_arena + L.ctx_of);
+    b->d_group_list = reinterpret_cast<int32_t *>(b->d_arena + L.list);
+    b->d_cells = reinterpret_cast<uint32_t *>(b->d_arena + L.cells);
+    b->d_pv = reinterpret_cast<uint32_t *>(b->d_arena + L.pv);
+    b->d_qcells = reinterpret_cast<uint16_t *>(b->d_arena + L.qcells);
+    b->d_entries = reinterpret_cast<uint16_t *>(b->d_arena + L.entries);
+    b->d_packed = reinterpret_cast<uint32_t *>(b->d_arena + L.packed);
+    b->d_stats = reinterpret_cast<uint2 *>(b->d_arena + L.stats);
+    if (!b->caller_tables)
+        CU(dalloc(&b->d_counts, L.scratch() / sizeof(uint32_t)));
     cudaStream_t st = nullptr;
     CU(db->kits->upload_stream(&st));
-    CU(cudaMemcpyAsync(b->d_arena, stage.get(), upload, cudaMemcpyHostToDevice, st));
-    if (!on_device) {
+    CU(cudaMemcpyAsync(b->d_arena, stage.get(), L.upload, cudaMemcpyHostToDevice, st));
+    if (b->caller_tables) {
         CU(hbg::launch_pack_cells(b->d_cells, (int32_t)ng, b->d_packed, st));
     } else {
-        hbg::TableArgs t{b->d_groups, reinterpret_cast<const hbg::TableSegment *>(b->d_arena + o_segs), b->d_letters,
-                         b->d_ctx_of, h.threshold, b->d_cells, b->d_packed, b->d_pv, b->d_entries, cap, b->d_qcells,
-                         b->d_stats, reinterpret_cast<uint32_t *>(b->d_arena + o_counts)};
-        const int32_t n_segs = (int32_t)segs.size();
+        hbg::TableArgs t{b->d_groups, reinterpret_cast<const hbg::TableSegment *>(b->d_arena + L.segments), 0, 0,
+                         b->d_letters, b->d_ctx_of, h.threshold, b->d_cells, b->d_packed, b->d_pv, b->d_entries,
+                         b->d_qcells, b->d_stats, b->d_counts};
+        for (int32_t g = 0, n; g < (int32_t)ng;) {
+            const int32_t end = slice_end(h, g, &n);
+            t.first_group = g;
+            t.first_seg = h.groups[g].seg_base;
+            CU(hbg::launch_tables(t, end - g, n, st));
+            g = end;
+        }
         std::vector<uint2> stats(ng);
-        CU(hbg::launch_tables(t, (int32_t)ng, n_segs, false, st));
         CU(cudaMemcpyAsync(stats.data(), b->d_stats, ng * sizeof(uint2), cudaMemcpyDeviceToHost, st));
         CU(cudaStreamSynchronize(st));
-        int64_t total = 0;
         bool again = false;
         for (size_t g = 0; g < ng; ++g) {
-            total += stats[g].x;
-            h.groups[g].n_entries = (int32_t)stats[g].x;
             h.groups[g].max_count = (int32_t)stats[g].y;
-            again = again || (int32_t)stats[g].y > hbg::kByteMaxCount || (int32_t)stats[g].x >= hbg::kByteMaxEntries;
-        }
-        if (total > cap) {
-            CU(dalloc(&b->d_more, (size_t)total + 64));
-            b->d_entries = t.entries = b->d_more;
-            t.entries_cap = total;
-            CU(hbg::launch_tables(t, (int32_t)ng, n_segs, true, st));
+            again = again || (int32_t)stats[g].y > hbg::kByteMaxCount;
         }
         if (again) {
-            rc = make_classes(b, &list);
+            rc = make_classes(b, &b->classes, &list);
             if (rc != HBG_OK)
                 return rc;
             CU(cudaMemcpyAsync(b->d_group_list, list.data(), list.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
         }
     }
     CU(cudaStreamSynchronize(st));   // the search may run on any stream
+    dfree_idle(b->d_counts);
     b->device = db->device;
     return HBG_OK;
 }
@@ -660,9 +691,9 @@ int32_t class_tile_subjects(const hbg_batch *b, int32_t n_subj, const hbg_db *db
 
 // Which classes byte_kernel takes, with which CTA, and the subjects that stay
 // with wordfinder_kernel: those whose positions do not fit its cells.
-void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, int device,
-                std::vector<LaunchShape> *shapes) {
-    shapes->assign(b->classes.size(), LaunchShape{32, 1, 1, 0, 0, 0});
+void plan_bytes(const hbg_batch *b, const std::vector<LaunchClass> &classes, const hbg_db *db, const hbg_gpu_options &o,
+                int device, std::vector<LaunchShape> *shapes) {
+    shapes->assign(classes.size(), LaunchShape{32, 1, 1, 0, 0, 0});
     hbg_gpu_options std_opt;
     hbg_default_gpu_options(&std_opt);
     if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx)
@@ -670,8 +701,8 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
     int optin = 0, sms = 1;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    for (size_t c = 0; c < b->classes.size(); ++c) {
-        const LaunchClass &lc = b->classes[c];
+    for (size_t c = 0; c < classes.size(); ++c) {
+        const LaunchClass &lc = classes[c];
         LaunchShape &sh = (*shapes)[c];
         if (!lc.cell)
             continue;
@@ -700,13 +731,13 @@ void plan_bytes(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, 
 // CTA size and grid of each launch class that wordfinder_kernel has a part of: the CTA is halved until its
 // per-warp tables fit the shared-memory carve-out; the grid is one wave at
 // the occupancy that leaves (or the caller's num_blocksx).
-int plan_launches(const hbg_batch *b, const hbg_db *db, const hbg_gpu_options &o, int device,
-                  std::vector<LaunchShape> *out) {
+int plan_launches(const hbg_batch *b, const std::vector<LaunchClass> &classes, const hbg_db *db, const hbg_gpu_options &o,
+                  int device, std::vector<LaunchShape> *out) {
     int optin = 0, sms = 1, beside = 0;
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    for (size_t c = 0; c < b->classes.size(); ++c) {
-        const LaunchClass &lc = b->classes[c];
+    for (size_t c = 0; c < classes.size(); ++c) {
+        const LaunchClass &lc = classes[c];
         LaunchShape &sh = (*out)[c];
         if (sh.byte_threads > 0 && sh.n_long == 0)
             continue;
@@ -786,47 +817,51 @@ void free_result_device(hbg_result *r) {
         r->kits->give(r->kit);
 }
 
-// Some class or subject of this search goes to wordfinder_kernel.
-bool uses_wordfinder(const hbg_result *r) {
-    for (const LaunchShape &sh : r->shapes)
-        if (sh.byte_threads == 0 || sh.n_long > 0)
-            return true;
-    return false;
+// Entries of the scratch that the launches of a search share: global diagonal
+// tables of wordfinder_kernel, flag ends of byte_kernel.
+int64_t gdiag_need(const hbg::HostBatch &h, const hbg_db *db, const std::vector<LaunchShape> &shapes) {
+    int64_t blocks = 0, threads = 0;
+    for (const LaunchShape &sh : shapes)
+        if (sh.byte_threads == 0 || sh.n_long > 0) {
+            blocks = std::max<int64_t>(blocks, sh.blocks);
+            threads = std::max<int64_t>(threads, sh.threads);
+        }
+    return blocks * (threads / 32) * global_diag_len(h, db);
 }
+int64_t side_need(const std::vector<LaunchClass> &classes, const std::vector<LaunchShape> &shapes) {
+    int64_t side = 0;
+    for (size_t c = 0; c < shapes.size(); ++c)
+        if (shapes[c].byte_threads > 0 && classes[c].cell == 1)
+            side = std::max<int64_t>(side, (int64_t)shapes[c].byte_blocks * (shapes[c].byte_threads / 32) * classes[c].table_len);
+    return side;
+}
+size_t counters_need(const hbg::HostBatch &h) { return 3 + 6 * h.queries.size() + 2 * h.groups.size(); }
 
 // Allocate (or grow) the result's device buffers for capacity cap.
 int prepare_result(hbg_result *r, int64_t cap) {
     const hbg::HostBatch &h = r->batch->host;
-    const size_t nq = h.queries.size(), ng = h.groups.size();
     if (!r->d_tile)
         CU(dalloc(&r->d_tile, kMaxLaunchClasses));
     // a failed allocation below leaves the recorded size at 0, so the next
     // search allocates again instead of using a missing buffer
-    if (r->n_counters < 3 + 6 * nq + 2 * ng) {   // first use, or a larger batch
+    if (r->n_counters < counters_need(h)) {   // first use, or a larger batch
         drop_graph(r);
         dfree(r->d_counters);
         r->kits->give(r->kit);
         r->n_counters = 0;
-        CU(dalloc(&r->d_counters, 3 + 6 * nq + 2 * ng));
-        CU(r->kits->take(3 + 6 * nq + 2 * ng, &r->kit));
-        r->n_counters = 3 + 6 * nq + 2 * ng;
+        CU(dalloc(&r->d_counters, counters_need(h)));
+        CU(r->kits->take(counters_need(h), &r->kit));
+        r->n_counters = counters_need(h);
     }
     r->gdiag_len = global_diag_len(h, r->db);
-    if (r->gdiag_len > 0 && uses_wordfinder(r)) {
-        const int64_t need = (int64_t)r->blocks * (r->threads / 32) * r->gdiag_len;
-        if (need > r->gdiag_entries) {
-            drop_graph(r);
-            dfree(r->d_gdiag);
-            r->gdiag_entries = 0;
-            CU(dalloc(&r->d_gdiag, (size_t)need));
-            r->gdiag_entries = need;
-        }
+    const int64_t gdiag = gdiag_need(h, r->db, r->shapes), side = side_need(r->batch->classes, r->shapes);
+    if (gdiag > r->gdiag_entries) {
+        drop_graph(r);
+        dfree(r->d_gdiag);
+        r->gdiag_entries = 0;
+        CU(dalloc(&r->d_gdiag, (size_t)gdiag));
+        r->gdiag_entries = gdiag;
     }
-    int64_t side = 0;
-    for (size_t c = 0; c < r->shapes.size(); ++c)
-        if (r->shapes[c].byte_threads > 0 && r->batch->classes[c].cell == 1)
-            side = std::max<int64_t>(side, (int64_t)r->shapes[c].byte_blocks * (r->shapes[c].byte_threads / 32) *
-                                               r->batch->classes[c].table_len);
     if (has_long(r->db, r->shapes))
         CU(KitPool::add_side(&r->kit));
     if (side > r->side_entries) {
@@ -1114,6 +1149,34 @@ bool valid_opts(const hbg_gpu_options *o) {
 }
 
 }  // namespace
+
+// Device memory of one search: the batch with the scratch of its table build, and
+// a result's buffers, as upload_batch and prepare_result allocate them.
+int hbg::search_bytes(const hbg_db *db, const hbg_batch *batch, const hbg_gpu_options *opt, int64_t cap, int64_t *bytes) {
+    return guarded([&] {
+        hbg_batch *b = const_cast<hbg_batch *>(batch);
+        DeviceScope ds(db->device);
+        CU(hbg::wordfinder_configure());
+        std::lock_guard<std::mutex> lock(b->tables_mu);
+        const BatchLayout L = lay_out(b);
+        std::vector<LaunchClass> classes;
+        std::vector<int32_t> list;
+        std::vector<LaunchShape> shapes;
+        int rc = make_classes(b, &classes, &list);
+        if (rc != HBG_OK)
+            return rc;
+        plan_bytes(b, classes, db, *opt, db->device, &shapes);
+        rc = plan_launches(b, classes, db, *opt, db->device, &shapes);
+        if (rc != HBG_OK)
+            return rc;
+        if (cap == 0)
+            cap = default_capacity(db, b);
+        *bytes = (int64_t)(L.total + L.scratch()) + cap * (int64_t)(2 * sizeof(hbg_hsp) + 2 * sizeof(uint64_t) + 2 * sizeof(uint32_t)) +
+                 256 * hbg::kOrderMaxGrid * (int64_t)sizeof(uint32_t) + (int64_t)counters_need(b->host) * 8 +
+                 kMaxLaunchClasses * 4 + gdiag_need(b->host, db, shapes) * 4 + side_need(classes, shapes) * 2;
+        return (int)HBG_OK;
+    });
+}
 
 extern "C" {
 
@@ -1820,11 +1883,12 @@ int hbg_batch_info(const hbg_batch *b, int32_t *nq, int32_t *ng, int64_t *qlen, 
     if (!entries && !device_bytes)
         return HBG_OK;
     return guarded([&] {
-        const int64_t n = batch_entries(b);
+        hbg_batch *m = const_cast<hbg_batch *>(b);
+        std::lock_guard<std::mutex> lock(m->tables_mu);
         if (entries)
-            *entries = n;
+            *entries = hbg::count_entries(&m->host);
         if (device_bytes)
-            *device_bytes = batch_device_bytes(b->host, n);
+            *device_bytes = (int64_t)lay_out(m).total;
         return HBG_OK;
     });
 }
@@ -1832,25 +1896,9 @@ int hbg_batch_info(const hbg_batch *b, int32_t *nq, int32_t *ng, int64_t *qlen, 
 int hbg_mem_required(const hbg_db *db, const hbg_batch *b, int64_t cap, int64_t *bytes) {
     if (!db || !b || !bytes || cap < 0)
         return fail(HBG_ERR_INVALID, "hbg_mem_required: bad argument");
-    if (cap == 0)
-        cap = default_capacity(db, b);
-    const hbg::HostBatch &h = b->host;
-    int64_t batch_bytes = 0;
-    const int rc = guarded([&] {
-        batch_bytes = batch_device_bytes(h, batch_entries(b));
-        return HBG_OK;
-    });
-    if (rc != HBG_OK)
-        return rc;
-    int64_t per_hsp = 2 * (int64_t)sizeof(hbg_hsp) + 2 * 8 + 2 * 4;
-    int64_t gdiag = 0;
-    if (global_diag_len(h, db) > 0) {
-        int sms = 152;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db->device);
-        gdiag = (int64_t)sms * 8 * 8 * global_diag_len(h, db) * 4;
-    }
-    *bytes = batch_bytes + cap * per_hsp + gdiag + 1024 * 1024;
-    return HBG_OK;
+    hbg_gpu_options o;
+    hbg_default_gpu_options(&o);
+    return hbg::search_bytes(db, b, &o, cap, bytes);
 }
 
 int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t cap,
@@ -1900,8 +1948,8 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
             delete r;
         return fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
     }
-    plan_bytes(batch, db, o, db->device, &r->shapes);
-    rc = plan_launches(batch, db, o, db->device, &r->shapes);
+    plan_bytes(batch, batch->classes, db, o, db->device, &r->shapes);
+    rc = plan_launches(batch, batch->classes, db, o, db->device, &r->shapes);
     if (rc != HBG_OK) {
         if (!*out)
             delete r;
@@ -2184,8 +2232,8 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     CU(hbg::wordfinder_configure());
     CU(hbg::byte_configure());
     std::vector<LaunchShape> shapes;   // host-side only; no device allocation
-    plan_bytes(batch, db, o, db->device, &shapes);
-    rc = plan_launches(batch, db, o, db->device, &shapes);
+    plan_bytes(batch, batch->classes, db, o, db->device, &shapes);
+    rc = plan_launches(batch, batch->classes, db, o, db->device, &shapes);
     if (rc != HBG_OK)
         return rc;
     cudaStream_t st = (cudaStream_t)stream;

@@ -113,22 +113,21 @@ struct TableSegment {             // letters of one query, up to kTableSegment w
 };
 constexpr int kTableSegment = 512;
 struct TableArgs {
-    HbgGroup *groups;             // entry_base is written
+    const HbgGroup *groups;
     const TableSegment *segs;     // in query order; a group's are seg_base ..
+    int32_t first_group, first_seg;   // of the groups and segments built by this launch
     const uint8_t *letters;
     const int32_t *ctx_of;
     int32_t threshold;
     uint32_t *cells;
     uint32_t *packed;
     uint32_t *pv;
-    uint16_t *entries;
-    int64_t entries_cap;          // a group whose entries would pass it is not filled
+    uint16_t *entries;            // a group's start at its entry_base
     uint16_t *query_cells;
     uint2 *stats;                 // per group: entries, fullest cell
-    uint32_t *counts;             // scratch: HBG_NUM_CELLS per segment
+    uint32_t *counts;             // scratch: HBG_NUM_CELLS per segment of the launch
 };
-bool tables_fit(int64_t n_segs);
-cudaError_t launch_tables(const TableArgs &a, int32_t n_groups, int32_t n_segs, bool fill_only, cudaStream_t stream);
+cudaError_t launch_tables(const TableArgs &a, int32_t n_groups, int32_t n_segs, cudaStream_t stream);
 cudaError_t launch_pack_cells(const uint32_t *cells, int32_t n_groups, uint32_t *packed, cudaStream_t stream);
 
 // Ordering pass: sort HSPs by (query, subject, subject offset, query offset),
@@ -167,6 +166,10 @@ cudaError_t launch_spread_letters(const uint8_t *raw, int64_t from, int64_t coun
 // non-sentinel and form word w.
 cudaError_t launch_db_histogram(const uint8_t *db, int64_t n, unsigned long long *hist,
                                 cudaStream_t stream);
+
+// Device bytes that one search of the batch with these options takes besides the
+// database (cap 0: default capacity).  In api.cu; for the server.
+int search_bytes(const hbg_db *db, const hbg_batch *b, const hbg_gpu_options *opt, int64_t cap, int64_t *bytes);
 
 }  // namespace hbg
 

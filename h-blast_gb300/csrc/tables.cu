@@ -37,7 +37,7 @@ walk_rows(TableArgs a) {
     __shared__ int8_t m[28 * 32];
     __shared__ int8_t most[32];                   // best score of each letter against any
     const int lane = threadIdx.x & 31;
-    const TableSegment S = a.segs[blockIdx.y];
+    const TableSegment S = a.segs[a.first_seg + blockIdx.y];
     const int g = S.group;
     for (int i = threadIdx.x; i < 28 * 32; i += blockDim.x)
         m[i] = c_blosum[i];
@@ -52,19 +52,6 @@ walk_rows(TableArgs a) {
     const HbgGroup &G = a.groups[g];
     const uint8_t *gs = a.letters + G.seq_base;
     const int32_t *gc = a.ctx_of + G.seq_base;
-    long long base = 0;
-    if (Fill) {
-        // entries of the groups before this one
-        for (int k = lane; k < g; k += 32)
-            base += a.stats[k].x;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            base += __shfl_xor_sync(kAll, base, o);
-        if (blockIdx.x == 0 && threadIdx.x == 0 && (int)blockIdx.y == G.seg_base)
-            a.groups[g].entry_base = base;
-        if (base + (long long)a.stats[g].x > a.entries_cap)
-            return;                               // the caller makes room and fills again
-    }
     const int r = blockIdx.x * kRowsPerCta + (threadIdx.x >> 5);
     if (r >= kLetters * kLetters)
         return;
@@ -72,7 +59,7 @@ walk_rows(TableArgs a) {
     const int row = x * 32 + y;
     uint32_t *const counts = a.counts + (size_t)blockIdx.y * HBG_NUM_CELLS + row * 32 + lane;
     uint32_t n = Fill ? a.cells[(size_t)g * HBG_CELL_STRIDE + row * 32 + lane] + *counts : 0u;
-    uint16_t *const ents = a.entries + base;
+    uint16_t *const ents = a.entries + G.entry_base;
     for (int p0 = S.begin; p0 < S.end; p0 += 32) {
         const int p = p0 + lane;
         int t = 0, c = 0;
@@ -100,7 +87,8 @@ walk_rows(TableArgs a) {
 // Per word of a group: a segment's count becomes the count of those before it,
 // and the sums are the word's count per query and (in packed) in the group.
 __global__ void __launch_bounds__(256) sum_segments(TableArgs a) {
-    const HbgGroup &G = a.groups[blockIdx.y];
+    const int g = a.first_group + blockIdx.y;
+    const HbgGroup &G = a.groups[g];
     const int w = blockIdx.x * 256 + threadIdx.x;
     uint32_t n = 0;
     const bool used = (w >> 10) < kLetters && ((w >> 5) & 31) < kLetters;
@@ -108,7 +96,7 @@ __global__ void __launch_bounds__(256) sum_segments(TableArgs a) {
         const int q = a.segs[G.seg_base + k].query;
         uint32_t first = n;
         for (;; ++k) {
-            uint32_t *const c = a.counts + (size_t)(G.seg_base + k) * HBG_NUM_CELLS + w;
+            uint32_t *const c = a.counts + (size_t)(G.seg_base - a.first_seg + k) * HBG_NUM_CELLS + w;
             const uint32_t here = used ? *c : 0u;
             *c = n;
             n += here;
@@ -117,7 +105,7 @@ __global__ void __launch_bounds__(256) sum_segments(TableArgs a) {
         }
         a.query_cells[(size_t)q * HBG_NUM_CELLS + w] = (uint16_t)(n - first);
     }
-    a.packed[(size_t)blockIdx.y * HBG_NUM_CELLS + w] = n;
+    a.packed[(size_t)g * HBG_NUM_CELLS + w] = n;
 }
 
 // One CTA per group: cells, presence vector, packed cells (from the words'
@@ -125,7 +113,7 @@ __global__ void __launch_bounds__(256) sum_segments(TableArgs a) {
 // group.  Thread t has row t.
 __global__ void __launch_bounds__(1024) scan_rows(TableArgs a) {
     __shared__ uint32_t sums[32], tops[32];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = blockIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = a.first_group + blockIdx.x;
     uint32_t *const pk = a.packed + (size_t)g * HBG_NUM_CELLS + t * 32;
     uint32_t total = 0, top = 0, bits = 0;
 #pragma unroll 8
@@ -175,27 +163,21 @@ pack_cells(const uint32_t *cells, uint32_t *packed) {
     packed[(size_t)blockIdx.y * HBG_NUM_CELLS + w] = cs[w] | ((cs[w + 1] - cs[w]) << 22);
 }
 
-// The grid's second dimension is limited; groups are taken 32768 at a time.
-constexpr int kMaxGroups = 32768;
-
 }  // namespace
 
-bool tables_fit(int64_t n_segs) { return n_segs <= kMaxGroups; }
-
-cudaError_t launch_tables(const TableArgs &a, int32_t n_groups, int32_t n_segs, bool fill_only, cudaStream_t stream) {
+cudaError_t launch_tables(const TableArgs &a, int32_t n_groups, int32_t n_segs, cudaStream_t stream) {
     const dim3 grid(kCtas, (unsigned)n_segs);
-    if (!fill_only) {
-        walk_rows<false><<<grid, kRowsPerCta * 32, 0, stream>>>(a);
-        sum_segments<<<dim3(HBG_NUM_CELLS / 256, n_groups), 256, 0, stream>>>(a);
-        scan_rows<<<n_groups, 1024, 0, stream>>>(a);
-    }
+    walk_rows<false><<<grid, kRowsPerCta * 32, 0, stream>>>(a);
+    sum_segments<<<dim3(HBG_NUM_CELLS / 256, n_groups), 256, 0, stream>>>(a);
+    scan_rows<<<n_groups, 1024, 0, stream>>>(a);
     walk_rows<true><<<grid, kRowsPerCta * 32, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_pack_cells(const uint32_t *cells, int32_t n_groups, uint32_t *packed, cudaStream_t stream) {
-    for (int32_t g0 = 0; g0 < n_groups; g0 += kMaxGroups) {
-        const int32_t n = n_groups - g0 < kMaxGroups ? n_groups - g0 : kMaxGroups;
+    constexpr int kMost = 32768;                  // the grid's second dimension is limited
+    for (int32_t g0 = 0; g0 < n_groups; g0 += kMost) {
+        const int32_t n = n_groups - g0 < kMost ? n_groups - g0 : kMost;
         pack_cells<<<dim3(HBG_NUM_CELLS / 256, n), 256, 0, stream>>>(cells + (size_t)g0 * HBG_CELL_STRIDE,
                                                                      packed + (size_t)g0 * HBG_NUM_CELLS);
     }

@@ -17,8 +17,8 @@
 // result equals a search of it alone.
 //
 // Memory: requests are chosen by an estimate of their device bytes; once the
-// batch is built its exact need (hbg_mem_required: lookup tables, HSP and
-// sort buffers, diagonal scratch) is checked against the budget left by the
+// batch is built its exact need (as hbg_mem_required has it: lookup tables and
+// the scratch to build them, HSP and sort buffers, diagonal scratch) is checked against the budget left by the
 // batches in flight and against the device's free memory.  A batch that does
 // not fit -- or whose search fails with HBG_ERR_NOMEM -- goes back to the
 // front of the queue and is retried with half as many requests; a lone
@@ -42,6 +42,7 @@
 #include <vector>
 
 #include "../../include/hblast_gpu.h"
+#include "../csrc/kernels.h"
 #include "batch_builder.h"
 
 namespace {
@@ -106,9 +107,10 @@ int64_t estimate_hsps(int64_t qlen, int64_t db_res) {
 
 int64_t estimate_bytes(int64_t qlen, int64_t db_res) {
     // lookup entries (~20 per letter, 2 B), letters + contexts (5 B), the
-    // query's cell counts (64 KiB), its share of group cells (132 KiB per
-    // 2000 letters), and HSP buffers (raw + ordered + sort keys, ~100 B each)
-    return 65536 + qlen * (40 + 5 + 70) + estimate_hsps(qlen, db_res) * 100;
+    // query's cell counts (64 KiB) and the scratch to build them (128 KiB per
+    // 512 letters), its share of group cells (260 KiB per 4056 letters), and HSP
+    // buffers (raw + ordered + sort keys, 96 B each)
+    return 65536 + 131072 * (qlen / 512 + 1) + qlen * (40 + 5 + 66) + estimate_hsps(qlen, db_res) * 96;
 }
 
 // Device memory left free beside a new batch (the runtime, other streams).
@@ -235,7 +237,7 @@ void launch_slot(hbg_server *S, Slot &sl, std::vector<int64_t> ids, int64_t est,
     int64_t need = 0;
     size_t free_b = 0, total_b = 0;
     if (rc == HBG_OK)
-        rc = hbg_mem_required(S->db, sl.batch, cap, &need);
+        rc = hbg::search_bytes(S->db, sl.batch, &S->opt, cap, &need);
     if (rc == HBG_OK && cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
         cudaGetLastError();
         free_b = (size_t)INT64_MAX;        // unknown: rely on the budget and on allocation failures

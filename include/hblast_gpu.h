@@ -300,14 +300,16 @@ int hbg_batch_tune(hbg_batch *batch, int32_t tile_subjects, int32_t global_table
 int hbg_batch_schedule(hbg_batch *batch, int32_t warps_per_subject, int64_t tile_bytes);
 
 int hbg_batch_destroy(hbg_batch *batch);
-/* Sizes of a batch; device_bytes is what its letters and
- * lookup tables take on the device. */
+/* Sizes of a batch; device_bytes is the device block that holds its letters and
+ * lookup tables. */
 int hbg_batch_info(const hbg_batch *batch, int32_t *n_queries, int32_t *n_groups,
                    int64_t *total_query_len, int64_t *lookup_entries, int64_t *device_bytes);
 
-/* Estimate of the device bytes one search of batch against db needs beyond
- * the resident database (replaces H_BLAST_check_memory, h_blast.cu:1280-1349).
- * hsp_capacity 0 = default sizing. */
+/* Device bytes one search of batch against db allocates beyond the resident
+ * database, with the default options: the batch's block and the scratch its
+ * table build gives back (up to 64 MiB), HSP buffers, diagonal scratch
+ * (replaces H_BLAST_check_memory, h_blast.cu:1280-1349).  hsp_capacity 0 =
+ * default sizing; a search that finds more HSPs than that allocates again. */
 int hbg_mem_required(const hbg_db *db, const hbg_batch *batch, int64_t hsp_capacity,
                      int64_t *bytes);
 

@@ -1,0 +1,50 @@
+"""Device memory of a search: hbg_mem_required against what the device hands out,
+in a process of its own so that no buffer of an earlier search is used again."""
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = Path(__file__).resolve().parent.parent
+
+_SEARCH = """
+import sys
+sys.path[:0] = {paths!r}
+import ctypes as C
+import numpy as np, torch, hblast
+from hblast import synth
+n, qlen, extra = {args!r}
+rng = np.random.default_rng(n)
+db = synth.make_db(rng, 1000, 300, 0.6, 30, 5000, 0, [synth.random_letters(rng, 300)], 100, 0.5)
+res, off = db.residues, db.offsets
+if extra:
+    res, off = np.concatenate([res, synth.random_letters(rng, extra)]), np.append(off, off[-1] + extra)
+gdb = hblast.Database(res, off)
+batch = hblast.Batch.proteins([hblast.ProteinQuery.blastp(synth.random_letters(rng, qlen)) for _ in range(n)])
+need = C.c_int64()
+assert hblast.lib().hbg_mem_required(gdb.handle, batch.handle, 1 << 20, C.byref(need)) == 0
+torch.cuda.synchronize()
+before = torch.cuda.mem_get_info()[0]
+s = hblast.Searcher(gdb, batch, hsp_capacity=1 << 20)
+s.launch()
+s.sync()
+print(need.value, before - torch.cuda.mem_get_info()[0], batch.info()["device_bytes"])
+"""
+
+
+@pytest.mark.parametrize("n,qlen,extra", [(1, 300, 0), (4000, 60, 0), (64, 1500, 0), (1, 20000, 0), (1, 65000, 0),
+                                          (1, 300, 40000), (1, 20000, 70000)])
+def test_memory_required_is_what_a_search_takes(built, n, qlen, extra):
+    """The device gives memory in blocks of 2 MiB, a dozen of them here, and the
+    kernels' code may be loaded at their first launch: 64 MiB of room either way."""
+    code = _SEARCH.format(paths=[str(ROOT / "h-blast_gb300"), str(ROOT)], args=(n, qlen, extra))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    need, taken, batch = map(int, r.stdout.split())
+    room = 64 << 20
+    assert batch <= need
+    assert taken <= need + room, (need, taken)
+    assert need <= taken + room, (need, taken)
