@@ -184,6 +184,7 @@ struct LaunchClass {
     int count;
     int cell;        // bytes of a diagonal cell in byte_kernel (0: these groups cannot use it)
     int table_len;   // its cells per warp
+    bool wide;       // its groups may have cells of kByteWide entries or more
 };
 struct LaunchShape {
     int threads;
@@ -310,6 +311,33 @@ struct hbg_db {
     int64_t bytes = 0;
 };
 
+// The device's build of a batch's tables: it runs on the stream of the batch's
+// first search, which therefore waits for nothing on the host; searches on other
+// streams wait for `done`.  Its scratch goes back when a search that came after
+// it has ended, or with the batch.
+struct TableBuild {
+    explicit TableBuild(int dev) : device(dev) {}
+    ~TableBuild() {
+        if (done) {
+            DeviceScope ds(device);
+            cudaEventDestroy(done);
+        }
+    }
+    void ended() {
+        DeviceScope ds(device);
+        std::lock_guard<std::mutex> lock(mu);
+        dfree_idle(d_counts);
+        over = true;
+    }
+    const int device;
+    cudaEvent_t done = nullptr;
+    uint32_t *d_counts = nullptr;
+    std::atomic<bool> over{false};
+
+  private:
+    std::mutex mu;
+};
+
 struct hbg_batch {
     uint64_t id = g_next_object_id++;
     hbg::HostBatch host;
@@ -326,8 +354,7 @@ struct hbg_batch {
     uint16_t *d_qcells = nullptr;
     int32_t *d_group_list = nullptr;   // groups ordered by launch class
     uint32_t *d_packed = nullptr;      // cells of byte_kernel
-    uint2 *d_stats = nullptr;          // per group: entries, fullest cell
-    uint32_t *d_counts = nullptr;      // scratch of the table build
+    std::shared_ptr<TableBuild> build; // running, or done
     std::vector<LaunchClass> classes;
     std::mutex tables_mu;              // host tables and entry counts are made when first asked for
     bool caller_tables = false;        // the tables are the caller's (in `host`)
@@ -351,7 +378,8 @@ struct hbg_result {
     // device
     hbg_hsp *d_raw = nullptr, *d_sorted = nullptr;
     unsigned long long *d_counters = nullptr;  // [0]=hsp count, then per query ext, kept, hits; per group
-                                               // hits; per query first, end of its HSPs, subjects passed
+                                               // hits; per query first, end of its HSPs, subjects passed; per
+                                               // group subjects taken; the ordering's barrier and error
     unsigned int *d_tile = nullptr;
     uint32_t *d_gdiag = nullptr;
     int64_t gdiag_entries = 0;
@@ -364,6 +392,7 @@ struct hbg_result {
     int64_t sort_cap = 0;
     // host
     std::shared_ptr<KitPool> kits;
+    std::shared_ptr<TableBuild> build;         // of the batch last searched
     HostKit kit;                               // events, pinned counters
     size_t n_counters = 0;
     std::vector<hbg_query_stats> stats;
@@ -382,10 +411,12 @@ namespace {
 
 void free_batch_device(hbg_batch *b) {
     dfree_idle(b->d_arena);
-    dfree_idle(b->d_counts);
+    if (b->build)
+        b->build->ended();
+    b->build.reset();
 }
 
-int upload_batch_buffers(hbg_batch *b, const hbg_db *db);
+int upload_batch_buffers(hbg_batch *b, const hbg_db *db, cudaStream_t stream);
 
 // Run host code that allocates or starts threads: what it throws must not leave
 // a C entry point.
@@ -405,7 +436,7 @@ struct BatchLayout {
     std::vector<hbg::TableSegment> segs;       // of the table build
     int32_t slice = 0;                         // most of them built at a time
     size_t groups = 0, ctx = 0, queries = 0, letters = 0, ctx_of = 0, list = 0, segments = 0, cells = 0, pv = 0, qcells = 0,
-           entries = 0, packed = 0, stats = 0;
+           entries = 0, packed = 0;
     size_t upload = 0, total = 0;
 
     size_t scratch() const { return (size_t)slice * HBG_NUM_CELLS * sizeof(uint32_t); }
@@ -477,7 +508,6 @@ BatchLayout lay_out(hbg_batch *b) {
     if (!b->caller_tables)
         tables();
     L.packed = place(ng * HBG_NUM_CELLS * sizeof(uint32_t));
-    L.stats = place(ng * sizeof(uint2));
     L.total = at;
     return L;
 }
@@ -492,14 +522,32 @@ void ensure_tables(const hbg_batch *batch) {
 
 // Upload at the first search; a failed upload gives back what it allocated,
 // so the batch can be searched again later.
-int upload_batch(hbg_batch *b, const hbg_db *db) {
+// Searches on `stream` come after the batch's table build.
+int after_build(const hbg_batch *b, cudaStream_t stream) {
+    if (!b->build || b->build->over)
+        return HBG_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(stream, &capture));
+    if (capture == cudaStreamCaptureStatusNone) {
+        CU(cudaStreamWaitEvent(stream, b->build->done, 0));
+    } else {                           // an event from outside the capture: wait here
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        CU(cudaThreadExchangeStreamCaptureMode(&mode));
+        const cudaError_t e = cudaEventSynchronize(b->build->done);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        CU(e);
+    }
+    return HBG_OK;
+}
+
+int upload_batch(hbg_batch *b, const hbg_db *db, cudaStream_t stream) {
     const int device = db->device;
     if (b->device == device)
-        return HBG_OK;
+        return after_build(b, stream);
     if (b->device >= 0)
         return fail(HBG_ERR_STATE, "batch already resident on another device");
     DeviceScope ds(device);
-    const int rc = guarded([&] { return upload_batch_buffers(b, db); });
+    const int rc = guarded([&] { return upload_batch_buffers(b, db, stream); });
     if (rc != HBG_OK) {
         cudaDeviceSynchronize();   // copies already issued may still read the host vectors
         free_batch_device(b);
@@ -520,16 +568,15 @@ constexpr int kByteTable16 = 4096;
 constexpr int kByteMinWarps = 2;
 
 // Bytes of a diagonal cell in byte_kernel for a group, 0 when it cannot take
-// the group: its window, table, cell counts or entry count do not fit, the
-// caller's own table lists an offset twice in a cell (two hits in one place), or
+// the group: its window, table or entry count do not fit, the caller's own table lists an offset twice in a cell (two hits in one place), or
 // the caller chose offset mode or a launch shape of wordfinder_kernel.
 int byte_cell(const hbg_batch *b, int32_t g) {
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
     if ((G.mode & 1) || b->tuned || b->team > 1 || b->tile_bytes > 0)
         return 0;
-    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.max_count > hbg::kByteMaxCount ||
-        G.n_entries >= hbg::kByteMaxEntries || b->repeated_entries)
+    if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.n_entries >= hbg::kByteMaxEntries ||
+        b->repeated_entries)
         return 0;
     return G.diag_len <= kByteTable16 ? 2 : 1;
 }
@@ -552,8 +599,10 @@ int make_classes(const hbg_batch *b, std::vector<LaunchClass> *classes, std::vec
     for (int32_t g = 0; g < (int32_t)h.groups.size(); ++g) {
         const HbgGroup &G = h.groups[g];
         const int size = G.placement ? 64 : std::max<int>(64, G.diag_len);
-        // byte_kernel's table with the cell size in the low bits, longest first
-        keyed.push_back({{G.mode, size, tiles ? 0 : -(4 * std::max<int>(64, G.diag_len) + byte_cell(b, g))}, g});
+        // byte_kernel's table, longest first, with the cell size and whether cells
+        // may be wide in the low bits
+        const int cell = byte_cell(b, g), wide = cell == 2 && G.max_cell >= hbg::kByteWide;
+        keyed.push_back({{G.mode, size, tiles ? 0 : -(8 * std::max<int>(64, G.diag_len) + 4 * wide + cell)}, g});
     }
     std::stable_sort(keyed.begin(), keyed.end(),
                      [](const auto &x, const auto &y) { return x.first < y.first; });
@@ -563,7 +612,8 @@ int make_classes(const hbg_batch *b, std::vector<LaunchClass> *classes, std::vec
         const bool global = h.groups[keyed[i].second].placement != 0;
         if (i == 0 || keyed[i].first != keyed[i - 1].first)
             classes->push_back(LaunchClass{keyed[i].first[0] + (global ? 2 : 0), keyed[i].first[1], (int)i, 0,
-                                             -keyed[i].first[2] & 3, -keyed[i].first[2] / 4});
+                                             -keyed[i].first[2] & 3, -keyed[i].first[2] / 8,
+                                             (-keyed[i].first[2] & 4) != 0});
         LaunchClass &lc = classes->back();
         lc.count++;
         if (lc.cell == 1)              // the longest group's exact table
@@ -576,13 +626,18 @@ int make_classes(const hbg_batch *b, std::vector<LaunchClass> *classes, std::vec
     return HBG_OK;
 }
 
-int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
+// The batch's letters go up on the database's upload stream, behind nothing but
+// other such copies, and the host waits for the copy; the tables are built on the
+// search's stream.  (Built on the upload stream, with the host waiting: 56 ms
+// for a 300-letter query while a batch was searched on another stream, whose
+// CTAs keep their SMs to the end; now 0.07.)
+int upload_batch_buffers(hbg_batch *b, const hbg_db *db, cudaStream_t stream) {
     hbg::HostBatch &h = b->host;
     const size_t ng = h.groups.size();
     std::unique_lock<std::mutex> lock(b->tables_mu);
     const BatchLayout L = lay_out(b);
     std::vector<int32_t> list;
-    int rc = make_classes(b, &b->classes, &list);   // again below if a cell turns out too full
+    const int rc = make_classes(b, &b->classes, &list);
     if (rc != HBG_OK)
         return rc;
     // one copy (ten of their own took 80 us)
@@ -624,18 +679,25 @@ int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
     b->d_qcells = reinterpret_cast<uint16_t *>(b->d_arena + L.qcells);
     b->d_entries = reinterpret_cast<uint16_t *>(b->d_arena + L.entries);
     b->d_packed = reinterpret_cast<uint32_t *>(b->d_arena + L.packed);
-    b->d_stats = reinterpret_cast<uint2 *>(b->d_arena + L.stats);
+    b->build = std::make_shared<TableBuild>(db->device);
+    TableBuild &build = *b->build;
+    CU(cudaEventCreateWithFlags(&build.done, cudaEventDisableTiming));
     if (!b->caller_tables)
-        CU(dalloc(&b->d_counts, L.scratch() / sizeof(uint32_t)));
-    cudaStream_t st = nullptr;
-    CU(db->kits->upload_stream(&st));
-    CU(cudaMemcpyAsync(b->d_arena, stage.get(), L.upload, cudaMemcpyHostToDevice, st));
+        CU(dalloc(&build.d_counts, L.scratch() / sizeof(uint32_t)));
+    cudaStream_t up = nullptr;
+    CU(db->kits->upload_stream(&up));
+    CU(cudaMemcpyAsync(b->d_arena, stage.get(), L.upload, cudaMemcpyHostToDevice, up));
+    CU(cudaStreamSynchronize(up));
+    // a captured build would run with the graph only
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CU(cudaStreamIsCapturing(stream, &capture));
+    cudaStream_t st = capture == cudaStreamCaptureStatusNone ? stream : up;
     if (b->caller_tables) {
         CU(hbg::launch_pack_cells(b->d_cells, (int32_t)ng, b->d_packed, st));
     } else {
         hbg::TableArgs t{b->d_groups, reinterpret_cast<const hbg::TableSegment *>(b->d_arena + L.segments), 0, 0,
                          b->d_letters, b->d_ctx_of, h.threshold, b->d_cells, b->d_packed, b->d_pv, b->d_entries,
-                         b->d_qcells, b->d_stats, b->d_counts};
+                         b->d_qcells, build.d_counts};
         for (int32_t g = 0, n; g < (int32_t)ng;) {
             const int32_t end = slice_end(h, g, &n);
             t.first_group = g;
@@ -643,23 +705,10 @@ int upload_batch_buffers(hbg_batch *b, const hbg_db *db) {
             CU(hbg::launch_tables(t, end - g, n, st));
             g = end;
         }
-        std::vector<uint2> stats(ng);
-        CU(cudaMemcpyAsync(stats.data(), b->d_stats, ng * sizeof(uint2), cudaMemcpyDeviceToHost, st));
-        CU(cudaStreamSynchronize(st));
-        bool again = false;
-        for (size_t g = 0; g < ng; ++g) {
-            h.groups[g].max_count = (int32_t)stats[g].y;
-            again = again || (int32_t)stats[g].y > hbg::kByteMaxCount;
-        }
-        if (again) {
-            rc = make_classes(b, &b->classes, &list);
-            if (rc != HBG_OK)
-                return rc;
-            CU(cudaMemcpyAsync(b->d_group_list, list.data(), list.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-        }
     }
-    CU(cudaStreamSynchronize(st));   // the search may run on any stream
-    dfree_idle(b->d_counts);
+    CU(cudaEventRecord(build.done, st));
+    if (st == up)
+        CU(cudaStreamSynchronize(up));
     b->device = db->device;
     return HBG_OK;
 }
@@ -802,8 +851,10 @@ void free_result_device(hbg_result *r) {
     if (r->graph_exec)
         cudaGraphExecDestroy(r->graph_exec);
     r->graph_exec = nullptr;
-    if (r->launched && !r->synced)
+    if (r->launched && !r->synced) {
         cudaStreamSynchronize(r->stream);    // nothing of this search may still run
+        r->build->ended();
+    }
     dfree_idle(r->d_raw);
     dfree_idle(r->d_sorted);
     dfree_idle(r->d_counters);
@@ -916,6 +967,7 @@ hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass 
     t.group_list = b->d_group_list + lc.first;
     t.n_list = lc.count;
     t.packed = b->d_packed;
+    t.cells = b->d_cells;
     t.entries = b->d_entries;
     t.pv = b->d_pv;
     t.letters = b->d_letters;
@@ -976,7 +1028,7 @@ int launch_finders(const hbg_db *db, const hbg_batch *b, const std::vector<Launc
         t.hsp_cap = a.hsp_cap;
         t.q_extended = a.q_extended;
         t.q_kept = a.q_kept;
-        CU(hbg::launch_byte(t, lc.cell, sh.byte_blocks, sh.byte_threads, st));
+        CU(hbg::launch_byte(t, lc.cell, lc.wide, sh.byte_blocks, sh.byte_threads, st));
         ++*launches;
     }
     auto subjects = [&](size_t c) { return shapes[c].byte_threads > 0 ? shapes[c].n_long : db->n; };
@@ -1746,7 +1798,7 @@ int hbg_batch_create_from_smallbone(const hbg_query *query, const hbg_word_param
                 v.assign(overflow + c.payload.cursor, overflow + c.payload.cursor + c.num_used);
             }
             std::sort(v.begin(), v.end());
-            h.groups[0].max_count = std::max(h.groups[0].max_count, c.num_used);
+            h.groups[0].max_cell = std::max(h.groups[0].max_cell, c.num_used);
             if (std::adjacent_find(v.begin(), v.end()) != v.end())
                 (*out)->repeated_entries = true;
             for (uint16_t x : v)
@@ -1914,7 +1966,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     if (!valid_opts(&o))
         return fail(HBG_ERR_INVALID, "num_threadsx must be a multiple of 32 in 32..256");
     DeviceScope ds(db->device);
-    int rc = upload_batch(batch, db);
+    int rc = upload_batch(batch, db, (cudaStream_t)stream);
     if (rc != HBG_OK)
         return rc;
     hbg_result *r = *out;
@@ -1943,6 +1995,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     }
     r->opt = o;
     r->stream = (cudaStream_t)stream;
+    r->build = batch->build;
     if (hbg::wordfinder_configure() != cudaSuccess || hbg::byte_configure() != cudaSuccess) {
         if (!*out)
             delete r;
@@ -2022,6 +2075,8 @@ int hbg_result_sync(hbg_result *r) {
         }
     }
     r->n_hsps = (int64_t)n;
+    if (!r->build->over)
+        r->build->ended();
     CU(cudaEventElapsedTime(&r->wf_ms, r->kit.ev[0], r->kit.ev[1]));
     CU(cudaEventElapsedTime(&r->ord_ms, r->kit.ev[1], r->kit.ev[2]));
     r->synced = true;
@@ -2114,8 +2169,6 @@ int hbg_result_free(hbg_result *r) {
     if (!r)
         return fail(HBG_ERR_INVALID, "null result");
     DeviceScope ds(r->device);
-    if (r->launched && !r->synced)
-        cudaStreamSynchronize(r->stream);
     free_result_device(r);
     delete r;
     return HBG_OK;
@@ -2237,6 +2290,9 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     if (rc != HBG_OK)
         return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    rc = after_build(batch, st);
+    if (rc != HBG_OK)
+        return rc;
     unsigned char *base = (unsigned char *)scratch;
     unsigned int *tile = (unsigned int *)base;
     unsigned long long *q_ext = (unsigned long long *)(base + 256);

@@ -391,7 +391,7 @@ __device__ __forceinline__ void stage_issue(WarpMem &wm, const uint8_t *s, int S
 }
 
 // Cell of the word at offset s0 + lane, 0 when it is empty: first entry |
-// count << 22.  Blocks up to the chunk's last letter are made resident first:
+// count << 22, counts of kByteWide and more as that.  Blocks up to the chunk's last letter are made resident first:
 // for each newly needed block b, wait for its copy (all but the newest group)
 // and issue b + 2 into the slot of b - 2, which no chunk needs any more.
 // Warp-collective.
@@ -417,11 +417,18 @@ __device__ __forceinline__ uint32_t scan_words(const uint8_t *s, int S, int &nex
     return ((pv[w >> 5] >> (w & 31)) & 1u) ? __ldg(packed + w) : 0u;
 }
 
+// Entries of the word at s when its packed cell says kByteWide or more.
+__device__ __noinline__ uint32_t wide_count(const uint8_t *s, const uint32_t *packed, const ByteArgs &a) {
+    const unsigned w = ((unsigned)s[0] << 10) | ((unsigned)s[1] << 5) | s[2];
+    const uint32_t *cs = a.cells + (size_t)((packed - a.packed) / HBG_NUM_CELLS) * HBG_CELL_STRIDE + w;
+    return __ldg(cs + 1) - __ldg(cs);
+}
+
 // One (group, subject) item: scanned 32 offsets at a time; the subject's hit
 // stream (CPU order) is applied 32 hits at a time across chunk boundaries.  A
 // chunk's last, partial batch waits in lanes 0..carry-1 for the next chunk's
 // first hits.  Warp-collective.
-template <typename Cell>
+template <typename Cell, bool Wide>
 __device__ __forceinline__ void process_item(Item<Cell> &it, const ByteArgs &a, const uint32_t *pv, const uint32_t *packed,
                                              const uint16_t *ents) {
     using K = Cells<Cell>;
@@ -462,7 +469,9 @@ __device__ __forceinline__ void process_item(Item<Cell> &it, const ByteArgs &a, 
         const uint32_t cell = cell_next;
         if (s0 + 32 <= it.S - 3)
             cell_next = scan_words(it.s, it.S, next, wm, pv, packed, s0 + 32);
-        const uint32_t c = cell >> 22;
+        uint32_t c = cell >> 22;
+        if (Wide && c == (uint32_t)kByteWide)
+            c = wide_count(it.s + s0 + lane, packed, a);
         const unsigned nz = __ballot_sync(kAll, c != 0);
         if (nz == 0)
             continue;
@@ -539,7 +548,11 @@ __device__ __forceinline__ int turn(int i, int n) { return i < n ? i : i - n; }
 // different ones) when the counter has run out.  Only then do its warps wait
 // for one another.  Groups that are done are passed a CTA's width at a time:
 // 5000 groups of 60 letters against 50 subjects 0.85 ms, one by one 2.6.
-template <typename Cell>
+//
+// Wide: packed cells may say kByteWide.  The check costs the 16-bit instantiation
+// 3 to 6 % (350 letters against 300,000 subjects 1.30 -> 1.38 ms), the 8-bit one
+// nothing.
+template <typename Cell, bool Wide>
 __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
     using K = Cells<Cell>;
     Head &hd = *reinterpret_cast<Head *>(g_byte_smem);
@@ -634,7 +647,7 @@ __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
             Item<Cell> it{(const uint8_t *)(uintptr_t)__shfl_sync(kAll, (unsigned long long)(uintptr_t)ds, ck), S,
                           __shfl_sync(kAll, dj, ck), tab, mem, len, (unsigned)window - 3u, rel, code, side,
                           a.letters + G.seq_base, a.ctx_of + G.seq_base, G.first_query};
-            process_item(it, a, hd.pv, packed, ents);
+            process_item<Cell, Wide>(it, a, hd.pv, packed, ents);
             top = S + it.rel;
         }
         __syncthreads();
@@ -649,8 +662,9 @@ __global__ void __launch_bounds__(kByteThreads, 1) byte_kernel(ByteArgs a) {
 
 namespace {
 
-const void *byte_kernel_of(int cell_bytes) {
-    return cell_bytes == 1 ? (const void *)byte_kernel<uint8_t> : (const void *)byte_kernel<uint16_t>;
+const void *byte_kernel_of(int cell_bytes, bool wide) {
+    return cell_bytes == 1 ? (const void *)byte_kernel<uint8_t, true>
+                           : wide ? (const void *)byte_kernel<uint16_t, true> : (const void *)byte_kernel<uint16_t, false>;
 }
 
 }  // namespace
@@ -663,7 +677,7 @@ cudaError_t byte_configure() {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    for (const void *k : {byte_kernel_of(1), byte_kernel_of(2)}) {
+    for (const void *k : {byte_kernel_of(1, true), byte_kernel_of(2, false), byte_kernel_of(2, true)}) {
         cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
         if (e != cudaSuccess)
             return e;
@@ -671,10 +685,10 @@ cudaError_t byte_configure() {
     return cudaSuccess;
 }
 
-cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threads, cudaStream_t stream) {
+cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, bool wide, int blocks, int threads, cudaStream_t stream) {
     ByteArgs args = a;
     void *params[] = {&args};
-    return cudaLaunchKernel(byte_kernel_of(cell_bytes), dim3((unsigned)blocks), dim3((unsigned)threads), params,
+    return cudaLaunchKernel(byte_kernel_of(cell_bytes, wide), dim3((unsigned)blocks), dim3((unsigned)threads), params,
                             byte_smem_bytes(cell_bytes, threads, a.table_len), stream);
 }
 

@@ -29,8 +29,8 @@ struct HbgGroup {
     int32_t n_queries;
     int32_t placement;    // 0: diagonal table in shared memory, 1: global scratch
     int32_t mode;         // 0: chunk mode (sparse hits), 1: offset mode (dense hits)
-    int32_t n_entries;    // lookup entries of the group, and of its fullest cell
-    int32_t max_count;
+    int32_t n_entries;    // lookup entries of the group
+    int32_t max_cell;     // no cell has more of them
     int32_t seg_base;     // table build: first of the group's segments in the batch, their number
     int32_t n_segs;
 };

@@ -70,7 +70,7 @@ cudaError_t launch_wordfinder(const WordFinderArgs &a, int mode, int blocks, int
 constexpr int kByteThreads = 768;     // largest CTA
 constexpr int kByteMinWindow = 5;     // smallest and largest two-hit window
 constexpr int kByteMaxWindow = 64;
-constexpr int kByteMaxCount = 1023;   // most entries of a cell
+constexpr int kByteWide = 1023;       // packed cells say no higher count: see the cells
 constexpr int kByteMaxEntries = 1 << 22;   // entries of a group are fewer
 struct ByteArgs {
     const uint8_t *db;
@@ -80,7 +80,8 @@ struct ByteArgs {
     int32_t sub_lo, n_subj;
     const HbgGroup *groups;
     const int32_t *group_list;
-    const uint32_t *packed;       // n_groups x HBG_NUM_CELLS: first entry | count << 22
+    const uint32_t *packed;       // n_groups x HBG_NUM_CELLS: first entry | min(count, kByteWide) << 22
+    const uint32_t *cells;        // n_groups x HBG_CELL_STRIDE
     const uint16_t *entries;
     const uint32_t *pv;
     const uint8_t *letters;
@@ -103,7 +104,8 @@ struct ByteArgs {
 __host__ __device__ constexpr int byte_table_len(int letters) { return (letters + 127) / 128 * 128; }
 size_t byte_smem_bytes(int cell_bytes, int threads, int table_len);
 cudaError_t byte_configure();
-cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, int blocks, int threads, cudaStream_t stream);
+// wide: the groups may have cells of kByteWide entries or more (8-bit cells: always allowed)
+cudaError_t launch_byte(const ByteArgs &a, int cell_bytes, bool wide, int blocks, int threads, cudaStream_t stream);
 
 // The lookup tables of a batch (tables.cu): from letters, contexts and queries
 // to cells, presence vectors, packed cells, entries and per-query cell counts.
@@ -124,7 +126,6 @@ struct TableArgs {
     uint32_t *pv;
     uint16_t *entries;            // a group's start at its entry_base
     uint16_t *query_cells;
-    uint2 *stats;                 // per group: entries, fullest cell
     uint32_t *counts;             // scratch: HBG_NUM_CELLS per segment of the launch
 };
 cudaError_t launch_tables(const TableArgs &a, int32_t n_groups, int32_t n_segs, cudaStream_t stream);

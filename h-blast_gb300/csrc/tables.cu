@@ -108,19 +108,23 @@ __global__ void __launch_bounds__(256) sum_segments(TableArgs a) {
     a.packed[(size_t)g * HBG_NUM_CELLS + w] = n;
 }
 
+// First entry and count of a cell in one word; where the count does not fit,
+// byte_kernel reads the cells.
+__device__ __forceinline__ uint32_t pack(uint32_t first, uint32_t count) {
+    return first | (min(count, (uint32_t)kByteWide) << 22);
+}
+
 // One CTA per group: cells, presence vector, packed cells (from the words'
-// counts in packed), and the number of entries and the fullest cell of the
-// group.  Thread t has row t.
+// counts in packed).  Thread t has row t.
 __global__ void __launch_bounds__(1024) scan_rows(TableArgs a) {
-    __shared__ uint32_t sums[32], tops[32];
+    __shared__ uint32_t sums[32];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, g = a.first_group + blockIdx.x;
     uint32_t *const pk = a.packed + (size_t)g * HBG_NUM_CELLS + t * 32;
-    uint32_t total = 0, top = 0, bits = 0;
+    uint32_t total = 0, bits = 0;
 #pragma unroll 8
     for (int z = 0; z < 32; ++z) {
         const uint32_t c = pk[z];
         total += c;
-        top = max(top, c);
         bits |= c ? 1u << z : 0u;
     }
     uint32_t incl = total;
@@ -130,37 +134,30 @@ __global__ void __launch_bounds__(1024) scan_rows(TableArgs a) {
         if (lane >= o)
             incl += v;
     }
-    top = __reduce_max_sync(kAll, top);
-    if (lane == 31) {
+    if (lane == 31)
         sums[warp] = incl;
-        tops[warp] = top;
-    }
     __syncthreads();
-    const uint32_t all = __reduce_add_sync(kAll, sums[lane]);
     const uint32_t before = __reduce_add_sync(kAll, lane < warp ? sums[lane] : 0u);
-    top = __reduce_max_sync(kAll, tops[lane]);
     uint32_t at = before + incl - total;
     uint32_t *const cs = a.cells + (size_t)g * HBG_CELL_STRIDE + t * 32;
 #pragma unroll 8
     for (int z = 0; z < 32; ++z) {
         const uint32_t c = pk[z];
         cs[z] = at;
-        pk[z] = at | (c << 22);
+        pk[z] = pack(at, c);
         at += c;
     }
     a.pv[(size_t)g * HBG_PV_WORDS + t] = bits;
-    if (t == 1023) {
+    if (t == 1023)
         cs[32] = at;
-        a.stats[g] = make_uint2(all, top);
-    }
 }
 
-// The cells of every group in one word each: first entry | count << 22.
+// The cells of every group in one word each.
 __global__ void __launch_bounds__(256)
 pack_cells(const uint32_t *cells, uint32_t *packed) {
     const uint32_t *cs = cells + (size_t)blockIdx.y * HBG_CELL_STRIDE;
     const int w = blockIdx.x * 256 + threadIdx.x;
-    packed[(size_t)blockIdx.y * HBG_NUM_CELLS + w] = cs[w] | ((cs[w + 1] - cs[w]) << 22);
+    packed[(size_t)blockIdx.y * HBG_NUM_CELLS + w] = pack(cs[w], cs[w + 1] - cs[w]);
 }
 
 }  // namespace

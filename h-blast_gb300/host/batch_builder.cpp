@@ -378,16 +378,30 @@ int64_t count_entries(HostBatch *out) {
         for (HbgGroup &G : b.groups) {
             const uint8_t *gs = b.letters.data() + G.seq_base;
             const int32_t *gc = b.ctx_of.data() + G.seq_base;
-            int64_t n = 0;
+            int64_t n = 0, letters[32] = {0};
             uint32_t word = 0;
             int32_t run = 0, before = -1;              // letters of one context so far
             for (int32_t p = 0; p < G.glen; ++p) {
                 run = gc[p] < 0 ? 0 : (gc[p] == before ? run + 1 : 1);
                 before = gc[p];
+                ++letters[gs[p] & 31];
                 word = ((word << 5) | gs[p]) & (HBG_NUM_CELLS - 1);
                 n += run >= HBG_WORD_SIZE ? count[word] : 0;
             }
             G.n_entries = (int32_t)n;
+            // The scores of a cell's words against it sum to at least threshold
+            // each, and to no more than three times what all letters of the
+            // group score against the best letter, negative scores left out.
+            // (Random proteins: 0.17 entries a letter at threshold 11.)
+            int64_t most = 0;
+            for (int x = 0; x < HBG_ALPHABET; ++x) {
+                int64_t sum = 0;
+                for (int y = 1; y < HBG_ALPHABET; ++y)
+                    sum += letters[y] * std::max<int>(kBlosum62[y * 32 + x], 0);
+                most = std::max(most, sum);
+            }
+            const int64_t words = std::max(0, G.glen - HBG_WORD_SIZE + 1);
+            G.max_cell = (int32_t)(b.threshold > 0 ? std::min(words, 3 * most / b.threshold) : words);
         }
         b.counted = true;
     }
@@ -448,7 +462,7 @@ void build_tables(HostBatch *out) {
         cs[HBG_NUM_CELLS] = acc;
         group_entries[g] = acc;
         G.n_entries = (int32_t)acc;
-        G.max_count = (int32_t)most;
+        G.max_cell = (int32_t)most;
         // expected hits per subject offset on typical proteins: entries of
         // words over the 20 standard letters, each such word taken as
         // equally likely (1 / 8000)

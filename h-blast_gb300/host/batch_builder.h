@@ -52,7 +52,7 @@ struct HostBatch {
     int32_t max_diag_len = 0;            // over groups with global placement
     int32_t smem_diag_len = 64;          // per-warp shared table: max over shared-placed groups
     double mode_hits = 0;                // offset-mode threshold
-    bool counted = false;                // the groups' n_entries are known
+    bool counted = false;                // the groups' n_entries and max_cell are known
 };
 
 // One query already in NCBI concatenated form.
@@ -72,7 +72,8 @@ std::string build_batch(const std::vector<QueryIn> &queries, int32_t threshold,
 
 // The lookup tables of a batch on the host; searches build theirs on the device.
 void build_tables(HostBatch *b);
-// Lookup entries the tables hold, without building them; per group in n_entries.
+// Lookup entries the tables hold, without building them; per group in n_entries,
+// with a bound for its fullest cell in max_cell.
 int64_t count_entries(HostBatch *b);
 
 // Standard-code six-frame translation (frames +1,+2,+3,-1,-2,-3, one sentinel

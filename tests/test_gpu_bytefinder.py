@@ -242,3 +242,26 @@ def test_long_subjects_beside_the_others(built, qlens, lens, own_stream):
             first = got
             check(got, pqs, res, off, threads=16)
         assert np.array_equal(got.hsps, first.hsps) and got.stats == first.stats
+
+
+@pytest.mark.parametrize("own_table", [False, True])
+@pytest.mark.parametrize("qlen", [1024, 1025, 1026, 1800, 4000, 9000])
+def test_cells_of_a_thousand_entries_and_more(built, qlen, own_table):
+    """A packed cell counts to 1022; here 1022, 1023, 1024 and more query offsets
+    share a word, in tables built on the device and in a caller's own."""
+    rng = np.random.default_rng(qlen)
+    q = np.concatenate([np.full(qlen, 11, np.uint8), synth.random_letters(rng, 60)])
+    subs = [np.full(n, 11, np.uint8) for n in (3, 4, 35, 70)]
+    subs += [np.concatenate([synth.random_letters(rng, 50), np.full(n, 11, np.uint8), q[-55:]]) for n in (0, 3, 10, 40)]
+    subs += [synth.random_letters(rng, 300)]
+    off = np.zeros(len(subs) + 1, np.int64)
+    off[1:] = np.cumsum([len(s) for s in subs])
+    res = np.concatenate(subs)
+    pq = hblast.ProteinQuery.blastp(q, 16, 30)
+    gdb = hblast.Database(res, off)
+    if own_table:
+        cs, ents = oracle.lookup_table(oracle.Query.blastp(q, 16, 30), 11)
+        batch = hblast.Batch.from_smallbone(pq, *smallbone_from_csr(cs, ents))
+    else:
+        batch = hblast.Batch.proteins([pq])
+    check(hblast.search(gdb, batch), [pq], res, off)

@@ -1,10 +1,16 @@
-"""Device memory of a search: hbg_mem_required against what the device hands out,
-in a process of its own so that no buffer of an earlier search is used again."""
+"""What a search asks of the device and the host beside its result: its memory,
+hbg_mem_required against what the device hands out (in a process of its own so that
+no buffer of an earlier search is used again), and no waiting for other searches."""
 import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
+
+import hblast
+from hblast import synth
+from test_gpu_parity import check
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +54,33 @@ def test_memory_required_is_what_a_search_takes(built, n, qlen, extra):
     assert batch <= need
     assert taken <= need + room, (need, taken)
     assert need <= taken + room, (need, taken)
+
+
+def test_first_search_of_a_batch_does_not_wait_for_another(built):
+    """While a search of 50 ms and more runs on one stream, a new batch is searched
+    on two others: the launches return while the first search still runs, and the
+    results are right although the batch's tables are built behind it."""
+    import torch
+    qs, db = synth.batched_blastp(seed=7, n_queries=64, n_subjects=200_000)
+    gdb = hblast.Database(db.residues, db.offsets)
+    long = hblast.Searcher(gdb, hblast.Batch.proteins([hblast.ProteinQuery.blastp(q) for q in qs]))
+    first, second, third = (torch.cuda.Stream() for _ in range(3))
+    pqs = [hblast.ProteinQuery.blastp(q[:200]) for q in qs[:2]]
+    want = hblast.search(gdb, hblast.Batch.proteins(pqs), hsp_capacity=1 << 20)      # (and buffers for the next ones)
+    check(want, pqs, db.residues, db.offsets, threads=16)
+    long.launch(first.cuda_stream)
+    long.sync()
+    for _ in range(3):
+        batch = hblast.Batch.proteins(pqs)
+        a, b = (hblast.Searcher(gdb, batch, hsp_capacity=1 << 20) for _ in range(2))
+        long.launch(first.cuda_stream)
+        a.launch(second.cuda_stream)
+        b.launch(third.cuda_stream)
+        assert not first.query()
+        for s in (b, a):
+            s.wait()
+            got = s.result()
+            assert np.array_equal(got.hsps, want.hsps) and got.stats == want.stats
+            s.close()
+        batch.close()
+        long.sync()

@@ -112,3 +112,40 @@ def test_search_static_longest_subject(built):
         got = d_hsps.cpu().numpy().view(HSP_DTYPE)[:len(ref.hsps)]
         got = got[np.lexsort((got["q_off"], got["s_off"], got["subject"], got["query"]))]
         assert d_counts[0] == len(ref.hsps) and np.array_equal(got, ref.hsps)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_search_static_right_behind_the_set_up_search(built, captured):
+    """The set-up search has been launched on another stream and not waited for: its
+    batch's tables may still be in the making, with a call that is captured as well."""
+    import torch
+    rng = np.random.default_rng(34)
+    db, batch = make_batch("blastp", rng)
+    gdb = hblast.Database(db.residues, db.offsets)
+    ref = hblast.search(gdb, batch)
+    nq = batch.info()["n_queries"]
+    d_hsps = torch.zeros(9 * (len(ref.hsps) + 8), dtype=torch.int32, device="cuda")
+    d_counts = torch.zeros(1 + 2 * nq, dtype=torch.int64, device="cuda")
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    assert call_static(gdb, batch, d_hsps, len(ref.hsps) + 8, d_counts, two) == 0     # the array's address
+    torch.cuda.synchronize()
+    for _ in range(3):
+        _, fresh = make_batch("blastp", np.random.default_rng(34))
+        d_hsps.fill_(-1)
+        torch.cuda.synchronize()
+        setup = hblast.Searcher(gdb, fresh)
+        setup.launch(one.cuda_stream)
+        if captured:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=two):
+                assert call_static(gdb, fresh, d_hsps, len(ref.hsps) + 8, d_counts, two) == 0, lib().hbg_last_error()
+            graph.replay()
+        else:
+            assert call_static(gdb, fresh, d_hsps, len(ref.hsps) + 8, d_counts, two) == 0
+        torch.cuda.synchronize()
+        got = d_hsps.cpu().numpy().view(HSP_DTYPE)[:len(ref.hsps)]
+        got = got[np.lexsort((got["q_off"], got["s_off"], got["subject"], got["query"]))]
+        assert d_counts[0] == len(ref.hsps) and np.array_equal(got, ref.hsps)
+        setup.wait()
+        assert np.array_equal(setup.result().hsps, ref.hsps)
+        setup.close()
