@@ -395,6 +395,7 @@ struct hbg_result {
     std::shared_ptr<TableBuild> build;         // of the batch last searched
     HostKit kit;                               // events, pinned counters
     size_t n_counters = 0;
+    size_t nq = 0, ng = 0;                     // queries and groups of the batch, which may go before its result
     std::vector<hbg_query_stats> stats;
     std::vector<int64_t> q_first, q_count;
     int64_t n_hsps = 0;
@@ -1996,6 +1997,8 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     r->opt = o;
     r->stream = (cudaStream_t)stream;
     r->build = batch->build;
+    r->nq = batch->host.queries.size();
+    r->ng = batch->host.groups.size();
     if (hbg::wordfinder_configure() != cudaSuccess || hbg::byte_configure() != cudaSuccess) {
         if (!*out)
             delete r;
@@ -2067,12 +2070,9 @@ int hbg_result_sync(hbg_result *r) {
         if ((int64_t)n > r->cap)
             return fail(HBG_ERR_STATE, "HSP count changed between identical launches");
     }
-    {
-        const size_t nq = r->batch->host.queries.size(), ng = r->batch->host.groups.size();
-        if (r->kit.counters[2 + 6 * nq + 2 * ng]) {   // a result may be launched again
-            r->launched = false;
-            return fail(HBG_ERR_CUDA, "the ordering pass gave up waiting for its own blocks");
-        }
+    if (r->kit.counters[2 + 6 * r->nq + 2 * r->ng]) {   // a result may be launched again
+        r->launched = false;
+        return fail(HBG_ERR_CUDA, "the ordering pass gave up waiting for its own blocks");
     }
     r->n_hsps = (int64_t)n;
     if (!r->build->over)
@@ -2091,7 +2091,7 @@ int hbg_result_wait(hbg_result *r) {
         return HBG_OK;
     // the ordered HSPs stay on the device (read with hbg_result_hsps); the
     // ordering pass left per-query ranges and subject counts beside the counters
-    const size_t nq = r->batch->host.queries.size(), ng = r->batch->host.groups.size();
+    const size_t nq = r->nq, ng = r->ng;
     const unsigned long long *rng = r->kit.counters + 1 + 3 * nq + ng;
     r->stats.assign(nq, hbg_query_stats{0, 0, 0, 0});
     r->q_first.assign(nq, 0);
@@ -2126,7 +2126,7 @@ int hbg_result_counts(const hbg_result *r, int64_t *n_hsps, int32_t *n_queries) 
     if (n_hsps)
         *n_hsps = r->n_hsps;
     if (n_queries)
-        *n_queries = (int32_t)r->batch->host.queries.size();
+        *n_queries = (int32_t)r->nq;
     return HBG_OK;
 }
 

@@ -84,3 +84,23 @@ def test_first_search_of_a_batch_does_not_wait_for_another(built):
             s.close()
         batch.close()
         long.sync()
+
+
+def test_batch_may_go_before_its_result(built):
+    """hbg_batch_destroy waits for the device: a search that it ends is then read
+    without the batch."""
+    rng = np.random.default_rng(3)
+    q = synth.random_letters(rng, 400)
+    db = synth.make_db(rng, 2000, 300, 0.6, 30, 3000, 0.05, [q], 100, 0.6)
+    gdb = hblast.Database(db.residues, db.offsets)
+    pqs = [hblast.ProteinQuery.blastp(q)]
+    s = hblast.Searcher(gdb, hblast.Batch.proteins(pqs))
+    s.launch()
+    s.batch.close()
+    more = [hblast.Batch.proteins(pqs * 50) for _ in range(20)]      # over the freed batch
+    s.sync()
+    assert s.n_hsps() > 0
+    s.wait()
+    check(s.result(), pqs, db.residues, db.offsets)
+    s.close()
+    del more
