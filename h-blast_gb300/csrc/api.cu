@@ -186,13 +186,26 @@ struct LaunchClass {
     int table_len;   // its cells per warp
     bool wide;       // its groups may have cells of kByteWide entries or more
 };
+// byte_kernel's part of a class.
 struct LaunchShape {
-    int threads;
-    int blocks;
-    int team;        // groups per tile (warps that share each subject)
-    int byte_threads;   // CTA and grid of byte_kernel (0: not used)
+    int byte_threads;   // CTA and grid (0: not used)
     int byte_blocks;
-    int n_long;      // subjects left to wordfinder_kernel: the longest n_long
+    int n_long;         // subjects left to wordfinder_kernel: the longest n_long
+};
+// A launch of wordfinder_kernel: groups [first, first + count) of the batch's
+// group list against the longest n_subj subjects.
+struct GeneralLaunch {
+    int mode, smem_diag;
+    int first, count;
+    int32_t n_subj, tile;   // subjects, of them per tile
+    int64_t tiles;
+    int threads, blocks;
+    int team;               // groups per tile (warps that share each subject)
+};
+struct SearchPlan {
+    std::vector<LaunchShape> shapes;   // one per launch class of the batch
+    std::vector<GeneralLaunch> general;
+    bool beside = false;               // both kernels have a part, at the same time
 };
 constexpr int kMaxLaunchClasses = 64;
 
@@ -372,9 +385,8 @@ struct hbg_result {
     cudaStream_t stream = nullptr;
     int device = 0;
     int64_t cap = 0;
-    int blocks = 0, threads = 256;   // the largest grid and CTA over launch classes
-    std::vector<LaunchShape> shapes; // one per launch class of the batch
-    hbg_gpu_options shape_opt{};     // options the shapes were computed for
+    SearchPlan plan;
+    hbg_gpu_options plan_opt{};      // options it was made for
     // device
     hbg_hsp *d_raw = nullptr, *d_sorted = nullptr;
     unsigned long long *d_counters = nullptr;  // [0]=hsp count, then per query ext, kept, hits; per group
@@ -405,7 +417,7 @@ struct hbg_result {
     int64_t launch_count = 0;
     cudaGraphExec_t graph_exec = nullptr;
     uint64_t db_id = 0, batch_id = 0;   // what the buffers were last prepared for
-    long long graph_key[6] = {0, 0, 0, 0, 0, 0};
+    long long graph_key[5] = {0, 0, 0, 0, 0};
 };
 
 namespace {
@@ -567,15 +579,16 @@ constexpr int kByteTable16 = 4096;
 // with wordfinder_kernel: 20,000 letters (10 warps) 3.7 / 8.1, 35,000 (6 warps)
 // 9.9 / 18.0, 50,000 (4) 20.6 / 32.3, 64,900 (3, the longest) 35.2 / 45.4.
 constexpr int kByteMinWarps = 2;
+// Fewest tiles, per CTA of a wave, with which a launch class of wordfinder_kernel
+// is launched by itself: what automatic tiles aim at.
+constexpr int kFewTiles = 8;
 
 // Bytes of a diagonal cell in byte_kernel for a group, 0 when it cannot take
-// the group: its window, table or entry count do not fit, the caller's own table lists an offset twice in a cell (two hits in one place), or
-// the caller chose offset mode or a launch shape of wordfinder_kernel.
+// the group: its window, table or entry count do not fit, or the caller's own
+// table lists an offset twice in a cell (two hits in one place).
 int byte_cell(const hbg_batch *b, int32_t g) {
     const hbg::HostBatch &h = b->host;
     const HbgGroup &G = h.groups[g];
-    if ((G.mode & 1) || b->tuned || b->team > 1 || b->tile_bytes > 0)
-        return 0;
     if (h.window < hbg::kByteMinWindow || h.window > hbg::kByteMaxWindow || G.n_entries >= hbg::kByteMaxEntries ||
         b->repeated_entries)
         return 0;
@@ -589,21 +602,16 @@ int make_classes(const hbg_batch *b, std::vector<LaunchClass> *classes, std::vec
     // launched by table size, so a short query's warps reserve only the
     // shared memory its table needs (the rest is L1 for cells and entries:
     // one 350-aa query vs 10 M subjects 8 % faster than with 2048-entry
-    // tables for every group).  Global-table groups of one length form a class
-    // of their own, all of them one class when the caller chose the tiles: a
-    // class alone then has too few.  Five groups of 2500 to 40,000 letters
-    // against 20,000 subjects, ms, together and apart: tiles of 64 subjects 61 /
-    // 105, of 64 KiB 120 / 233; automatic tiles in offset mode 48 / 27, four
-    // groups to a pass 145 / 75.
+    // tables for every group); groups that byte_kernel can take by its table
+    // and whether their cells may be wide, longest first.  With tiles of the
+    // caller's (not byte_kernel's) all of a size stay in the order they came.
     const bool tiles = b->tile_subjects > 0 || b->tile_bytes > 0;
     std::vector<std::pair<std::array<int, 3>, int32_t>> keyed;
     for (int32_t g = 0; g < (int32_t)h.groups.size(); ++g) {
         const HbgGroup &G = h.groups[g];
         const int size = G.placement ? 64 : std::max<int>(64, G.diag_len);
-        // byte_kernel's table, longest first, with the cell size and whether cells
-        // may be wide in the low bits
         const int cell = byte_cell(b, g), wide = cell == 2 && G.max_cell >= hbg::kByteWide;
-        keyed.push_back({{G.mode, size, tiles ? 0 : -(8 * std::max<int>(64, G.diag_len) + 4 * wide + cell)}, g});
+        keyed.push_back({{G.mode, size, cell && !tiles ? -(8 * std::max<int>(64, G.diag_len) + 4 * wide + cell) : 0}, g});
     }
     std::stable_sort(keyed.begin(), keyed.end(),
                      [](const auto &x, const auto &y) { return x.first < y.first; });
@@ -728,33 +736,31 @@ int32_t global_diag_len(const hbg::HostBatch &h, const hbg_db *db) {
 // up to 128, fewer when the class has too little work to give every CTA about
 // eight tiles (small databases and single queries would otherwise leave most
 // SMs idle).
-int32_t class_tile_subjects(const hbg_batch *b, int32_t n_subj, const hbg_db *db, const LaunchClass &lc, int blocks) {
+int32_t class_tile_subjects(const hbg_batch *b, int32_t n_subj, const hbg_db *db, int count, int blocks) {
     if (b->tile_subjects > 0)
         return b->tile_subjects;
     if (b->tile_bytes > 0) {                  // subjects of the database's mean length
         const int64_t mean = std::max<int64_t>(1, db->n_res / std::max<int32_t>(1, db->n));
         return (int32_t)std::max<int64_t>(1, std::min<int64_t>(1 << 20, b->tile_bytes / mean));
     }
-    const int64_t want = (int64_t)n_subj * lc.count / (8 * (int64_t)std::max(blocks, 1));
+    const int64_t want = (int64_t)n_subj * count / (8 * (int64_t)std::max(blocks, 1));
     return (int32_t)std::max<int64_t>(8, std::min<int64_t>(128, want));
 }
 
 // Which classes byte_kernel takes, with which CTA, and the subjects that stay
 // with wordfinder_kernel: those whose positions do not fit its cells.
 void plan_bytes(const hbg_batch *b, const std::vector<LaunchClass> &classes, const hbg_db *db, const hbg_gpu_options &o,
-                int device, std::vector<LaunchShape> *shapes) {
-    shapes->assign(classes.size(), LaunchShape{32, 1, 1, 0, 0, 0});
+                int optin, int sms, std::vector<LaunchShape> *shapes) {
+    shapes->assign(classes.size(), LaunchShape{0, 0, 0});
     hbg_gpu_options std_opt;
     hbg_default_gpu_options(&std_opt);
-    if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx)
+    if (o.num_blocksx != std_opt.num_blocksx || o.num_threadsx != std_opt.num_threadsx || b->tuned || b->team > 1 ||
+        b->tile_bytes > 0)
         return;                                  // the caller chose a launch shape of wordfinder_kernel
-    int optin = 0, sms = 1;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     for (size_t c = 0; c < classes.size(); ++c) {
         const LaunchClass &lc = classes[c];
         LaunchShape &sh = (*shapes)[c];
-        if (!lc.cell)
+        if (!lc.cell || (lc.mode & 1))
             continue;
         // one CTA per SM, with as many warps as their tables leave room for
         int t = hbg::kByteThreads;
@@ -778,68 +784,105 @@ void plan_bytes(const hbg_batch *b, const std::vector<LaunchClass> &classes, con
     }
 }
 
-// CTA size and grid of each launch class that wordfinder_kernel has a part of: the CTA is halved until its
-// per-warp tables fit the shared-memory carve-out; the grid is one wave at
-// the occupancy that leaves (or the caller's num_blocksx).
-int plan_launches(const hbg_batch *b, const std::vector<LaunchClass> &classes, const hbg_db *db, const hbg_gpu_options &o,
-                  int device, std::vector<LaunchShape> *out) {
-    int optin = 0, sms = 1, beside = 0;
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    for (size_t c = 0; c < classes.size(); ++c) {
-        const LaunchClass &lc = classes[c];
-        LaunchShape &sh = (*out)[c];
-        if (sh.byte_threads > 0 && sh.n_long == 0)
+// CTA size and CTAs per SM of wordfinder_kernel: the CTA is halved until its
+// per-warp tables fit the shared-memory carve-out.
+int general_shape(const hbg_batch *b, const hbg_gpu_options &o, int optin, int mode, int smem_diag, int *threads,
+                  int *per_sm) {
+    // num_threadsx is the largest CTA size: take the size (halving down to 64)
+    // that keeps the most warps resident per SM -- large diagonal tables fill
+    // shared memory, and smaller CTAs pack it better
+    // with several groups per pass (team > 1) the CTA keeps at least one
+    // warp per group
+    int best_warps = -1;
+    *threads = 0;
+    for (int t = o.num_threadsx; t >= 32; t = t > 64 ? ((t / 2) + 31) / 32 * 32 : 0) {
+        const int team = std::min(b->team, t / 32);
+        if (team < b->team && *threads > 0)
+            break;
+        if (hbg::wordfinder_smem_bytes(t, smem_diag, team) > (size_t)optin)
             continue;
-        // num_threadsx is the largest CTA size: per class take the size (halving
-        // down to 64) that keeps the most warps resident per SM -- large diagonal
-        // tables fill shared memory, and smaller CTAs pack it better
-        // with several groups per pass (team > 1) the CTA keeps at least one
-        // warp per group
-        int best_t = 0, best_per = 0, best_warps = -1;
-        for (int t = o.num_threadsx; t >= 32; t = t > 64 ? ((t / 2) + 31) / 32 * 32 : 0) {
-            const int team = std::min(b->team, t / 32);
-            if (team < b->team && best_t > 0)
-                break;
-            if (hbg::wordfinder_smem_bytes(t, lc.smem_diag, team) > (size_t)optin)
-                continue;
-            int per = 0;
-            if (hbg::wordfinder_occupancy(lc.mode, t, lc.smem_diag, team, &per) != cudaSuccess || per < 1)
-                per = 1;
-            if (per * (t / 32) > best_warps) {
-                best_t = t;
-                best_per = per;
-                best_warps = per * (t / 32);
-            }
-            if (o.num_blocksx > 0)
-                break;                 // a fixed grid keeps the caller's CTA size when it fits
+        int per = 0;
+        if (hbg::wordfinder_occupancy(mode, t, smem_diag, team, &per) != cudaSuccess || per < 1)
+            per = 1;
+        if (per * (t / 32) > best_warps) {
+            *threads = t;
+            *per_sm = per;
+            best_warps = per * (t / 32);
         }
-        if (best_t == 0)
-            return fail(HBG_ERR_TOO_LONG, "group diagonal tables exceed shared memory");
-        const int blocks = o.num_blocksx > 0 ? o.num_blocksx : sms * best_per;
-        sh.threads = best_t;
-        sh.blocks = blocks;
-        sh.team = std::min(b->team, best_t / 32);
-        if (sh.byte_threads > 0) {     // a few long subjects: as many CTAs as they make tiles
-            const int32_t tile = class_tile_subjects(b, sh.n_long, db, lc, blocks);
-            sh.blocks = (int)std::min<int64_t>(blocks, (int64_t)((sh.n_long + tile - 1) / tile) * lc.count);
-            beside = std::max(beside, sh.blocks);
+        if (o.num_blocksx > 0)
+            break;                 // a fixed grid keeps the caller's CTA size when it fits
+    }
+    return *threads > 0 ? HBG_OK : fail(HBG_ERR_TOO_LONG, "group diagonal tables exceed shared memory");
+}
+
+// The launches of a search.  Neighbouring classes that wordfinder_kernel does not
+// tell apart share a launch, longest groups first, when one of them alone has too
+// few tiles for its CTAs, or when the CTAs are small (few warps work on the last
+// tiles).  ms, together and apart: three groups of 11,000 to 39,000 letters against
+// 81 subjects, three to a pass, 5.0 / 9.0; 40 groups of 1100 to 4100 letters against
+// 217 subjects, global tables, 1.32 / 2.86; 128 threads, five groups of 2500 to
+// 40,000 letters against 20,000 subjects, 36.9 / 44.2.  With tiles enough: the last
+// in offset mode 48 / 27.
+// The grid is one wave (or the caller's num_blocksx), at most a CTA per tile.
+int plan_search(const hbg_batch *b, const std::vector<LaunchClass> &classes, const hbg_db *db, const hbg_gpu_options &o,
+                SearchPlan *plan) {
+    int optin = 0, sms = 1;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, db->device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db->device);
+    plan_bytes(b, classes, db, o, optin, sms, &plan->shapes);
+    plan->general.clear();
+    hbg_gpu_options std_opt;
+    hbg_default_gpu_options(&std_opt);
+    auto subjects = [&](size_t c) { return plan->shapes[c].byte_threads > 0 ? plan->shapes[c].n_long : db->n; };
+    int most = 0;                      // CTAs that search long subjects beside byte_kernel
+    bool some = false;
+    for (size_t c = 0, e; c < classes.size(); c = e) {
+        GeneralLaunch l{classes[c].mode, classes[c].smem_diag, classes[c].first, 0, subjects(c), 0, 0, 0, 0, 1};
+        for (e = c; e < classes.size() && classes[e].mode == l.mode && classes[e].smem_diag == l.smem_diag &&
+                    subjects(e) == l.n_subj; ++e)
+            l.count += classes[e].count;
+        some = some || plan->shapes[c].byte_threads > 0;
+        if (l.n_subj == 0)
+            continue;
+        int per = 1;
+        const int rc = general_shape(b, o, optin, l.mode, l.smem_diag, &l.threads, &per);
+        if (rc != HBG_OK)
+            return rc;
+        l.team = std::min(b->team, l.threads / 32);
+        const int wave = o.num_blocksx > 0 ? o.num_blocksx : sms * per;
+        auto size = [&](GeneralLaunch *x) {
+            x->tile = class_tile_subjects(b, x->n_subj, db, x->count, wave);
+            x->tiles = (int64_t)((x->n_subj + x->tile - 1) / x->tile) * ((x->count + x->team - 1) / x->team);
+            x->blocks = o.num_blocksx > 0 ? wave : (int)std::min<int64_t>(wave, x->tiles);
+        };
+        bool together = o.num_threadsx < std_opt.num_threadsx;
+        for (size_t k = c; k < e; ++k) {
+            GeneralLaunch x = l;
+            x.count = classes[k].count;
+            size(&x);
+            together = together || x.tiles < kFewTiles * (int64_t)wave;
+        }
+        for (size_t k = c; k < e; ++k) {
+            GeneralLaunch x = l;
+            if (!together) {
+                x.first = classes[k].first;
+                x.count = classes[k].count;
+            }
+            size(&x);
+            if (plan->shapes[c].byte_threads > 0)
+                most = std::max(most, x.blocks);
+            plan->general.push_back(x);
+            if (together)
+                break;
         }
     }
     // the long subjects are searched beside byte_kernel, which leaves SMs for
     // them (its CTAs stay to the end and fill theirs)
-    for (LaunchShape &sh : *out)
+    plan->beside = some && most > 0;
+    for (LaunchShape &sh : plan->shapes)
         if (sh.byte_threads > 0)
-            sh.byte_blocks = std::max(1, sh.byte_blocks - std::min(beside, sms / 8));
+            sh.byte_blocks = std::max(1, sh.byte_blocks - std::min(most, sms / 8));
     return HBG_OK;
-}
-
-// byte_kernel and wordfinder_kernel both have a part of the search.
-bool has_long(const hbg_db *db, const std::vector<LaunchShape> &shapes) {
-    for (const LaunchShape &sh : shapes)
-        if (sh.byte_threads > 0 && sh.n_long > 0 && sh.n_long < db->n)
-            return true;
-    return false;
 }
 
 void drop_graph(hbg_result *r) {
@@ -871,20 +914,18 @@ void free_result_device(hbg_result *r) {
 
 // Entries of the scratch that the launches of a search share: global diagonal
 // tables of wordfinder_kernel, flag ends of byte_kernel.
-int64_t gdiag_need(const hbg::HostBatch &h, const hbg_db *db, const std::vector<LaunchShape> &shapes) {
-    int64_t blocks = 0, threads = 0;
-    for (const LaunchShape &sh : shapes)
-        if (sh.byte_threads == 0 || sh.n_long > 0) {
-            blocks = std::max<int64_t>(blocks, sh.blocks);
-            threads = std::max<int64_t>(threads, sh.threads);
-        }
-    return blocks * (threads / 32) * global_diag_len(h, db);
+int64_t gdiag_need(const hbg::HostBatch &h, const hbg_db *db, const SearchPlan &plan) {
+    int64_t warps = 0;
+    for (const GeneralLaunch &l : plan.general)
+        warps = std::max<int64_t>(warps, (int64_t)l.blocks * (l.threads / 32));
+    return warps * global_diag_len(h, db);
 }
-int64_t side_need(const std::vector<LaunchClass> &classes, const std::vector<LaunchShape> &shapes) {
+int64_t side_need(const std::vector<LaunchClass> &classes, const SearchPlan &plan) {
     int64_t side = 0;
-    for (size_t c = 0; c < shapes.size(); ++c)
-        if (shapes[c].byte_threads > 0 && classes[c].cell == 1)
-            side = std::max<int64_t>(side, (int64_t)shapes[c].byte_blocks * (shapes[c].byte_threads / 32) * classes[c].table_len);
+    for (size_t c = 0; c < classes.size(); ++c)
+        if (plan.shapes[c].byte_threads > 0 && classes[c].cell == 1)
+            side = std::max<int64_t>(side, (int64_t)plan.shapes[c].byte_blocks * (plan.shapes[c].byte_threads / 32) *
+                                               classes[c].table_len);
     return side;
 }
 size_t counters_need(const hbg::HostBatch &h) { return 3 + 6 * h.queries.size() + 2 * h.groups.size(); }
@@ -906,7 +947,7 @@ int prepare_result(hbg_result *r, int64_t cap) {
         r->n_counters = counters_need(h);
     }
     r->gdiag_len = global_diag_len(h, r->db);
-    const int64_t gdiag = gdiag_need(h, r->db, r->shapes), side = side_need(r->batch->classes, r->shapes);
+    const int64_t gdiag = gdiag_need(h, r->db, r->plan), side = side_need(r->batch->classes, r->plan);
     if (gdiag > r->gdiag_entries) {
         drop_graph(r);
         dfree(r->d_gdiag);
@@ -914,7 +955,7 @@ int prepare_result(hbg_result *r, int64_t cap) {
         CU(dalloc(&r->d_gdiag, (size_t)gdiag));
         r->gdiag_entries = gdiag;
     }
-    if (has_long(r->db, r->shapes))
+    if (r->plan.beside)
         CU(KitPool::add_side(&r->kit));
     if (side > r->side_entries) {
         drop_graph(r);
@@ -988,37 +1029,28 @@ hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass 
 }
 
 // The word finder's launches: byte_kernel for each class it takes, then
-// wordfinder_kernel for the rest.  With smaller CTAs than the default the classes
-// that wordfinder_kernel does not tell apart share one launch, longest groups
-// first: few warps work on a class's last tiles.  Threads 128, ms, together and
-// apart: five groups of 2500 to 40,000 letters against 20,000 subjects 36.9 / 44.2,
-// seven of 300 to 20,000 14.3 / 19.9, six of 3000 and three of 6000 9.4 / 10.3.
-// `a` holds scratch and outputs (tile_counter: one counter per class), `next` a
-// subject counter per group, both zeroed.  The caller has run
-// wordfinder_configure and byte_configure (not stream operations).
+// wordfinder_kernel for the rest.  `a` holds scratch and outputs (tile_counter: one
+// counter per launch), `next` a subject counter per group, both zeroed.  The
+// caller has run wordfinder_configure and byte_configure (not stream operations).
 //
 // Subjects too long for byte_kernel's cells are few and one warp walks each, so
 // with `kit` they go on its side stream (without, `next` may be a.g_hits, which
 // byte_kernel must find zeroed: it goes first): one query of 350 letters against
 // 300,000 subjects 1.30 ms, with one subject of 35,000 letters besides 1.60, after
 // the others 2.85; 16 queries of 500 letters against 100,000 4.67, 11.0, 15.8.
-int launch_finders(const hbg_db *db, const hbg_batch *b, const std::vector<LaunchShape> &shapes,
-                   const hbg_gpu_options &opt, hbg::WordFinderArgs a, unsigned long long *next, uint16_t *side,
-                   const HostKit *kit, cudaStream_t st, int *launches) {
-    const bool beside = kit && has_long(db, shapes);
+int launch_finders(const hbg_db *db, const hbg_batch *b, const SearchPlan &plan, hbg::WordFinderArgs a,
+                   unsigned long long *next, uint16_t *side, const HostKit *kit, cudaStream_t st, int *launches) {
+    if (db->n == 0)
+        return HBG_OK;
+    const bool beside = kit && plan.beside;
     cudaStream_t other = beside ? kit->side : st;   // wordfinder_kernel's
     if (beside) {
         CU(cudaEventRecord(kit->fork, st));
         CU(cudaStreamWaitEvent(other, kit->fork, 0));
     }
-    hbg_gpu_options std_opt;
-    hbg_default_gpu_options(&std_opt);
-    const bool together = opt.num_threadsx < std_opt.num_threadsx;
-    unsigned int *const tiles = a.tile_counter;
-    const size_t n = db->n > 0 ? b->classes.size() : 0;
-    for (size_t c = 0; c < n; ++c) {
+    for (size_t c = 0; c < b->classes.size(); ++c) {
         const LaunchClass &lc = b->classes[c];
-        const LaunchShape &sh = shapes[c];
+        const LaunchShape &sh = plan.shapes[c];
         if (sh.byte_threads == 0 || sh.n_long >= db->n)
             continue;
         hbg::ByteArgs t = byte_args(db, b, lc, sh);
@@ -1032,24 +1064,17 @@ int launch_finders(const hbg_db *db, const hbg_batch *b, const std::vector<Launc
         CU(hbg::launch_byte(t, lc.cell, lc.wide, sh.byte_blocks, sh.byte_threads, st));
         ++*launches;
     }
-    auto subjects = [&](size_t c) { return shapes[c].byte_threads > 0 ? shapes[c].n_long : db->n; };
-    for (size_t c = 0, e; c < n; c = e) {
-        LaunchClass lc = b->classes[c];
-        for (e = c + 1; together && e < n && b->classes[e].mode == lc.mode && b->classes[e].smem_diag == lc.smem_diag &&
-                        subjects(e) == subjects(c); ++e)
-            lc.count += b->classes[e].count;
-        a.n_subj = subjects(c);
-        if (a.n_subj == 0)
-            continue;
-        a.tile_subjects = class_tile_subjects(b, a.n_subj, db, lc, shapes[c].blocks);
-        a.tiles_per_group = (a.n_subj + a.tile_subjects - 1) / a.tile_subjects;
-        a.team = shapes[c].team;
-        a.n_list = lc.count;
-        a.group_list = b->d_group_list + lc.first;
-        a.n_tiles = (int64_t)a.tiles_per_group * ((lc.count + a.team - 1) / a.team);
-        a.tile_counter = tiles + c;
-        a.smem_diag = lc.smem_diag;
-        CU(hbg::launch_wordfinder(a, lc.mode, shapes[c].blocks, shapes[c].threads, other));
+    for (const GeneralLaunch &l : plan.general) {
+        a.n_subj = l.n_subj;
+        a.tile_subjects = l.tile;
+        a.tiles_per_group = (l.n_subj + l.tile - 1) / l.tile;
+        a.n_tiles = l.tiles;
+        a.team = l.team;
+        a.n_list = l.count;
+        a.group_list = b->d_group_list + l.first;
+        a.smem_diag = l.smem_diag;
+        CU(hbg::launch_wordfinder(a, l.mode, l.blocks, l.threads, other));
+        ++a.tile_counter;
         ++*launches;
     }
     if (beside) {
@@ -1112,8 +1137,7 @@ int enqueue_search(hbg_result *r) {
         cap_status == cudaStreamCaptureStatusActive ? cudaEventRecordExternal : cudaEventRecordDefault;
     CU(cudaEventRecordWithFlags(r->kit.ev[0], st, ev_flags));
     int wf_launches = 0;
-    const int rc = launch_finders(db, b, r->shapes, r->shape_opt, a, r->d_counters + 1 + 6 * nq + ng, r->d_side, &r->kit, st,
-                                  &wf_launches);
+    const int rc = launch_finders(db, b, r->plan, a, r->d_counters + 1 + 6 * nq + ng, r->d_side, &r->kit, st, &wf_launches);
     if (rc != HBG_OK)
         return rc;
     CU(cudaEventRecordWithFlags(r->kit.ev[1], st, ev_flags));
@@ -1157,10 +1181,9 @@ int enqueue_search(hbg_result *r) {
 // (captured on its second launch) instead of ~30 separate launches.
 int launch_search(hbg_result *r) {
     const bool graphable = r->stream != nullptr && r->launch_count > 0;
-    const long long key[6] = {(long long)r->batch_id, (long long)r->cap,
-                              ((long long)r->shape_opt.num_blocksx << 32) | (unsigned)r->shape_opt.num_threadsx,
-                              r->blocks, (long long)r->gdiag_entries,
-                              (long long)(uintptr_t)r->stream};
+    const long long key[5] = {(long long)r->batch_id, (long long)r->cap,
+                              ((long long)r->plan_opt.num_blocksx << 32) | (unsigned)r->plan_opt.num_threadsx,
+                              (long long)r->gdiag_entries, (long long)(uintptr_t)r->stream};
     if (!graphable) {
         int rc = enqueue_search(r);
         if (rc != HBG_OK)
@@ -1214,19 +1237,18 @@ int hbg::search_bytes(const hbg_db *db, const hbg_batch *batch, const hbg_gpu_op
         const BatchLayout L = lay_out(b);
         std::vector<LaunchClass> classes;
         std::vector<int32_t> list;
-        std::vector<LaunchShape> shapes;
+        SearchPlan plan;
         int rc = make_classes(b, &classes, &list);
         if (rc != HBG_OK)
             return rc;
-        plan_bytes(b, classes, db, *opt, db->device, &shapes);
-        rc = plan_launches(b, classes, db, *opt, db->device, &shapes);
+        rc = plan_search(b, classes, db, *opt, &plan);
         if (rc != HBG_OK)
             return rc;
         if (cap == 0)
             cap = default_capacity(db, b);
         *bytes = (int64_t)(L.total + L.scratch()) + cap * (int64_t)(2 * sizeof(hbg_hsp) + 2 * sizeof(uint64_t) + 2 * sizeof(uint32_t)) +
                  256 * hbg::kOrderMaxGrid * (int64_t)sizeof(uint32_t) + (int64_t)counters_need(b->host) * 8 +
-                 kMaxLaunchClasses * 4 + gdiag_need(b->host, db, shapes) * 4 + side_need(classes, shapes) * 2;
+                 kMaxLaunchClasses * 4 + gdiag_need(b->host, db, plan) * 4 + side_need(classes, plan) * 2;
         return (int)HBG_OK;
     });
 }
@@ -2004,20 +2026,13 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
             delete r;
         return fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
     }
-    plan_bytes(batch, batch->classes, db, o, db->device, &r->shapes);
-    rc = plan_launches(batch, batch->classes, db, o, db->device, &r->shapes);
+    rc = plan_search(batch, batch->classes, db, o, &r->plan);
     if (rc != HBG_OK) {
         if (!*out)
             delete r;
         return rc;
     }
-    r->shape_opt = o;
-    r->blocks = 0;
-    r->threads = 32;
-    for (const LaunchShape &sh : r->shapes) {
-        r->blocks = std::max(r->blocks, sh.blocks);
-        r->threads = std::max(r->threads, sh.threads);
-    }
+    r->plan_opt = o;
     // a default capacity that does not fit the device falls back to the
     // smallest one: a search that finds more HSPs is run again with room for them
     const int64_t least = std::max<int64_t>(1 << 20, (int64_t)db->n);
@@ -2284,9 +2299,8 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
         return rc;
     CU(hbg::wordfinder_configure());
     CU(hbg::byte_configure());
-    std::vector<LaunchShape> shapes;   // host-side only; no device allocation
-    plan_bytes(batch, batch->classes, db, o, db->device, &shapes);
-    rc = plan_launches(batch, batch->classes, db, o, db->device, &shapes);
+    SearchPlan plan;                   // host-side only; no device allocation
+    rc = plan_search(batch, batch->classes, db, o, &plan);
     if (rc != HBG_OK)
         return rc;
     cudaStream_t st = (cudaStream_t)stream;
@@ -2335,7 +2349,7 @@ extern "C" int hbg_search_static(const hbg_db *db, const hbg_batch *batch, const
     // 16-bit cells (longer groups are refused above), so no side table; the
     // group counters serve as subject counters
     int launches = 0;
-    rc = launch_finders(db, batch, shapes, o, a, g_hits, nullptr, nullptr, st, &launches);
+    rc = launch_finders(db, batch, plan, a, g_hits, nullptr, nullptr, st, &launches);
     if (rc != HBG_OK)
         return rc;
     // per-query extension and kept counts follow the HSP count in d_counts
