@@ -259,6 +259,8 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
                 b.contexts.push_back(C);
                 for (int32_t i = 0; i < q.ctx_len[c]; ++i)
                     b.ctx_of[at + q.ctx_off[c] + i] = ci;
+                if (q.ctx_len[c] >= HBG_WORD_SIZE)
+                    b.runs.push_back({g, glen + q.ctx_off[c], q.ctx_len[c]});
             }
             // letters between contexts are sentinels whatever the caller put there
             for (int32_t i = 0; i < q.len; ++i)
@@ -369,26 +371,43 @@ const uint16_t *neighbour_counts(int32_t threshold) {
     return t.data();
 }
 
+// Groups of so few words need no bound for their fullest cell, any count fits a
+// packed cell; nor do those of so many letters: byte_kernel's 8-bit tables, which
+// they have, take any count.
+constexpr int64_t kMaxCellAlways = 1022, kMaxCellNever = 4096;
+
 int64_t count_entries(HostBatch *out) {
     HostBatch &b = *out;
     if (!b.cells.empty())
         return (int64_t)b.entries.size();
     if (!b.counted) {
         const uint16_t *count = neighbour_counts(b.threshold);
-        for (HbgGroup &G : b.groups) {
-            const uint8_t *gs = b.letters.data() + G.seq_base;
-            const int32_t *gc = b.ctx_of.data() + G.seq_base;
-            int64_t n = 0, letters[32] = {0};
-            uint32_t word = 0;
-            int32_t run = 0, before = -1;              // letters of one context so far
-            for (int32_t p = 0; p < G.glen; ++p) {
-                run = gc[p] < 0 ? 0 : (gc[p] == before ? run + 1 : 1);
-                before = gc[p];
-                ++letters[gs[p] & 31];
-                word = ((word << 5) | gs[p]) & (HBG_NUM_CELLS - 1);
-                n += run >= HBG_WORD_SIZE ? count[word] : 0;
+        for (HbgGroup &G : b.groups)
+            G.n_entries = 0;
+        for (const HostBatch::Run &r : b.runs) {
+            const uint8_t *s = b.letters.data() + b.groups[r.group].seq_base + r.at;
+            auto of = [&](uint32_t x, uint32_t y, uint32_t z) { return (uint32_t)count[(x << 10) | (y << 5) | z]; };
+            uint32_t n[4] = {0, 0, 0, 0};          // a run has less than 2^32 entries
+            int32_t p = 0;
+            for (; p + 6 <= r.len; p += 4) {
+                n[0] += of(s[p], s[p + 1], s[p + 2]);
+                n[1] += of(s[p + 1], s[p + 2], s[p + 3]);
+                n[2] += of(s[p + 2], s[p + 3], s[p + 4]);
+                n[3] += of(s[p + 3], s[p + 4], s[p + 5]);
             }
-            G.n_entries = (int32_t)n;
+            for (; p + HBG_WORD_SIZE <= r.len; ++p)
+                n[0] += of(s[p], s[p + 1], s[p + 2]);
+            b.groups[r.group].n_entries += (int32_t)(n[0] + n[1] + n[2] + n[3]);
+        }
+        for (HbgGroup &G : b.groups) {
+            const int64_t words = std::max(0, G.glen - HBG_WORD_SIZE + 1);
+            G.max_cell = (int32_t)words;
+            if (b.threshold <= 0 || words <= kMaxCellAlways || G.glen > kMaxCellNever)
+                continue;
+            const uint8_t *gs = b.letters.data() + G.seq_base;
+            int32_t letters[4][32] = {{0}};            // by place: equal letters in a row would wait for one another
+            for (int32_t p = 0; p < G.glen; ++p)
+                ++letters[p & 3][gs[p] & 31];
             // The scores of a cell's words against it sum to at least threshold
             // each, and to no more than three times what all letters of the
             // group score against the best letter, negative scores left out.
@@ -397,11 +416,11 @@ int64_t count_entries(HostBatch *out) {
             for (int x = 0; x < HBG_ALPHABET; ++x) {
                 int64_t sum = 0;
                 for (int y = 1; y < HBG_ALPHABET; ++y)
-                    sum += letters[y] * std::max<int>(kBlosum62[y * 32 + x], 0);
+                    sum += (int64_t)(letters[0][y] + letters[1][y] + letters[2][y] + letters[3][y]) *
+                           std::max<int>(kBlosum62[y * 32 + x], 0);
                 most = std::max(most, sum);
             }
-            const int64_t words = std::max(0, G.glen - HBG_WORD_SIZE + 1);
-            G.max_cell = (int32_t)(b.threshold > 0 ? std::min(words, 3 * most / b.threshold) : words);
+            G.max_cell = (int32_t)std::min(words, 3 * most / b.threshold);
         }
         b.counted = true;
     }

@@ -41,6 +41,10 @@ struct HostBatch {
     std::vector<HbgGroup> groups;
     std::vector<HbgContext> contexts;
     std::vector<HbgQueryDesc> queries;
+    struct Run {                         // letters of one context
+        int32_t group, at, len;          // offset in the group
+    };
+    std::vector<Run> runs;               // by group, contexts that hold a word
     std::vector<uint8_t> letters;        // all groups, gaps included
     std::vector<int32_t> ctx_of;         // per letter, -1 outside contexts
     // lookup tables: empty until build_tables

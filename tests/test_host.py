@@ -269,10 +269,11 @@ sys.path[:0] = {paths!r}
 import numpy as np, hblast
 from hblast import synth
 q = synth.random_letters(np.random.default_rng(0), 20000)
+hblast.Batch.proteins([hblast.ProteinQuery.blastp(q)], threshold=0).lookup_table(0)   # the neighbour lists
 b = hblast.Batch.proteins([hblast.ProteinQuery.blastp(q)] * 3, threshold=0, max_group_len=1)
-n = b.info()["lookup_entries"]                       # and the library's first allocations
+n = b.info()["lookup_entries"]
 used = resource.getpagesize() * int(open("/proc/self/statm").read().split()[0])
-resource.setrlimit(resource.RLIMIT_AS, (used + (192 << 20), resource.RLIM_INFINITY))
+resource.setrlimit(resource.RLIMIT_AS, (used + n, resource.RLIM_INFINITY))   # half of the entries
 for _ in range(2):
     try:
         b.lookup_table(0)
