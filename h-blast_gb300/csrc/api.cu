@@ -2021,18 +2021,20 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
     r->build = batch->build;
     r->nq = batch->host.queries.size();
     r->ng = batch->host.groups.size();
-    if (hbg::wordfinder_configure() != cudaSuccess || hbg::byte_configure() != cudaSuccess) {
-        if (!*out)
-            delete r;
-        return fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
+    // a repeated search has its plan
+    if (r->launch_count == 0 || memcmp(&r->plan_opt, &o, sizeof(o)) != 0) {
+        if (hbg::wordfinder_configure() != cudaSuccess || hbg::byte_configure() != cudaSuccess)
+            rc = fail(HBG_ERR_CUDA, "cannot configure the word-finder kernel (wrong GPU?)");
+        else
+            rc = plan_search(batch, batch->classes, db, o, &r->plan);
+        if (rc != HBG_OK) {
+            r->launch_count = 0;                 // no plan
+            if (!*out)
+                delete r;
+            return rc;
+        }
+        r->plan_opt = o;
     }
-    rc = plan_search(batch, batch->classes, db, o, &r->plan);
-    if (rc != HBG_OK) {
-        if (!*out)
-            delete r;
-        return rc;
-    }
-    r->plan_opt = o;
     // a default capacity that does not fit the device falls back to the
     // smallest one: a search that finds more HSPs is run again with room for them
     const int64_t least = std::max<int64_t>(1 << 20, (int64_t)db->n);
