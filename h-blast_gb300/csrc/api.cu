@@ -229,7 +229,7 @@ class KitPool {
         if (upload_)
             cudaStreamDestroy(upload_);
     }
-    // A stream for copies that must not wait for the caller's work.
+    // A stream for copies that must not wait for anybody's kernels.
     cudaError_t upload_stream(cudaStream_t *out) {
         std::lock_guard<std::mutex> lock(mu_);
         cudaError_t e = upload_ ? cudaSuccess : cudaStreamCreateWithFlags(&upload_, cudaStreamNonBlocking);

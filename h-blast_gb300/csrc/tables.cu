@@ -10,9 +10,10 @@
 // ascending.  Two such walks (count, fill) with prefix sums between.  Bound by
 // the walks' chains of shuffles and look-ups, so long queries are cut into
 // segments walked side by side (20,000 letters in one: 300 us a walk).
-// From the call to the launched search, upload included: 300 letters 0.15 ms,
-// 20,000 letters 0.30, 64 queries of 50,000 letters 0.53; the host build alone
-// took 0.13, 3.4 and 2.8 ms.
+// From the call to the end of a search of one subject, upload and build
+// included: 300 letters 0.16 ms, 20,000 letters 0.39, 64 queries of 50,000 letters
+// 0.60, of which the caller waits 0.05, 0.07 and 0.14; the host build alone took
+// 0.13, 3.4 and 2.2 ms.
 #include <cuda_runtime.h>
 
 #include "kernels.h"

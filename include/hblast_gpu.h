@@ -93,10 +93,13 @@ typedef struct hbg_word_params {
 /* Mirror of BlastGPUOptions (NF/blast_options.h:503-514), the values of the
  * -gpu, -gpu_threads, -gpu_blocks, -method and -num_threads flags
  * (NF/blast_args.cpp:2705-2778).  num_threadsx is the largest CTA size (a
- * multiple of 32, 32..1024): with num_blocksx 0 (one persistent wave sized
+ * multiple of 32, 32..256): with num_blocksx 0 (one persistent wave sized
  * from the SM count) each launch uses the size, halving down to 64, that
  * keeps the most warps resident (large diagonal tables fill shared memory);
- * with num_blocksx > 0 both are used as given when they fit.  method selects
+ * with num_blocksx > 0 both are used as given when they fit.  Both shape the
+ * general word finder: leave them at their defaults (0 and 256) to let the
+ * library use its faster one, with diagonal tables in shared memory and a
+ * launch shape of its own (most searches 1.3 to 3 times as fast).  method selects
  * the device among the visible ones (0 = first);
  * use_gpu 0 makes hbg_search return HBG_ERR_NO_DEVICE (this library has no
  * CPU path). */
@@ -197,8 +200,8 @@ int hbg_db_open_blastdb(const char *path, const hbg_gpu_options *opt, hbg_db **o
 /* ---- query batches -------------------------------------------------------- */
 
 /* Pack a batch of protein queries; its neighbourhood lookup tables are built on
- * the device by the first search, and on the host when a caller asks to see
- * them (the work NCBI's BlastAaLookupTableNew/BlastAaLookupIndexQuery do
+ * the device, on the stream of the first search and ahead of it, and on the host
+ * when a caller asks to see them (the work NCBI's BlastAaLookupTableNew/BlastAaLookupIndexQuery do
  * before H-BLAST reads the table at h_blast.cu:940-958, with cells sorted as
  * lut_sorting does at h_blast.cu:165-194).  Queries are packed into groups
  * that share one scan of the database; results are identical to searching
@@ -272,11 +275,13 @@ int hbg_batch_lookup_table(const hbg_batch *batch, int32_t g, uint32_t *cells,
  * chunk mode (32 offsets compacted at a time; best for sparse groups), 1 =
  * offset mode (one subject offset at a time, lanes over its cell; best for
  * dense groups).  The builder picks by expected hits per offset; results do
- * not depend on the choice.  Call before the batch's first search. */
+ * not depend on the choice.  Groups in mode 1 are searched by the general word
+ * finder (see hbg_gpu_options).  Call before the batch's first search. */
 int hbg_batch_set_mode(hbg_batch *batch, int32_t g, int32_t mode);
 
 /* Work-unit and table placement knobs for tuning (results do not depend on
- * them).  tile_subjects: subjects per work unit a CTA takes (8..4096; 0 =
+ * them).  They shape the general word finder: a batch with tile_subjects or
+ * global_tables set is searched by it (see hbg_gpu_options).  tile_subjects: subjects per work unit a CTA takes (8..4096; 0 =
  * automatic: 128, fewer when the work is small); with the benchmark's length
  * law a tile of 128 subjects is about 46 KB of subject letters.
  * global_tables 1: every group keeps its diagonal table (32-bit cells) in
@@ -285,7 +290,8 @@ int hbg_batch_set_mode(hbg_batch *batch, int32_t g, int32_t mode);
  * arrays are global, h_blast_kernel.cu:603-630.) */
 int hbg_batch_tune(hbg_batch *batch, int32_t tile_subjects, int32_t global_tables);
 
-/* Scheduling knobs for tuning (results do not depend on them).
+/* Scheduling knobs for tuning (results do not depend on them), of the general
+ * word finder, which then searches the batch (see hbg_gpu_options).
  * warps_per_subject (1..8): how many query groups share each pass over a
  * block of subjects.  1 (default): the warps of a CTA take different subjects
  * of one group.  W > 1: a CTA searches W groups at a time, warp w serving
