@@ -206,6 +206,8 @@ struct SearchPlan {
     std::vector<LaunchShape> shapes;   // one per launch class of the batch
     std::vector<GeneralLaunch> general;
     bool beside = false;               // both kernels have a part, at the same time
+    int lanes = 1;                     // streams that byte_kernel's launches are spread over
+    int sides() const { return lanes - 1 + beside; }
 };
 constexpr int kMaxLaunchClasses = 64;
 
@@ -214,8 +216,11 @@ constexpr int kMaxLaunchClasses = 64;
 // small search, so a database keeps a few for its next searches.
 struct HostKit {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    cudaStream_t side = nullptr;  // for work beside the caller's stream, with the
-    cudaEvent_t fork = nullptr, join = nullptr;   // events around it: made when first needed
+    // for work beside the caller's stream, with the events around it: made when
+    // first needed
+    static constexpr int kSides = 3;
+    cudaStream_t side[kSides] = {nullptr, nullptr, nullptr};
+    cudaEvent_t fork = nullptr, join[kSides] = {nullptr, nullptr, nullptr};
     unsigned long long *counters = nullptr;
     size_t n = 0;                 // counters it has room for
 };
@@ -264,13 +269,23 @@ class KitPool {
         }
         return e;
     }
-    // The kit's side stream and its events.
-    static cudaError_t add_side(HostKit *k) {
-        cudaError_t e = k->side ? cudaSuccess : cudaStreamCreateWithFlags(&k->side, cudaStreamNonBlocking);
-        for (cudaEvent_t *ev : {&k->fork, &k->join})
-            if (e == cudaSuccess && !*ev)
-                e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+    // The kit's first n side streams and their events.
+    static cudaError_t add_sides(HostKit *k, int n) {
+        cudaError_t e = cudaSuccess;
+        for (int i = 0; i < n; ++i) {
+            if (e == cudaSuccess && !k->side[i])
+                e = cudaStreamCreateWithFlags(&k->side[i], cudaStreamNonBlocking);
+            for (cudaEvent_t *ev : {&k->fork, &k->join[i]})
+                if (e == cudaSuccess && !*ev)
+                    e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        }
         return e;
+    }
+    // Nothing on the side streams still runs.
+    static void wait_sides(const HostKit &k) {
+        for (cudaStream_t st : k.side)
+            if (st)
+                cudaStreamSynchronize(st);
     }
     // Give back a kit that no GPU work still uses.
     void give(HostKit &k) {
@@ -291,11 +306,14 @@ class KitPool {
         for (cudaEvent_t &ev : k.ev)
             if (ev)
                 cudaEventDestroy(ev);
-        for (cudaEvent_t ev : {k.fork, k.join})
-            if (ev)
-                cudaEventDestroy(ev);
-        if (k.side)
-            cudaStreamDestroy(k.side);
+        if (k.fork)
+            cudaEventDestroy(k.fork);
+        for (int i = 0; i < HostKit::kSides; ++i) {
+            if (k.join[i])
+                cudaEventDestroy(k.join[i]);
+            if (k.side[i])
+                cudaStreamDestroy(k.side[i]);
+        }
         if (k.counters)
             cudaFreeHost(k.counters);
         k = HostKit();
@@ -879,6 +897,19 @@ int plan_search(const hbg_batch *b, const std::vector<LaunchClass> &classes, con
     // the long subjects are searched beside byte_kernel, which leaves SMs for
     // them (its CTAs stay to the end and fill theirs)
     plan->beside = some && most > 0;
+    // byte_kernel's launches side by side hide the walk of the longest subjects at
+    // the end of one; where a warp's share of a group is more than twice that walk
+    // it is over by then, and a launch is better off with all SMs (14 nucleotide
+    // queries against 175,000 subjects 18.03 ms side by side, 17.79 in turn)
+    int n = 0;
+    bool tails = false;
+    for (size_t c = 0; c < classes.size(); ++c) {
+        const LaunchShape &sh = plan->shapes[c];
+        n += sh.byte_threads > 0;
+        tails = tails || db->n_res * classes[c].count < 2 * (int64_t)sh.byte_blocks * (sh.byte_threads / 32) * db->max_len;
+    }
+    // (one beside wordfinder_kernel's: a second would take the SMs left for it)
+    plan->lanes = tails && !plan->beside ? std::max(1, std::min(n, HostKit::kSides + 1)) : 1;
     for (LaunchShape &sh : plan->shapes)
         if (sh.byte_threads > 0)
             sh.byte_blocks = std::max(1, sh.byte_blocks - std::min(most, sms / 8));
@@ -920,12 +951,13 @@ int64_t gdiag_need(const hbg::HostBatch &h, const hbg_db *db, const SearchPlan &
         warps = std::max<int64_t>(warps, (int64_t)l.blocks * (l.threads / 32));
     return warps * global_diag_len(h, db);
 }
+int64_t side_need(const LaunchClass &lc, const LaunchShape &sh) {
+    return sh.byte_threads > 0 && lc.cell == 1 ? (int64_t)sh.byte_blocks * (sh.byte_threads / 32) * lc.table_len : 0;
+}
 int64_t side_need(const std::vector<LaunchClass> &classes, const SearchPlan &plan) {
     int64_t side = 0;
-    for (size_t c = 0; c < classes.size(); ++c)
-        if (plan.shapes[c].byte_threads > 0 && classes[c].cell == 1)
-            side = std::max<int64_t>(side, (int64_t)plan.shapes[c].byte_blocks * (plan.shapes[c].byte_threads / 32) *
-                                               classes[c].table_len);
+    for (size_t c = 0; c < classes.size(); ++c)    // launches run side by side
+        side += side_need(classes[c], plan.shapes[c]);
     return side;
 }
 size_t counters_need(const hbg::HostBatch &h) { return 3 + 6 * h.queries.size() + 2 * h.groups.size(); }
@@ -955,8 +987,7 @@ int prepare_result(hbg_result *r, int64_t cap) {
         CU(dalloc(&r->d_gdiag, (size_t)gdiag));
         r->gdiag_entries = gdiag;
     }
-    if (r->plan.beside)
-        CU(KitPool::add_side(&r->kit));
+    CU(KitPool::add_sides(&r->kit, r->plan.sides()));
     if (side > r->side_entries) {
         drop_graph(r);
         dfree(r->d_side);
@@ -1033,22 +1064,29 @@ hbg::ByteArgs byte_args(const hbg_db *db, const hbg_batch *b, const LaunchClass 
 // counter per launch), `next` a subject counter per group, both zeroed.  The
 // caller has run wordfinder_configure and byte_configure (not stream operations).
 //
-// Subjects too long for byte_kernel's cells are few and one warp walks each, so
-// with `kit` they go on its side stream (without, `next` may be a.g_hits, which
-// byte_kernel must find zeroed: it goes first): one query of 350 letters against
-// 300,000 subjects 1.30 ms, with one subject of 35,000 letters besides 1.60, after
-// the others 2.85; 16 queries of 500 letters against 100,000 4.67, 11.0, 15.8.
+// With `kit`, launches run side by side on its streams: at the end of one, a few
+// warps walk its last or longest subjects while the next could have the other SMs.
+// (Without, one after another, byte_kernel's first: `next` may be a.g_hits, which
+// it must find zeroed.)  ms, side by side and in turn: groups of 100, 300, 900, 2000
+// and 4000 letters against 20,000 subjects 1.14 / 1.29; three of 5000 to 34,000
+// against 17 subjects and one of 33,000 letters 102 / 202 (175 in one launch of
+// wordfinder_kernel).  Short tables first: where the long ones' CTAs get half of
+// the SMs at first, their last group starts late with its longest subject (100 to
+// 1500 letters in two launches against 200,000 subjects 14.13 / 14.05; 14.06 so).
+// Subjects too long for byte_kernel's cells, a warp each: one query of 350 letters
+// against 300,000 subjects 1.30 ms, with one subject of 35,000 letters besides 1.60,
+// after the others 2.85; 16 queries of 500 letters against 100,000 4.67, 11.0, 15.8.
 int launch_finders(const hbg_db *db, const hbg_batch *b, const SearchPlan &plan, hbg::WordFinderArgs a,
                    unsigned long long *next, uint16_t *side, const HostKit *kit, cudaStream_t st, int *launches) {
     if (db->n == 0)
         return HBG_OK;
-    const bool beside = kit && plan.beside;
-    cudaStream_t other = beside ? kit->side : st;   // wordfinder_kernel's
-    if (beside) {
+    const int sides = kit ? plan.sides() : 0;
+    if (sides > 0)
         CU(cudaEventRecord(kit->fork, st));
-        CU(cudaStreamWaitEvent(other, kit->fork, 0));
-    }
-    for (size_t c = 0; c < b->classes.size(); ++c) {
+    for (int i = 0; i < sides; ++i)
+        CU(cudaStreamWaitEvent(kit->side[i], kit->fork, 0));
+    int lane = 0;                      // of byte_kernel's next launch; 0: st
+    for (size_t c = b->classes.size(); c-- > 0;) {
         const LaunchClass &lc = b->classes[c];
         const LaunchShape &sh = plan.shapes[c];
         if (sh.byte_threads == 0 || sh.n_long >= db->n)
@@ -1056,14 +1094,18 @@ int launch_finders(const hbg_db *db, const hbg_batch *b, const SearchPlan &plan,
         hbg::ByteArgs t = byte_args(db, b, lc, sh);
         t.next = next;
         t.side = side;
+        if (side)
+            side += side_need(lc, sh);
         t.hsps = a.hsps;
         t.hsp_count = a.hsp_count;
         t.hsp_cap = a.hsp_cap;
         t.q_extended = a.q_extended;
         t.q_kept = a.q_kept;
-        CU(hbg::launch_byte(t, lc.cell, lc.wide, sh.byte_blocks, sh.byte_threads, st));
+        CU(hbg::launch_byte(t, lc.cell, lc.wide, sh.byte_blocks, sh.byte_threads, lane == 0 ? st : kit->side[lane - 1]));
+        lane = sides > 0 ? (lane + 1) % plan.lanes : 0;
         ++*launches;
     }
+    cudaStream_t other = kit && plan.beside ? kit->side[sides - 1] : st;   // wordfinder_kernel's, in turn: they share scratch
     for (const GeneralLaunch &l : plan.general) {
         a.n_subj = l.n_subj;
         a.tile_subjects = l.tile;
@@ -1077,9 +1119,9 @@ int launch_finders(const hbg_db *db, const hbg_batch *b, const SearchPlan &plan,
         ++a.tile_counter;
         ++*launches;
     }
-    if (beside) {
-        CU(cudaEventRecord(kit->join, other));
-        CU(cudaStreamWaitEvent(st, kit->join, 0));
+    for (int i = 0; i < sides; ++i) {
+        CU(cudaEventRecord(kit->join[i], kit->side[i]));
+        CU(cudaStreamWaitEvent(st, kit->join[i], 0));
     }
     return HBG_OK;
 }
@@ -2048,8 +2090,7 @@ int hbg_search(hbg_db *db, hbg_batch *batch, const hbg_gpu_options *opt, int64_t
         rc = launch_search(r);
     if (rc != HBG_OK) {
         cudaStreamSynchronize(r->stream);       // a partly enqueued search may still run
-        if (r->kit.side)
-            cudaStreamSynchronize(r->kit.side);
+        KitPool::wait_sides(r->kit);
         if (!*out) {
             free_result_device(r);
             delete r;
@@ -2077,8 +2118,7 @@ int hbg_result_sync(hbg_result *r) {
             rc = launch_search(r);
         if (rc != HBG_OK) {
             cudaStreamSynchronize(r->stream);
-            if (r->kit.side)
-                cudaStreamSynchronize(r->kit.side);
+            KitPool::wait_sides(r->kit);
             r->launched = false;
             return rc;
         }

@@ -264,3 +264,34 @@ def test_cells_of_a_thousand_entries_and_more(built, qlen, own_table):
     else:
         batch = hblast.Batch.proteins([pq])
     check(hblast.search(gdb, batch), [pq], res, off)
+
+
+@pytest.mark.parametrize("lens", [(5000, 9000), (20, 100, 300, 900, 2000, 4000, 5000, 9000, 17000), (4000, 17000, 33000)])
+@pytest.mark.parametrize("own_stream", [False, True])
+def test_launches_side_by_side(built, lens, own_stream):
+    """One launch per table length, side by side on up to four streams, 8-bit ones
+    with flag ends of their own: as the oracle, and the same in every repetition."""
+    import torch
+    rng = np.random.default_rng(len(lens))
+    qs = [synth.random_letters(rng, n) for n in lens]
+    res, off = database(rng, np.concatenate(qs), (5000, 20000))
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 25) for q in qs]
+    s = hblast.Searcher(hblast.Database(res, off), hblast.Batch.proteins(pqs, threshold=10, max_group_len=1))
+    stream = torch.cuda.Stream() if own_stream else None
+    first = None
+    for _ in range(6):
+        s.launch(stream.cuda_stream if stream else None)
+        s.wait()
+        got = s.result()
+        if first is None:
+            assert s.timing()[2] == len(lens) + 1
+            first = got
+            for k, q in enumerate(qs):
+                ref, subj, cnt = oracle.search(oracle.Query.blastp(q, 16, 25), res, off, threshold=10, nthreads=8)
+                mine = got.for_query(k)
+                assert len(mine) == len(ref) and np.array_equal(mine["subject"], subj)
+                for f in ("q_start", "s_start", "q_off", "s_off", "len", "score"):
+                    assert np.array_equal(mine[f], ref[f]), (k, f)
+                st = got.stats[k]
+                assert (st["lookup_hits"], st["init_extends"], st["good_init_extends"]) == tuple(int(c) for c in cnt)
+        assert np.array_equal(got.hsps, first.hsps) and got.stats == first.stats
