@@ -18,6 +18,7 @@
 #include <mutex>
 #include <new>
 #include <numeric>
+#include <shared_mutex>
 #include <string>
 #include <vector>
 
@@ -145,6 +146,22 @@ void dfree_idle(T *&p) {
     if (!keep)
         dfree(p);
     p = nullptr;
+}
+
+// A wait for the whole device is an error while any of its streams is captured,
+// and ends the capture.  So captures of this library hold this mutex shared, and
+// its waits for a device hold it alone; a search that would be captured meanwhile
+// is launched directly.
+std::shared_mutex &capture_mutex() {
+    static std::shared_mutex *m = new std::shared_mutex;   // never destroyed, like the pool
+    return *m;
+}
+cudaError_t wait_device() {
+    std::unique_lock<std::shared_mutex> lock(capture_mutex());
+    const cudaError_t e = cudaDeviceSynchronize();
+    if (e != cudaSuccess)
+        cudaGetLastError();   // must not surface at a later launch check
+    return e;
 }
 
 // Zeros before the first letter of a letter buffer; 64 follow the last:
@@ -441,7 +458,15 @@ struct hbg_result {
 namespace {
 
 void free_batch_device(hbg_batch *b) {
-    dfree_idle(b->d_arena);
+    // searches of this batch may run on any stream: wait for the device (as
+    // cudaFree would), then keep the buffers for reuse
+    if (wait_device() == cudaSuccess) {
+        dfree_idle(b->d_arena);
+    } else {                                   // a caller captures: cudaFree waits by itself
+        dfree(b->d_arena);
+        if (b->build)
+            dfree(b->build->d_counts);
+    }
     if (b->build)
         b->build->ended();
     b->build.reset();
@@ -580,7 +605,6 @@ int upload_batch(hbg_batch *b, const hbg_db *db, cudaStream_t stream) {
     DeviceScope ds(device);
     const int rc = guarded([&] { return upload_batch_buffers(b, db, stream); });
     if (rc != HBG_OK) {
-        cudaDeviceSynchronize();   // copies already issued may still read the host vectors
         free_batch_device(b);
         b->device = -1;
     }
@@ -1226,12 +1250,14 @@ int launch_search(hbg_result *r) {
     const long long key[5] = {(long long)r->batch_id, (long long)r->cap,
                               ((long long)r->plan_opt.num_blocksx << 32) | (unsigned)r->plan_opt.num_threadsx,
                               (long long)r->gdiag_entries, (long long)(uintptr_t)r->stream};
-    if (!graphable) {
+    const bool same_graph = r->graph_exec && memcmp(key, r->graph_key, sizeof(key)) == 0;
+    std::shared_lock<std::shared_mutex> capture(capture_mutex(), std::defer_lock);
+    if (!graphable || (!same_graph && !capture.try_lock())) {
         int rc = enqueue_search(r);
         if (rc != HBG_OK)
             return rc;
     } else {
-        if (!r->graph_exec || memcmp(key, r->graph_key, sizeof(key)) != 0) {
+        if (!same_graph) {
             drop_graph(r);
             cudaGraph_t graph = nullptr;
             CU(cudaStreamBeginCapture(r->stream, cudaStreamCaptureModeThreadLocal));
@@ -1251,6 +1277,7 @@ int launch_search(hbg_result *r) {
                 return fail(HBG_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
             }
             memcpy(r->graph_key, key, sizeof(key));
+            capture.unlock();
         }
         CU(cudaGraphLaunch(r->graph_exec, r->stream));
     }
@@ -1412,7 +1439,7 @@ int db_create(int device, int32_t n, const std::vector<int64_t> &off, const std:
     }
     CUB(cudaMemset(db->d_hist, 0, sizeof(unsigned long long) * HBG_NUM_CELLS));
     CUB(hbg::launch_db_histogram(db->d_letters, letters_len, db->d_hist, 0));
-    CUB(cudaDeviceSynchronize());
+    CUB(wait_device());
 #undef CUB
     db->sched_len.resize(n);
     for (int32_t i = 0; i < n; ++i)
@@ -1535,7 +1562,7 @@ int hbg_db_open(const uint8_t *residues, const int64_t *offsets, int32_t n,
         if (e == cudaSuccess)
             e = cudaMemcpy(&bad, d_bad, sizeof(bad), cudaMemcpyDeviceToHost);
         else
-            cudaDeviceSynchronize();                // nothing may still use the buffers
+            wait_device();                          // nothing may still use the buffers
         dfree_idle(d_raw);
         dfree_idle(d_first);
         dfree_idle(d_bad);
@@ -1974,9 +2001,6 @@ int hbg_batch_destroy(hbg_batch *b) {
         return fail(HBG_ERR_INVALID, "null batch");
     if (b->device >= 0) {
         DeviceScope ds(b->device);
-        // searches of this batch may run on any stream: wait for the device
-        // (as cudaFree would), then keep the buffers for reuse
-        cudaDeviceSynchronize();
         free_batch_device(b);
     }
     delete b;

@@ -104,3 +104,44 @@ def test_batch_may_go_before_its_result(built):
     check(s.result(), pqs, db.residues, db.offsets)
     s.close()
     del more
+
+
+def test_threads_capture_and_destroy(built):
+    """Four threads that launch kept results again, which captures a graph, and
+    destroy batches, which waits for the device: neither disturbs the other."""
+    import threading
+
+    import torch
+    rng = np.random.default_rng(8)
+    qs = [synth.random_letters(rng, n) for n in (60, 300, 900, 2500, 6000)]
+    db = synth.make_db(rng, 2000, 300, 0.6, 30, 3000, 0.05, qs, 50, 0.6)
+    gdb = hblast.Database(db.residues, db.offsets)
+    pqs = [hblast.ProteinQuery.blastp(q, 16, 30) for q in qs]
+    want = {n: hblast.search(gdb, hblast.Batch.proteins(pqs[:n], max_group_len=1)) for n in range(1, 6)}
+    check(want[5], pqs, db.residues, db.offsets, threads=16)
+    faults = []
+
+    def work(k):
+        stream = torch.cuda.Stream()
+        try:
+            for i in range(40):
+                n = 1 + (i + k) % 5
+                batch = hblast.Batch.proteins(pqs[:n], max_group_len=1)
+                s = hblast.Searcher(gdb, batch)
+                for _ in range(3):
+                    s.launch(stream.cuda_stream)
+                    s.wait()
+                    got = s.result()
+                    if not np.array_equal(got.hsps, want[n].hsps) or got.stats != want[n].stats:
+                        faults.append((k, i))
+                s.close()
+                batch.close()
+        except Exception as e:
+            faults.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not faults
