@@ -228,8 +228,8 @@ struct SearchPlan {
 };
 constexpr int kMaxLaunchClasses = 64;
 
-// What a search keeps on the host side beside its device buffers: events and
-// the pinned copy of its counters.  Making and freeing them took 250 us of a
+// What a search keeps on the host side beside its device buffers: events, the
+// pinned copy of its counters, streams for launches side by side.  Making and freeing them took 250 us of a
 // small search, so a database keeps a few for its next searches.
 struct HostKit {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
