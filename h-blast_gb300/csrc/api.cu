@@ -922,16 +922,21 @@ int plan_search(const hbg_batch *b, const std::vector<LaunchClass> &classes, con
     // them (its CTAs stay to the end and fill theirs)
     plan->beside = some && most > 0;
     // byte_kernel's launches side by side hide the walk of the longest subjects at
-    // the end of one; where a warp's share of a group is more than twice that walk
-    // it is over by then, and a launch is better off with all SMs (14 nucleotide
-    // queries against 175,000 subjects 18.03 ms side by side, 17.79 in turn)
+    // the end of one.  Where the warps' shares of all groups together are more than
+    // five such walks they are better off in turn, each with all SMs: 14 nucleotide
+    // queries against 175,000 subjects 18.03 ms side by side, 17.79 in turn (a share
+    // of some 40 walks); 14 proteins in groups of 1000 letters and more against
+    // 22,000 subjects 1.086, 1.049 (eight)
     int n = 0;
-    bool tails = false;
+    double share = 0;                  // letters of a warp
     for (size_t c = 0; c < classes.size(); ++c) {
         const LaunchShape &sh = plan->shapes[c];
-        n += sh.byte_threads > 0;
-        tails = tails || db->n_res * classes[c].count < 2 * (int64_t)sh.byte_blocks * (sh.byte_threads / 32) * db->max_len;
+        if (sh.byte_threads == 0)
+            continue;
+        ++n;
+        share += (double)db->n_res * classes[c].count / (sh.byte_blocks * (sh.byte_threads / 32));
     }
+    const bool tails = share < 5.0 * db->max_len;
     // (one beside wordfinder_kernel's: a second would take the SMs left for it)
     plan->lanes = tails && !plan->beside ? std::max(1, std::min(n, HostKit::kSides + 1)) : 1;
     for (LaunchShape &sh : plan->shapes)
