@@ -90,6 +90,7 @@ struct hbg_server {
     int64_t batches = 0, completed = 0, largest = 0, requeued = 0;
     int32_t admit_cap = 0;   // > 0: the next batch takes at most this many requests
     bool hold = false;       // a lone request waits for a running batch to end
+    Clock::time_point launched;   // the last batch
     bool stop = false;
     std::thread th;
 };
@@ -283,6 +284,7 @@ void launch_slot(hbg_server *S, Slot &sl, std::vector<int64_t> ids, int64_t est,
         return;
     }
     S->batches++;
+    S->launched = Clock::now();
     S->largest = std::max<int64_t>(S->largest, (int64_t)ids.size());
     S->admit_cap = 0;
 }
@@ -355,8 +357,11 @@ void dispatcher(hbg_server *S) {
         }
         if (S->stop && S->pending.empty() && !busy)
             break;
-        // poll running searches often; otherwise sleep until work arrives
-        S->cv_work.wait_for(lk, busy ? std::chrono::microseconds(100) : std::chrono::microseconds(5000));
+        // poll running searches often, most of all those that may end soon (a
+        // batch's tables are built after its launch has returned); otherwise sleep
+        // until work arrives
+        const bool young = Clock::now() - S->launched < std::chrono::milliseconds(1);
+        S->cv_work.wait_for(lk, std::chrono::microseconds(!busy ? 5000 : young ? 10 : 100));
     }
 }
 
