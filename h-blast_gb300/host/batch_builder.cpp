@@ -147,6 +147,23 @@ void parallel_for(int64_t n, const std::function<void(int64_t)> &body) {
         std::rethrow_exception(first);
 }
 
+// Every letter is in 1..27, eight at a time.
+bool letters_valid(const uint8_t *s, int32_t n) {
+    constexpr uint64_t kOnes = 0x0101010101010101ull, kTop = 0x80 * kOnes;
+    uint64_t bad = 0;
+    int32_t i = 0;
+    for (; i + 8 <= n; i += 8) {
+        uint64_t w;
+        memcpy(&w, s + i, 8);
+        // the top bit of a byte: set if it is zero (or follows one that is), 28..127, 128..255
+        bad |= ((w - kOnes) & ~w) | (w + (0x80 - HBG_ALPHABET) * kOnes) | w;
+    }
+    bad &= kTop;
+    for (; i < n; ++i)
+        bad |= s[i] == 0 || s[i] >= HBG_ALPHABET;
+    return bad == 0;
+}
+
 int32_t next_pow2(int32_t v) {
     int32_t n = 1;
     while (n < v)
@@ -185,6 +202,7 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
     std::vector<int32_t> group_of(qs.size());
     int32_t cur_len = 0, cur_n = 0;
     int32_t n_groups = 0;
+    int64_t total = 0;                           // letters of the groups before this one
     for (size_t k = 0; k < qs.size(); ++k) {
         const QueryIn &q = qs[k];
         if (q.len <= 0 || q.len > HBG_MAX_QUERY_LEN)
@@ -201,16 +219,14 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
                 return "query " + std::to_string(k) + ": contexts overlap or are unordered";
             if (q.xdrop[c] < 0)
                 return "query " + std::to_string(k) + ": negative x_dropoff";
-            for (int32_t i = 0; i < q.ctx_len[c]; ++i) {
-                uint8_t r = q.seq[q.ctx_off[c] + i];
-                if (r == 0 || r >= HBG_ALPHABET)
-                    return "query " + std::to_string(k) + ": letter outside NCBIstdaa 1..27";
-            }
+            if (!letters_valid(q.seq + q.ctx_off[c], q.ctx_len[c]))
+                return "query " + std::to_string(k) + ": letter outside NCBIstdaa 1..27";
         }
         int32_t need = (cur_n > 0 ? window : 0) + q.len;
         if (cur_n == 0 || cur_len + need > max_group_len || cur_n >= kMaxQueriesPerGroup) {
             if (cur_n > 0)
                 ++n_groups;
+            total += cur_len;
             cur_len = q.len;
             cur_n = 1;
         } else {
@@ -225,6 +241,8 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
     // --- lay out letters, queries, contexts ---
     b.groups.resize(n_groups);
     b.queries.resize(qs.size());
+    b.letters.reserve((size_t)(total + cur_len));
+    b.ctx_of.reserve((size_t)(total + cur_len));
     int64_t seq_pos = 0;
     for (int32_t g = 0, k = 0; g < n_groups; ++g) {
         HbgGroup &G = b.groups[g];
@@ -246,9 +264,14 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
             Q.len = q.len;
             Q.first_ctx = (int32_t)b.contexts.size();
             Q.n_ctx = (int32_t)q.ctx_off.size();
-            size_t at = b.letters.size();
-            b.letters.insert(b.letters.end(), q.seq, q.seq + q.len);
-            b.ctx_of.insert(b.ctx_of.end(), q.len, -1);
+            // contexts in order; letters between them are sentinels whatever the
+            // caller put there
+            int32_t put = 0;
+            auto gap = [&](int32_t end) {
+                b.letters.insert(b.letters.end(), end - put, 0);
+                b.ctx_of.insert(b.ctx_of.end(), end - put, -1);
+                put = end;
+            };
             for (int32_t c = 0; c < Q.n_ctx; ++c) {
                 HbgContext C;
                 C.query = k;
@@ -257,15 +280,14 @@ std::string build_batch(const std::vector<QueryIn> &qs, int32_t threshold,
                 C.cutoff = q.cutoff[c];
                 int32_t ci = (int32_t)b.contexts.size();
                 b.contexts.push_back(C);
-                for (int32_t i = 0; i < q.ctx_len[c]; ++i)
-                    b.ctx_of[at + q.ctx_off[c] + i] = ci;
+                gap(q.ctx_off[c]);
+                b.letters.insert(b.letters.end(), q.seq + put, q.seq + put + q.ctx_len[c]);
+                b.ctx_of.insert(b.ctx_of.end(), q.ctx_len[c], ci);
+                put += q.ctx_len[c];
                 if (q.ctx_len[c] >= HBG_WORD_SIZE)
                     b.runs.push_back({g, glen + q.ctx_off[c], q.ctx_len[c]});
             }
-            // letters between contexts are sentinels whatever the caller put there
-            for (int32_t i = 0; i < q.len; ++i)
-                if (b.ctx_of[at + i] < 0)
-                    b.letters[at + i] = 0;
+            gap(q.len);
             glen += q.len;
             ++k;
         }

@@ -294,3 +294,25 @@ def test_tables_without_host_memory_are_an_error(built):
     code = _LITTLE_MEMORY.format(paths=[str(p) for p in (ROOT / "h-blast_gb300", ROOT)])
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and r.stdout.strip() == "ok", (r.returncode, r.stdout, r.stderr)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 23, 40])
+def test_bad_letters_are_found_at_every_place(built, n):
+    """Letters are checked eight at a time: one outside 1..27 is found wherever it
+    stands in a context, and all letters inside are accepted; between contexts any
+    letter may stand and counts as a sentinel."""
+    good = np.array([1 + i % 27 for i in range(n)], np.uint8)
+    hblast.Batch.proteins([hblast.ProteinQuery.blastp(good)]).close()
+    for at in range(n):
+        for letter in (0, 28, 100, 127, 128, 155, 156, 255):
+            q = good.copy()
+            q[at] = letter
+            with pytest.raises(hblast.HblastError, match="letter outside"):
+                hblast.Batch.proteins([hblast.ProteinQuery.blastp(q)])
+    s = np.concatenate([good, [255, 99], good, [0], good]).astype(np.uint8)
+    two = hblast.Batch.proteins([hblast.ProteinQuery(s, [0, n + 2, 2 * n + 3], [n] * 3, [16] * 3, [41] * 3)])
+    clean = s.copy()
+    clean[[n, n + 1]] = 0
+    ref = hblast.Batch.proteins([hblast.ProteinQuery(clean, [0, n + 2, 2 * n + 3], [n] * 3, [16] * 3, [41] * 3)])
+    for x, y in zip(two.lookup_table(0), ref.lookup_table(0)):
+        assert np.array_equal(x, y)
